@@ -169,14 +169,14 @@ static __global__ void k_divb(DevCfg c, const double* __restrict__ p, const doub
 // ---------------------------------------------------------------------------
 // EMHD pre-pass: u_mu and T of the stage element at every zone
 // ---------------------------------------------------------------------------
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void k_emhd_prepass(DevCfg c, const double* __restrict__ ps, const double* __restrict__ geoC,
                                         double* __restrict__ uT) {
   long long z = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (z >= c.Z) return;
   int i, j, k;
   zijk(c, z, i, j, k);
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
   const long long Z = c.Z;
   ElemT<double, double> e;
@@ -224,8 +224,8 @@ GRIM_D void recon_zone(const DevCfg& c, const double* __restrict__ ps, long long
 // by the caller) while the left element is evaluated, then the left
 // state's fluxes (slots 0, 1) while the right element is; slot [v][thread],
 // 3 x DOF doubles per thread.  Neither holds registers across an element.
-template <int COND, int VISC>
-GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const ZoneGeo<double>& G,
+template <int COND, int VISC, class GT>
+GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const GT& G,
                          double* __restrict__ flux, long long z, double* __restrict__ park) {
   constexpr int NF = 5 + COND + VISC;
   constexpr int DOF = NF + 3;
@@ -286,9 +286,9 @@ GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const ZoneG
 // The same face flux with both states' elements evaluated side by side
 // (no shared-memory parking): twice the independent arithmetic per thread
 // for more registers, which the autotuner weighs against occupancy.
-template <int COND, int VISC>
+template <int COND, int VISC, class GT>
 GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const double* pr,
-                              const ZoneGeo<double>& G, double* __restrict__ flux, long long z) {
+                              const GT& G, double* __restrict__ flux, long long z) {
   constexpr int NF = 5 + COND + VISC;
   constexpr int DOF = NF + 3;
   const long long Z = c.Z;
@@ -328,7 +328,7 @@ GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const 
 // X1 faces: warp w of a row covers faces i0 .. i0+30; lane l reconstructs
 // zone i0 - 1 + l and, for l >= 1, computes the face between zones
 // i0 - 2 + l and i0 - 1 + l with the left state shuffled from lane l - 1.
-template <int COND, int VISC, int MINB, bool PAIR, int RS>
+template <int COND, int VISC, bool FLAT, int MINB, bool PAIR, int RS>
 __global__ void __launch_bounds__(128, MINB) k_face_flux_x1(DevCfg c, const double* __restrict__ ps,
                                                       const double* __restrict__ geoF, double* __restrict__ flux) {
   constexpr int DOF = 8 + COND + VISC;
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_x1(DevCfg c, const doub
 #pragma unroll
   for (int v = 0; v < DOF; v++) pl[v] = __shfl_up_sync(0xffffffffu, ro[v], 1);
   if (lane == 0 || iz > c.N1T - 3) return;
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, geoF, z, iz, j, 0., 0.5);
   if constexpr (PAIR) {
     riemann_face_pair<COND, VISC>(c, 0, pl, lo, G, flux, z);
@@ -433,7 +433,7 @@ GRIM_D void tma_load_4d(void* dst, const CUtensorMap* map, unsigned long long* b
       : "memory");
 }
 
-template <int COND, int VISC, int MINB, int RS, bool PAIR>
+template <int COND, int VISC, bool FLAT, int MINB, int RS, bool PAIR>
 __global__ void __launch_bounds__(128, MINB) k_face_flux_x1_tma(const __grid_constant__ CUtensorMap tmap, DevCfg c,
                                                                  const double* __restrict__ geoF,
                                                                  double* __restrict__ flux, DevState* st) {
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_x1_tma(const __grid_con
     for (int v = 0; v < DOF; v++) pl[v] = __shfl_up_sync(0xffffffffu, ro[v], 1);
     if (lane > 0 && reconOK) {
       const long long z = zidx(c, iz, j, k);
-      ZoneGeo<double> G;
+      Geo<FLAT, double> G;
       load_geo(G, c, geoF, z, iz, j, 0., 0.5);
       if constexpr (PAIR) {
         riemann_face_pair<COND, VISC>(c, 0, pl, lo, G, flux, z);
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_x1_tma(const __grid_con
 // box is (4, 12, 1, dof) for X2 and (4, 1, 12, dof) for X3; x starts at 4q
 // (32-byte aligned) and the box along DIR at 7 x chunk (never negative).
 constexpr int kStripRows = 12;
-template <int COND, int VISC, int MINB, int DIR, int RS, bool PAIR>
+template <int COND, int VISC, bool FLAT, int MINB, int DIR, int RS, bool PAIR>
 __global__ void __launch_bounds__(128, MINB) k_face_flux_strip_tma(const __grid_constant__ CUtensorMap tmap, DevCfg c,
                                                                     const double* __restrict__ geoF,
                                                                     const double* __restrict__ geoC,
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_strip_tma(const __grid_
     for (int v = 0; v < DOF; v++) pl[v] = __shfl_up_sync(0xffffffffu, ro[v], QI);
     if (lane >= QI && reconOK) {
       const long long z = (DIR == 1) ? zidx(c, i, x, other) : zidx(c, i, other, x);
-      ZoneGeo<double> G;
+      Geo<FLAT, double> G;
       // X3 faces use the centre geometry of each side (fvmfluxes.cpp:150-151),
       // one and the same: the metric does not depend on X3
       if (DIR == 2)
@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_strip_tma(const __grid_
 // state moves QI lanes up by shuffle, giving (32/QI - 1) x QI faces per
 // warp.  With QI = 4 each warp-wide load still covers whole 32-byte
 // sectors (4 consecutive doubles along i), as in the X1 kernel.
-template <int COND, int VISC, int QI, int MINB, bool PAIR, int DIR, int RS>
+template <int COND, int VISC, bool FLAT, int QI, int MINB, bool PAIR, int DIR, int RS>
 __global__ void __launch_bounds__(128, MINB) k_face_flux_strip(DevCfg c, const double* __restrict__ ps,
                                                          const double* __restrict__ geoF,
                                                          const double* __restrict__ geoC, double* __restrict__ flux) {
@@ -664,7 +664,7 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_strip(DevCfg c, const d
 #pragma unroll
   for (int v = 0; v < DOF; v++) pl[v] = __shfl_up_sync(0xffffffffu, ro[v], QI);
   if (lane < QI || !reconOK) return;
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   // X3 faces use the centre geometry of each side (fvmfluxes.cpp:150-151),
   // which is one and the same: the metric does not depend on X3
   if (dir == 2)
@@ -737,7 +737,7 @@ static __global__ void k_emf(DevCfg c, const double* __restrict__ F1, const doub
 // stream that wants warps in flight more than registers (measured on the
 // 3D torus: 64 registers with a few spills beat 85 and 98 without)
 constexpr int kEpiMinBlocks[3] = {4, 5, 8};
-template <int COND, int VISC, int PART>
+template <int COND, int VISC, bool FLAT, int PART>
 __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(DevCfg c, int stage, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
   }
 
   }  // PART != 1
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
   if constexpr (PART != 2) {
   // ---- stage element at the centre (elemOld / elemHalfStep)
@@ -863,8 +863,8 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
   double S[NF];
 #pragma unroll
   for (int v = 0; v < NF; v++) S[v] = 0.;
-  const bool needS = (c.metric != GRIM_MINKOWSKI) || COND || VISC;
-  if (c.metric != GRIM_MINKOWSKI) {
+  constexpr bool needS = !FLAT || COND || VISC;
+  if constexpr (!FLAT) {
     double T[4][4];
 #pragma unroll
     for (int ka = 0; ka < 4; ka++)
@@ -915,7 +915,7 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
       gu[1][mu] = st(mu, 0, c.dX[0]);
       gu[2][mu] = (c.dim > 1) ? st(mu, 1, c.dX[1]) : 0.;
       gu[3][mu] = (c.dim > 2) ? st(mu, 2, c.dX[2]) : 0.;
-      if (c.metric != GRIM_MINKOWSKI) {
+      if constexpr (!FLAT) {
 #pragma unroll
         for (int nu = 0; nu < 4; nu++)
 #pragma unroll
@@ -930,14 +930,20 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
       gT[3] = (c.dim > 2) ? st(4, 2, c.dX[2]) : 0.;
     }
     double dv = 0.;
+    // in Minkowski only the diagonal enters, and nothing along X^0 (gu[0]
+    // is zero) here and below
+    if constexpr (FLAT) {
+      dv = gu[1][1] + gu[2][2] + gu[3][3];
+    } else {
 #pragma unroll
-    for (int mu = 0; mu < 4; mu++)
+      for (int mu = 0; mu < 4; mu++)
 #pragma unroll
-      for (int nu = 0; nu < 4; nu++) dv += G.gcon[mu][nu] * gu[mu][nu];
+        for (int nu = 0; nu < 4; nu++) dv += G.gcon[mu][nu] * gu[mu][nu];
+    }
     if (VISC) {
       double d0 = -dv * e.rho * e.nu;
 #pragma unroll
-      for (int mu = 0; mu < 4; mu++)
+      for (int mu = FLAT ? 1 : 0; mu < 4; mu++)
 #pragma unroll
         for (int nu = 0; nu < 4; nu++) d0 += 3. * e.rho * e.nu * e.bCon[mu] * e.bCon[nu] / e.bSqr * gu[mu][nu];
       double d0t = (c.hoVisc == 1) ? d0 * sqrt(e.tau / e.rho / e.nu / e.temperature) : d0;
@@ -948,7 +954,7 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
     if (COND) {
       double qq = 0.;
 #pragma unroll
-      for (int mu = 0; mu < 4; mu++) {
+      for (int mu = FLAT ? 1 : 0; mu < 4; mu++) {
         qq -= e.rho * e.chi * e.bCon[mu] / e.bNorm * gT[mu];
 #pragma unroll
         for (int nu = 0; nu < 4; nu++) qq -= e.rho * e.chi * e.temperature * e.bCon[nu] / e.bNorm * e.uCon[mu] * gu[mu][nu];
@@ -996,8 +1002,8 @@ GRIM_D void atomic_max_pos(double* addr, double v) {
 }
 
 // one zone's sum over directions of max(c_max/dX_d, |c_min/dX_d|)
-template <int COND, int VISC>
-GRIM_D double elem_inv_dt(const DevCfg& c, const ElemT<double, double>& e, const ZoneGeo<double>& G) {
+template <int COND, int VISC, class GT>
+GRIM_D double elem_inv_dt(const DevCfg& c, const ElemT<double, double>& e, const GT& G) {
   double acc = 0.;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
@@ -1018,8 +1024,8 @@ GRIM_D double elem_inv_dt(const DevCfg& c, const ElemT<double, double>& e, const
   }
   return acc;
 }
-template <int COND, int VISC>
-GRIM_D double zone_inv_dt(const DevCfg& c, const double* pv, const ZoneGeo<double>& G) {
+template <int COND, int VISC, class GT>
+GRIM_D double zone_inv_dt(const DevCfg& c, const double* pv, const GT& G) {
   ElemT<double, double> e;
   elem_of<COND, VISC>(e, c, pv, G);
   return elem_inv_dt<COND, VISC>(c, e, G);
@@ -1040,7 +1046,7 @@ GRIM_D void block_max_to(double best, double* out) {
   }
 }
 
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void k_dt_speeds(DevCfg c, const double* __restrict__ p, const double* __restrict__ geoC,
                                      int mode, DevState* st) {
   long long z = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1056,7 +1062,7 @@ __global__ void k_dt_speeds(DevCfg c, const double* __restrict__ p, const double
     double pv[DOF];
 #pragma unroll
     for (int v = 0; v < DOF; v++) pv[v] = zero ? 0. : p[(long long)v * Z + src];
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
     if (!in_exchange_ghost(c, i, j, k)) best = zone_inv_dt<COND, VISC>(c, pv, G);
   }
@@ -1075,7 +1081,7 @@ __global__ void k_dt_speeds(DevCfg c, const double* __restrict__ p, const double
 // Every step of the reference's sequence acts on one zone at a time, so the
 // fused pass gives the same values (the NaN flag is counted beforehand over
 // the interior of src, which the copy leaves unchanged).
-template <int COND, int VISC, bool FLOOR, bool POST>
+template <int COND, int VISC, bool FLAT, bool FLOOR, bool POST>
 __global__ void __launch_bounds__(128) k_stage_finish(DevCfg c, TorusCfg t, const double* __restrict__ src,
                                                       double* __restrict__ dst, const double* __restrict__ geoC,
                                                       const unsigned long long* nanFlag, int dtOn, DevState* st) {
@@ -1092,7 +1098,7 @@ __global__ void __launch_bounds__(128) k_stage_finish(DevCfg c, TorusCfg t, cons
     double q[DOF];
 #pragma unroll
     for (int v = 0; v < DOF; v++) q[v] = zero ? 0. : src[(long long)v * Z + s];
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
     // the floors' last element, when it is that of the final state, serves
     // the dt speeds below (the same function of the same values)
@@ -1142,7 +1148,7 @@ GRIM_D double obs_join(int v, double a, double b) {
   return v == OBS_RHOMAX ? fmax(a, b) : (v == OBS_BETAMIN ? fmin(a, b) : a + b);
 }
 
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void __launch_bounds__(128, 5) k_torus_obs_partial(DevCfg c, const double* __restrict__ p,
                                                            const double* __restrict__ geoC, double volElem,
                                                            double every, const DevState* st,
@@ -1163,7 +1169,7 @@ __global__ void __launch_bounds__(128, 5) k_torus_obs_partial(DevCfg c, const do
     double q[DOF];
 #pragma unroll
     for (int v = 0; v < DOF; v++) q[v] = p[(long long)v * Z + z];
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
     ElemT<double, double> e;
     elem_of<COND, VISC>(e, c, q, G);
@@ -1248,12 +1254,12 @@ static __global__ void k_advance_time(DevState* st) {
 // ---------------------------------------------------------------------------
 // Newton
 // ---------------------------------------------------------------------------
-template <int COND, int VISC>
+template <int COND, int VISC, class GT>
 GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, int stage, const StageBufs& b,
-                             long long z, const ZoneGeo<double>& G) {
+                             long long z, const GT& G) {
   constexpr int NF = 5 + COND + VISC;
   const long long Z = c.Z;
-  const bool needS = (c.metric != GRIM_MINKOWSKI) || COND || VISC;
+  constexpr bool needS = !GT::flat || COND || VISC;
   const double dt = b.st->dt;
   K.dtp = (stage == GRIM_HALF_STEP) ? dt / 2. : dt;
   K.idtp = 1. / K.dtp;
@@ -1394,7 +1400,7 @@ GRIM_D double l2sum(const double* R) {
 
 // Parity Newton, launch 0: floor, residual, per-zone l2 and the count of
 // unconverged zones for iteration 0 (solve.cpp:17-41)
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void __launch_bounds__(128) k_newton_fd_init(DevCfg c, int stage, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1404,7 +1410,7 @@ __global__ void __launch_bounds__(128) k_newton_fd_init(DevCfg c, int stage, Sta
     const long long z = interior_to_z(c, n);
     int i, j, k;
     zijk(c, z, i, j, k);
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
     StageConst<NF> K;
     load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -1432,7 +1438,7 @@ __global__ void __launch_bounds__(128) k_newton_fd_init(DevCfg c, int stage, Sta
 // solve, quadratic backtracking, update; then the floor + residual + count
 // of iteration it+1.  Returns at once when iteration `it` found every zone
 // converged (the reference's global break).
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void __launch_bounds__(128) k_newton_fd_iter(DevCfg c, int stage, int it, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
   if (b.st->count[stage][it] == 0ULL) return;
@@ -1443,7 +1449,7 @@ __global__ void __launch_bounds__(128) k_newton_fd_iter(DevCfg c, int stage, int
     const long long z = interior_to_z(c, n);
     int i, j, k;
     zijk(c, z, i, j, k);
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
     StageConst<NF> K;
     load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -1522,8 +1528,8 @@ __global__ void __launch_bounds__(128) k_newton_fd_iter(DevCfg c, int stage, int
 // and solve in FP32, residual in FP64, i.e. FP32 inexact Newton refined by
 // the FP64 residual).
 // ---------------------------------------------------------------------------
-template <int COND, int VISC, class T, bool GENERIC = false>
-GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>& K, const ZoneGeo<T>& Gt,
+template <int COND, int VISC, class T, bool GENERIC = false, class GT>
+GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>& K, const GT& Gt,
                              const DevCfg& c, T J[5 + COND + VISC][5 + COND + VISC]) {
   constexpr int NF = 5 + COND + VISC;
   if constexpr (COND == 0 && VISC == 0 && !GENERIC) {
@@ -1548,8 +1554,8 @@ GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>&
 // the solve and the backtracking line search (solve.cpp:80-199 per zone).
 // Returns with conv set when the test passed (`it` = the updates taken) or
 // with it == itEnd.
-template <int COND, int VISC, class T>
-GRIM_D void fast_newton_iters(const DevCfg& c, const StageConst<5 + COND + VISC>& K, const ZoneGeo<double>& G,
+template <int COND, int VISC, class T, class GT>
+GRIM_D void fast_newton_iters(const DevCfg& c, const StageConst<5 + COND + VISC>& K, const GT& G,
                               double* P, double* R, bool& haveR, double& l2first, int& it, bool& conv,
                               int itEnd) {
   constexpr int NF = 5 + COND + VISC;
@@ -1565,12 +1571,8 @@ GRIM_D void fast_newton_iters(const DevCfg& c, const StageConst<5 + COND + VISC>
     {
       // the Jacobian's geometry, converted where it is used rather than
       // kept beside the FP64 copy across the iterations
-      ZoneGeo<T> Gt;
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = (T)G.gcov[m][q]; Gt.gcon[m][q] = (T)G.gcon[m][q]; }
-      Gt.g = (T)G.g; Gt.alpha = (T)G.alpha; Gt.ialpha = (T)G.ialpha; Gt.x1 = (T)G.x1; Gt.x2 = (T)G.x2; Gt.dyn = (T)G.dyn;
+      Geo<GT::flat, T> Gt;
+      convert_geo(Gt, G);
       tangent_jacobian<COND, VISC, T>(P, K, Gt, c, J);
     }
     T bv[NF], xv[NF];
@@ -1606,8 +1608,8 @@ GRIM_D void fast_newton_iters(const DevCfg& c, const StageConst<5 + COND + VISC>
 // last step whose line search ran out was applied unevaluated: its residual
 // is formed here, at the floored state the next iteration would see.
 // Returns true when the zone is above tolerance.
-template <int COND, int VISC>
-GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>& K, const ZoneGeo<double>& G,
+template <int COND, int VISC, class GT>
+GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>& K, const GT& G,
                               const double* P, double* R, bool haveR, double l2first) {
   constexpr int NF = 5 + COND + VISC;
   if (!haveR) {
@@ -1623,7 +1625,7 @@ GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>
 }
 
 constexpr int kNewtonMinBlocks = 3;  // blocks per SM of the ideal FP32-Jacobian Newton
-template <int COND, int VISC, class T>
+template <int COND, int VISC, bool FLAT, class T>
 __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b,
                                                               const int* __restrict__ list, long long nlist) {
   constexpr int NF = 5 + COND + VISC;
@@ -1635,7 +1637,7 @@ __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kN
     const long long z = list ? (long long)list[n] : interior_to_z(c, n);
     int i, j, k;
     zijk(c, z, i, j, k);
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
     StageConst<NF> K;
     load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -1699,7 +1701,7 @@ struct DeferStash {
   int haveR[kDeferCap];
 };
 
-template <class T>
+template <class T, bool FLAT>
 __global__ void __launch_bounds__(32 * kDeferWarps, kNewtonMinBlocks) k_newton_defer(DevCfg c, int stage, StageBufs b,
                                                                                   long long nlist) {
   constexpr int NF = 5;
@@ -1747,7 +1749,7 @@ __global__ void __launch_bounds__(32 * kDeferWarps, kNewtonMinBlocks) k_newton_d
       z = tail ? (long long)S.z[sl] : interior_to_z(c, n);
       int i, j, k;
       zijk(c, z, i, j, k);
-      ZoneGeo<double> G;
+      Geo<FLAT, double> G;
       load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
       if (tail) {
         K.dtp = dtp;
@@ -1836,13 +1838,13 @@ GRIM_D void list_append(int* list, unsigned long long* count, int zone, bool tak
 
 // Launch 0, one zone: floors, residual, stored state; true when the zone
 // is above tolerance (goes on the worklist).
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 GRIM_D bool list_init_zone(const DevCfg& c, int stage, const StageBufs& b, long long z) {
   constexpr int NF = 5 + COND + VISC;
   const long long Z = c.Z;
   int i, j, k;
   zijk(c, z, i, j, k);
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
   StageConst<NF> K;
   load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -1864,21 +1866,17 @@ GRIM_D bool list_init_zone(const DevCfg& c, int stage, const StageBufs& b, long 
 // Launch it >= 1, one zone on the worklist: one Newton update from the
 // stored state; true when the zone stays above tolerance (and it is not
 // the last iteration).
-template <int COND, int VISC, class T>
+template <int COND, int VISC, bool FLAT, class T>
 GRIM_D bool list_iter_zone(const DevCfg& c, int stage, int it, const StageBufs& b, long long z) {
   constexpr int NF = 5 + COND + VISC;
   const long long Z = c.Z;
   const bool last = (it == c.maxIter);
   int i, j, k;
   zijk(c, z, i, j, k);
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
-  ZoneGeo<T> Gt;
-#pragma unroll
-  for (int m = 0; m < 4; m++)
-#pragma unroll
-    for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = (T)G.gcov[m][q]; Gt.gcon[m][q] = (T)G.gcon[m][q]; }
-  Gt.g = (T)G.g; Gt.alpha = (T)G.alpha; Gt.ialpha = (T)G.ialpha; Gt.x1 = (T)G.x1; Gt.x2 = (T)G.x2; Gt.dyn = (T)G.dyn;
+  Geo<FLAT, T> Gt;
+  convert_geo(Gt, G);
   StageConst<NF> K;
   load_stage_const<COND, VISC>(K, c, stage, b, z, G);
   double P[NF], R[NF];
@@ -1931,7 +1929,7 @@ GRIM_D bool list_iter_zone(const DevCfg& c, int stage, int it, const StageBufs& 
   return !conv && !last;
 }
 
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void __launch_bounds__(128) k_newton_list_init(DevCfg c, int stage, StageBufs b) {
   for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < c.Zint; n0 += (long long)gridDim.x * blockDim.x) {
     const long long n = n0 + threadIdx.x;
@@ -1939,14 +1937,14 @@ __global__ void __launch_bounds__(128) k_newton_list_init(DevCfg c, int stage, S
     long long z = 0;
     if (n < c.Zint) {
       z = interior_to_z(c, n);
-      take = list_init_zone<COND, VISC>(c, stage, b, z);
+      take = list_init_zone<COND, VISC, FLAT>(c, stage, b, z);
     }
     hist_add(b.st->itHist[stage], 0, n < c.Zint && !take);
     list_append(b.list[0], &b.st->listCount[0], (int)z, take);
   }
 }
 
-template <int COND, int VISC, class T>
+template <int COND, int VISC, bool FLAT, class T>
 __global__ void __launch_bounds__(128) k_newton_list_iter(DevCfg c, int stage, int it, StageBufs b) {
   const int in = (it - 1) & 1, out = it & 1;
   const long long count = (long long)b.st->listCount[in];
@@ -1957,7 +1955,7 @@ __global__ void __launch_bounds__(128) k_newton_list_iter(DevCfg c, int stage, i
     int zone = 0;
     if (n < count) {
       zone = b.list[in][n];
-      take = list_iter_zone<COND, VISC, T>(c, stage, it, b, zone);
+      take = list_iter_zone<COND, VISC, FLAT, T>(c, stage, it, b, zone);
     }
     hist_add(b.st->itHist[stage], min(it, 15), n < count && !take);
     if (!last) list_append(b.list[out], &b.st->listCount[out], zone, take);
@@ -1990,7 +1988,7 @@ GRIM_D void batch_hist_add(const BatchEntry* tbl, int stage, int p, int bin, boo
     atomicAdd(&tbl[p].b[stage].st->itHist[stage][bin], (unsigned long long)__popc(peers));
 }
 
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void __launch_bounds__(128) k_batch_list_init(const BatchEntry* __restrict__ tbl, int nprob,
                                                          long long total, int stage, BatchState* bs) {
   for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < total; n0 += (long long)gridDim.x * blockDim.x) {
@@ -2001,14 +1999,14 @@ __global__ void __launch_bounds__(128) k_batch_list_init(const BatchEntry* __res
       p = batch_problem(tbl, nprob, gidx_);
       const DevCfg& c = tbl[p].c;
       const long long z = interior_to_z(c, gidx_ - tbl[p].offset);
-      take = list_init_zone<COND, VISC>(c, stage, tbl[p].b[stage], z);
+      take = list_init_zone<COND, VISC, FLAT>(c, stage, tbl[p].b[stage], z);
     }
     batch_hist_add(tbl, stage, p, 0, gidx_ < total && !take);
     list_append(bs->list[0], &bs->listCount[0], (int)gidx_, take);
   }
 }
 
-template <int COND, int VISC, class T>
+template <int COND, int VISC, bool FLAT, class T>
 __global__ void __launch_bounds__(128) k_batch_list_iter(const BatchEntry* __restrict__ tbl, int nprob, int stage,
                                                          int it, int lastIt, BatchState* bs) {
   const int in = (it - 1) & 1, out = it & 1;
@@ -2024,7 +2022,7 @@ __global__ void __launch_bounds__(128) k_batch_list_iter(const BatchEntry* __res
       const long long z = interior_to_z(c, gidx_ - tbl[p].offset);
       // a problem past its own maxIter leaves the list (its last update
       // was counted there)
-      if (it <= c.maxIter) take = list_iter_zone<COND, VISC, T>(c, stage, it, tbl[p].b[stage], z);
+      if (it <= c.maxIter) take = list_iter_zone<COND, VISC, FLAT, T>(c, stage, it, tbl[p].b[stage], z);
     }
     batch_hist_add(tbl, stage, p, min(it, 15), n < count && !take);
     {
@@ -2043,7 +2041,7 @@ __global__ void __launch_bounds__(128) k_batch_list_iter(const BatchEntry* __res
 // ---------------------------------------------------------------------------
 // kernels behind the test entry points
 // ---------------------------------------------------------------------------
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void k_residual(DevCfg c, int stage, StageBufs b, const double* __restrict__ pg,
                                     double* __restrict__ out) {
   constexpr int NF = 5 + COND + VISC;
@@ -2058,7 +2056,7 @@ __global__ void k_residual(DevCfg c, int stage, StageBufs b, const double* __res
     for (int v = 0; v < NF; v++) out[(long long)v * Z + z] = 0.;
     return;
   }
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
   StageConst<NF> K;
   load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -2072,7 +2070,7 @@ __global__ void k_residual(DevCfg c, int stage, StageBufs b, const double* __res
   for (int v = 0; v < NF; v++) out[(long long)v * Z + z] = R[v];
 }
 
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void k_jacobian(DevCfg c, int stage, StageBufs b, const double* __restrict__ pg,
                                     double* __restrict__ jac, int tangent) {
   constexpr int NF = 5 + COND + VISC;
@@ -2088,7 +2086,7 @@ __global__ void k_jacobian(DevCfg c, int stage, StageBufs b, const double* __res
 #pragma unroll
     for (int q = 0; q < NF; q++) J[a][q] = 0.;
   if (inner) {
-    ZoneGeo<double> G;
+    Geo<FLAT, double> G;
     load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
     StageConst<NF> K;
     load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -2104,13 +2102,8 @@ __global__ void k_jacobian(DevCfg c, int stage, StageBufs b, const double* __res
     } else if (tangent == 3) {
       // the form and precision the mixed Newton uses: geometry rounded to
       // FP32, the Jacobian in FP32
-      ZoneGeo<float> Gt;
-#pragma unroll
-      for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = (float)G.gcov[m][q]; Gt.gcon[m][q] = (float)G.gcon[m][q]; }
-      Gt.g = (float)G.g; Gt.alpha = (float)G.alpha; Gt.ialpha = (float)G.ialpha; Gt.x1 = (float)G.x1;
-      Gt.x2 = (float)G.x2; Gt.dyn = (float)G.dyn;
+      Geo<FLAT, float> Gt;
+      convert_geo(Gt, G);
       float Jf[NF][NF];
       tangent_jacobian<COND, VISC, float>(P, K, Gt, c, Jf);
 #pragma unroll
@@ -2144,7 +2137,7 @@ __global__ void k_jacobian(DevCfg c, int stage, StageBufs b, const double* __res
 // (fluidElement::computeFluxes, physics.cpp:185-217; fdir 0 gives the
 // conserved variables) and / or its characteristic speeds along the
 // spatial direction dir into mn, mx
-template <int COND, int VISC>
+template <int COND, int VISC, bool FLAT>
 __global__ void k_conserved(DevCfg c, const double* __restrict__ p, const double* __restrict__ geoC,
                                      double* __restrict__ out, int fdir, int dir, double* mn, double* mx) {
   constexpr int NF = 5 + COND + VISC;
@@ -2153,7 +2146,7 @@ __global__ void k_conserved(DevCfg c, const double* __restrict__ p, const double
   const long long Z = c.Z;
   int i, j, k;
   zijk(c, z, i, j, k);
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
   ElemT<double, double> e;
   elem_set<COND, VISC>(e, p[z], p[Z + z], p[2 * Z + z], p[3 * Z + z], p[4 * Z + z], p[(long long)c.B1 * Z + z],
@@ -2253,6 +2246,24 @@ static inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) 
     else if ((c).viscosity) KERNEL<0, 1>(__VA_ARGS__);                  \
     else KERNEL<0, 0>(__VA_ARGS__);                                     \
   } while (0)
+// the same, and the kernel of the configuration's metric (FLAT: Minkowski)
+#define GRIM_GEO_DISPATCH(c, KERNEL, ...)                                     \
+  do {                                                                        \
+    const bool flat_ = (c).metric == GRIM_MINKOWSKI;                          \
+    if ((c).conduction && (c).viscosity) {                                    \
+      if (flat_) KERNEL<1, 1, true>(__VA_ARGS__);                             \
+      else KERNEL<1, 1, false>(__VA_ARGS__);                                  \
+    } else if ((c).conduction) {                                              \
+      if (flat_) KERNEL<1, 0, true>(__VA_ARGS__);                             \
+      else KERNEL<1, 0, false>(__VA_ARGS__);                                  \
+    } else if ((c).viscosity) {                                               \
+      if (flat_) KERNEL<0, 1, true>(__VA_ARGS__);                             \
+      else KERNEL<0, 1, false>(__VA_ARGS__);                                  \
+    } else {                                                                  \
+      if (flat_) KERNEL<0, 0, true>(__VA_ARGS__);                             \
+      else KERNEL<0, 0, false>(__VA_ARGS__);                                  \
+    }                                                                         \
+  } while (0)
 
 #if !defined(GRIM_ONLY_FACES)
 void ghost_fill(const DevCfg& c, double* prim, int nv, cudaStream_t s) {
@@ -2262,12 +2273,12 @@ void communicate(const DevCfg& c, double* prim, int nv, cudaStream_t s) {
   k_communicate<<<nblk(c.Z, 256), 256, 0, s>>>(c, prim, nv);
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void emhd_prepass_t(const DevCfg& c, const double* ps, const double* geoC, double* uT, cudaStream_t s) {
-  k_emhd_prepass<C, V><<<nblk(c.Z, 128), 128, 0, s>>>(c, ps, geoC, uT);
+  k_emhd_prepass<C, V, F><<<nblk(c.Z, 128), 128, 0, s>>>(c, ps, geoC, uT);
 }
 void emhd_prepass(const DevCfg& c, const double* ps, const double* geoC, double* uT, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, emhd_prepass_t, c, ps, geoC, uT, s);
+  GRIM_GEO_DISPATCH(c, emhd_prepass_t, c, ps, geoC, uT, s);
 }
 
 #endif  // !GRIM_ONLY_FACES
@@ -2280,19 +2291,19 @@ void emhd_prepass(const DevCfg& c, const double* ps, const double* geoC, double*
 // the reconstruction scheme is a compile-time constant of the X1 kernels
 // as of the TMA ones: one scheme's code per kernel keeps the instruction
 // footprint small
-template <int C, int V, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = false>
 static void face_x1_launch(const DevCfg& c, const double* ps, const double* geoF, double* flux, cudaStream_t s) {
   const long long warps = (long long)c.nfj * c.nfk * ((c.N1T - 5 + 30) / 31);
   const size_t park = PAIR ? 0 : 3 * (8 + C + V) * 128 * sizeof(double);
   const unsigned nb = nblk(warps * 32, 128);
   switch (c.reconstruction) {
-    case GRIM_WENO5: k_face_flux_x1<C, V, MINB, PAIR, GRIM_WENO5><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
-    case GRIM_PPM: k_face_flux_x1<C, V, MINB, PAIR, GRIM_PPM><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
-    case GRIM_MP5: k_face_flux_x1<C, V, MINB, PAIR, GRIM_MP5><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
-    default: k_face_flux_x1<C, V, MINB, PAIR, GRIM_MINMOD><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
+    case GRIM_WENO5: k_face_flux_x1<C, V, F, MINB, PAIR, GRIM_WENO5><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
+    case GRIM_PPM: k_face_flux_x1<C, V, F, MINB, PAIR, GRIM_PPM><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
+    case GRIM_MP5: k_face_flux_x1<C, V, F, MINB, PAIR, GRIM_MP5><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
+    default: k_face_flux_x1<C, V, F, MINB, PAIR, GRIM_MINMOD><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
   }
 }
-template <int C, int V, int QI, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int QI, int MINB, bool PAIR = false>
 static void face_strip_launch(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,
                               double* flux, cudaStream_t s) {
   const int NT = (dir == 1) ? c.N2T : c.N3T;
@@ -2303,8 +2314,8 @@ static void face_strip_launch(const DevCfg& c, int dir, const double* ps, const 
   // one kernel per reconstruction scheme, as for the X1 faces
 #define GRIM_STRIP_RS(RS)                                                                                  \
   do {                                                                                                     \
-    if (dir == 1) k_face_flux_strip<C, V, QI, MINB, PAIR, 1, RS><<<nb, 128, park, s>>>(c, ps, geoF, geoC, flux); \
-    else k_face_flux_strip<C, V, QI, MINB, PAIR, 2, RS><<<nb, 128, park, s>>>(c, ps, geoF, geoC, flux);        \
+    if (dir == 1) k_face_flux_strip<C, V, F, QI, MINB, PAIR, 1, RS><<<nb, 128, park, s>>>(c, ps, geoF, geoC, flux); \
+    else k_face_flux_strip<C, V, F, QI, MINB, PAIR, 2, RS><<<nb, 128, park, s>>>(c, ps, geoF, geoC, flux);        \
   } while (0)
   switch (c.reconstruction) {
     case GRIM_WENO5: GRIM_STRIP_RS(GRIM_WENO5); break;
@@ -2324,7 +2335,7 @@ static int sm_count() {
   }
   return n;
 }
-template <int C, int V, int MINB, int RS, bool PAIR>
+template <int C, int V, bool F, int MINB, int RS, bool PAIR>
 static void face_x1_tma_launch_rs(const DevCfg& c, const CUtensorMap* tmap, const double* geoF, double* flux,
                                   DevState* st, cudaStream_t s) {
   constexpr int DOF = 8 + C + V;
@@ -2335,25 +2346,25 @@ static void face_x1_tma_launch_rs(const DevCfg& c, const CUtensorMap* tmap, cons
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(attrDevices & (1ULL << dev))) {
-    cudaFuncSetAttribute(k_face_flux_x1_tma<C, V, MINB, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_face_flux_x1_tma<C, V, F, MINB, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
     attrDevices |= 1ULL << dev;
   }
-  k_face_flux_x1_tma<C, V, MINB, RS, PAIR><<<sm_count() * MINB, 32 * nw, smem, s>>>(*tmap, c, geoF, flux, st);
+  k_face_flux_x1_tma<C, V, F, MINB, RS, PAIR><<<sm_count() * MINB, 32 * nw, smem, s>>>(*tmap, c, geoF, flux, st);
 }
 // the reconstruction scheme becomes a compile-time constant of the TMA
 // kernels: one scheme's code per kernel keeps the instruction footprint small
-template <int C, int V, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = false>
 static void face_x1_tma_launch(const DevCfg& c, const CUtensorMap* tmap, const double* geoF, double* flux,
                                DevState* st, cudaStream_t s) {
   switch (c.reconstruction) {
-    case GRIM_WENO5: face_x1_tma_launch_rs<C, V, MINB, GRIM_WENO5, PAIR>(c, tmap, geoF, flux, st, s); break;
-    case GRIM_PPM: face_x1_tma_launch_rs<C, V, MINB, GRIM_PPM, PAIR>(c, tmap, geoF, flux, st, s); break;
-    case GRIM_MP5: face_x1_tma_launch_rs<C, V, MINB, GRIM_MP5, PAIR>(c, tmap, geoF, flux, st, s); break;
-    default: face_x1_tma_launch_rs<C, V, MINB, GRIM_MINMOD, PAIR>(c, tmap, geoF, flux, st, s); break;
+    case GRIM_WENO5: face_x1_tma_launch_rs<C, V, F, MINB, GRIM_WENO5, PAIR>(c, tmap, geoF, flux, st, s); break;
+    case GRIM_PPM: face_x1_tma_launch_rs<C, V, F, MINB, GRIM_PPM, PAIR>(c, tmap, geoF, flux, st, s); break;
+    case GRIM_MP5: face_x1_tma_launch_rs<C, V, F, MINB, GRIM_MP5, PAIR>(c, tmap, geoF, flux, st, s); break;
+    default: face_x1_tma_launch_rs<C, V, F, MINB, GRIM_MINMOD, PAIR>(c, tmap, geoF, flux, st, s); break;
   }
 }
-template <int C, int V, int MINB, int RS, bool PAIR>
+template <int C, int V, bool F, int MINB, int RS, bool PAIR>
 static void face_strip_tma_launch_rs(const DevCfg& c, int dir, const CUtensorMap* tmap, const double* geoF,
                                      const double* geoC, double* flux, DevState* st, cudaStream_t s) {
   constexpr int DOF = 8 + C + V;
@@ -2363,89 +2374,89 @@ static void face_strip_tma_launch_rs(const DevCfg& c, int dir, const CUtensorMap
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 64 && !(attrDevices & (1ULL << dev))) {
-    cudaFuncSetAttribute(k_face_flux_strip_tma<C, V, MINB, 1, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_face_flux_strip_tma<C, V, F, MINB, 1, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
-    cudaFuncSetAttribute(k_face_flux_strip_tma<C, V, MINB, 2, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_face_flux_strip_tma<C, V, F, MINB, 2, RS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
     attrDevices |= 1ULL << dev;
   }
   if (dir == 1)
-    k_face_flux_strip_tma<C, V, MINB, 1, RS, PAIR>
+    k_face_flux_strip_tma<C, V, F, MINB, 1, RS, PAIR>
         <<<sm_count() * MINB, 32 * nw, smem, s>>>(tmap[1], c, geoF, geoC, flux, st);
   else
-    k_face_flux_strip_tma<C, V, MINB, 2, RS, PAIR>
+    k_face_flux_strip_tma<C, V, F, MINB, 2, RS, PAIR>
         <<<sm_count() * MINB, 32 * nw, smem, s>>>(tmap[2], c, geoF, geoC, flux, st);
 }
-template <int C, int V, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = false>
 static void face_strip_tma_launch(const DevCfg& c, int dir, const CUtensorMap* tmap, const double* geoF,
                                   const double* geoC, double* flux, DevState* st, cudaStream_t s) {
   switch (c.reconstruction) {
     case GRIM_WENO5:
-      face_strip_tma_launch_rs<C, V, MINB, GRIM_WENO5, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s);
+      face_strip_tma_launch_rs<C, V, F, MINB, GRIM_WENO5, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s);
       break;
-    case GRIM_PPM: face_strip_tma_launch_rs<C, V, MINB, GRIM_PPM, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s); break;
-    case GRIM_MP5: face_strip_tma_launch_rs<C, V, MINB, GRIM_MP5, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+    case GRIM_PPM: face_strip_tma_launch_rs<C, V, F, MINB, GRIM_PPM, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+    case GRIM_MP5: face_strip_tma_launch_rs<C, V, F, MINB, GRIM_MP5, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s); break;
     default:
-      face_strip_tma_launch_rs<C, V, MINB, GRIM_MINMOD, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s);
+      face_strip_tma_launch_rs<C, V, F, MINB, GRIM_MINMOD, PAIR>(c, dir, tmap, geoF, geoC, flux, st, s);
       break;
   }
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void face_flux_t(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,
                         double* flux, int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s) {
   if constexpr (C == 0 && V == 0) {
     if (dir == 0) {
       if ((variant == 2 || variant == 3 || variant == 5) && tmap && st) {
-        if (variant == 5) face_x1_tma_launch<C, V, 3, true>(c, &tmap[0], geoF, flux, st, s);
-        else if (variant == 3) face_x1_tma_launch<C, V, 4>(c, &tmap[0], geoF, flux, st, s);
-        else face_x1_tma_launch<C, V, 3>(c, &tmap[0], geoF, flux, st, s);
+        if (variant == 5) face_x1_tma_launch<C, V, F, 3, true>(c, &tmap[0], geoF, flux, st, s);
+        else if (variant == 3) face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s);
+        else face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s);
       } else if (variant == 6) {
-        face_x1_launch<C, V, 4, true>(c, ps, geoF, flux, s);
+        face_x1_launch<C, V, F, 4, true>(c, ps, geoF, flux, s);
       } else if (variant == 4 || variant == 5) {
-        face_x1_launch<C, V, 3, true>(c, ps, geoF, flux, s);
+        face_x1_launch<C, V, F, 3, true>(c, ps, geoF, flux, s);
       } else if (variant == 1 || variant == 3) {
-        face_x1_launch<C, V, 4>(c, ps, geoF, flux, s);
+        face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s);
       } else {
-        face_x1_launch<C, V, 3>(c, ps, geoF, flux, s);
+        face_x1_launch<C, V, F, 3>(c, ps, geoF, flux, s);
       }
       return;
     }
     if (variant >= 8 && tmap && st) {
-      if (variant == 11) face_strip_tma_launch<C, V, 4, true>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else if (variant == 10) face_strip_tma_launch<C, V, 3, true>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else if (variant == 9) face_strip_tma_launch<C, V, 4>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_tma_launch<C, V, 3>(c, dir, tmap, geoF, geoC, flux, st, s);
+      if (variant == 11) face_strip_tma_launch<C, V, F, 4, true>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else if (variant == 10) face_strip_tma_launch<C, V, F, 3, true>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else if (variant == 9) face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s);
       return;
     }
     switch (variant) {
-      case 8: face_strip_launch<C, V, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 10: face_strip_launch<C, V, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 11: face_strip_launch<C, V, 4, 4, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 9: face_strip_launch<C, V, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 1: face_strip_launch<C, V, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 2: face_strip_launch<C, V, 2, 3>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 3: face_strip_launch<C, V, 2, 4>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 4: face_strip_launch<C, V, 8, 3>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 5: face_strip_launch<C, V, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 6: face_strip_launch<C, V, 8, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 7: face_strip_launch<C, V, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      default: face_strip_launch<C, V, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 8: face_strip_launch<C, V, F, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 10: face_strip_launch<C, V, F, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 11: face_strip_launch<C, V, F, 4, 4, true>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 9: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 1: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 2: face_strip_launch<C, V, F, 2, 3>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 3: face_strip_launch<C, V, F, 2, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 4: face_strip_launch<C, V, F, 8, 3>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 5: face_strip_launch<C, V, F, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 6: face_strip_launch<C, V, F, 8, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 7: face_strip_launch<C, V, F, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
+      default: face_strip_launch<C, V, F, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
     }
   } else {
     // EMHD elements need more registers: two resident blocks; variant 1
     // stages the stencils with TMA
     if (dir == 0) {
-      if (variant == 1 && tmap && st) face_x1_tma_launch<C, V, 2>(c, &tmap[0], geoF, flux, st, s);
-      else face_x1_launch<C, V, 2>(c, ps, geoF, flux, s);
+      if (variant == 1 && tmap && st) face_x1_tma_launch<C, V, F, 2>(c, &tmap[0], geoF, flux, st, s);
+      else face_x1_launch<C, V, F, 2>(c, ps, geoF, flux, s);
     } else {
-      if (variant == 1 && tmap && st) face_strip_tma_launch<C, V, 2>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_launch<C, V, 4, 2>(c, dir, ps, geoF, geoC, flux, s);
+      if (variant == 1 && tmap && st) face_strip_tma_launch<C, V, F, 2>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else face_strip_launch<C, V, F, 4, 2>(c, dir, ps, geoF, geoC, flux, s);
     }
   }
 }
 void face_flux(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC, double* flux,
                int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, face_flux_t, c, dir, ps, geoF, geoC, flux, variant, tmap, st, s);
+  GRIM_GEO_DISPATCH(c, face_flux_t, c, dir, ps, geoF, geoC, flux, variant, tmap, st, s);
 }
 // X1: 0, 1 = register budget 3 / 4 blocks; 2, 3 = the same with TMA-staged
 // rows (when the caller has a tensor map of the primitives); 4 = both face
@@ -2467,61 +2478,61 @@ int face_variants(const DevCfg& c, int dir) {
 #endif  // !GRIM_SKIP_FACES
 
 #if !defined(GRIM_ONLY_FACES)
-template <int C, int V>
+template <int C, int V, bool F>
 static void stage_epilogue_t(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
-  if (c.metric != GRIM_MINKOWSKI || C || V) {
+  if constexpr (!F || C || V) {
     // centre half first: the flux half's induction reads its consOld
-    k_stage_epilogue<C, V, 1><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
-    k_stage_epilogue<C, V, 2><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    k_stage_epilogue<C, V, F, 1><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    k_stage_epilogue<C, V, F, 2><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
   } else {
     // no explicit sources: one kernel
-    k_stage_epilogue<C, V, 0><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    k_stage_epilogue<C, V, F, 0><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
   }
 }
 void stage_epilogue(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, stage_epilogue_t, c, stage, b, s);
+  GRIM_GEO_DISPATCH(c, stage_epilogue_t, c, stage, b, s);
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void dt_speeds_t(const DevCfg& c, const double* p, const double* geoC, int mode, DevState* st,
                         cudaStream_t s) {
-  k_dt_speeds<C, V><<<nblk(c.Z, 256), 256, 0, s>>>(c, p, geoC, mode, st);
+  k_dt_speeds<C, V, F><<<nblk(c.Z, 256), 256, 0, s>>>(c, p, geoC, mode, st);
 }
 void dt_speeds(const DevCfg& c, const double* p, const double* geoC, int mode, DevState* st, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, dt_speeds_t, c, p, geoC, mode, st, s);
+  GRIM_GEO_DISPATCH(c, dt_speeds_t, c, p, geoC, mode, st, s);
 }
 void dt_update(DevState* st, double courant, double maxInc, cudaStream_t s) {
   k_dt_update<<<1, 32, 0, s>>>(st, courant, maxInc);
 }
 void advance_time(DevState* st, cudaStream_t s) { k_advance_time<<<1, 32, 0, s>>>(st); }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void newton_fd_init_t(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
-  k_newton_fd_init<C, V><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+  k_newton_fd_init<C, V, F><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
 }
 void newton_fd_init(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, newton_fd_init_t, c, stage, b, s);
+  GRIM_GEO_DISPATCH(c, newton_fd_init_t, c, stage, b, s);
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void newton_fd_iter_t(const DevCfg& c, int stage, int it, const StageBufs& b, cudaStream_t s) {
-  k_newton_fd_iter<C, V><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, it, b);
+  k_newton_fd_iter<C, V, F><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, it, b);
 }
 void newton_fd_iter(const DevCfg& c, int stage, int it, const StageBufs& b, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, newton_fd_iter_t, c, stage, it, b, s);
+  GRIM_GEO_DISPATCH(c, newton_fd_iter_t, c, stage, it, b, s);
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void newton_fast_t(const DevCfg& c, int stage, const StageBufs& b, int mode, const int* list,
                           long long nlist, cudaStream_t s) {
   if (nlist <= 0) return;
   if (mode == GRIM_NEWTON_MIXED32)
-    k_newton_fast<C, V, float><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
+    k_newton_fast<C, V, F, float><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
   else
-    k_newton_fast<C, V, double><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
+    k_newton_fast<C, V, F, double><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
 }
 void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, const int* list, long long nlist,
                  cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, newton_fast_t, c, stage, b, mode, list, nlist, s);
+  GRIM_GEO_DISPATCH(c, newton_fast_t, c, stage, b, mode, list, nlist, s);
 }
 
 #ifdef GRIM_FAST_MATH
@@ -2533,10 +2544,12 @@ bool newton_defer(const DevCfg& c, int stage, const StageBufs& b, int mode, cuda
     int dev = 0, sms = 148, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_newton_defer<float>, 32 * kDeferWarps, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_newton_defer<float, false>, 32 * kDeferWarps, 0);
     grid = sms * (per > 0 ? per : 1);
   }
-  if (c.Zint > 0) k_newton_defer<float><<<grid, 32 * kDeferWarps, 0, s>>>(c, stage, b, c.Zint);
+  if (c.Zint <= 0) return true;
+  if (c.metric == GRIM_MINKOWSKI) k_newton_defer<float, true><<<grid, 32 * kDeferWarps, 0, s>>>(c, stage, b, c.Zint);
+  else k_newton_defer<float, false><<<grid, 32 * kDeferWarps, 0, s>>>(c, stage, b, c.Zint);
   return true;
 }
 #endif
@@ -2551,69 +2564,69 @@ static int persistent_blocks() {
   }
   return nb;
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void newton_list_t(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
   const int nb = persistent_blocks();
   cudaMemsetAsync(b.st->listCount, 0, sizeof(b.st->listCount), s);
-  k_newton_list_init<C, V><<<nb, 128, 0, s>>>(c, stage, b);
+  k_newton_list_init<C, V, F><<<nb, 128, 0, s>>>(c, stage, b);
   for (int it = 1; it <= c.maxIter; it++) {
     // the list this launch appends to starts empty
     cudaMemsetAsync(&b.st->listCount[it & 1], 0, sizeof(unsigned long long), s);
     if (mode == GRIM_NEWTON_MIXED32)
-      k_newton_list_iter<C, V, float><<<nb, 128, 0, s>>>(c, stage, it, b);
+      k_newton_list_iter<C, V, F, float><<<nb, 128, 0, s>>>(c, stage, it, b);
     else
-      k_newton_list_iter<C, V, double><<<nb, 128, 0, s>>>(c, stage, it, b);
+      k_newton_list_iter<C, V, F, double><<<nb, 128, 0, s>>>(c, stage, it, b);
   }
 }
 void newton_list(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, newton_list_t, c, stage, b, mode, s);
+  GRIM_GEO_DISPATCH(c, newton_list_t, c, stage, b, mode, s);
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void batch_newton_t(const DevCfg& c0, const BatchEntry* tbl, int nprob, long long total, int maxIter, int stage,
                            int mode, BatchState* bs, cudaStream_t s) {
   (void)c0;
   const int nb = persistent_blocks();
   cudaMemsetAsync(bs->listCount, 0, sizeof(bs->listCount), s);
-  k_batch_list_init<C, V><<<nb, 128, 0, s>>>(tbl, nprob, total, stage, bs);
+  k_batch_list_init<C, V, F><<<nb, 128, 0, s>>>(tbl, nprob, total, stage, bs);
   for (int it = 1; it <= maxIter; it++) {
     cudaMemsetAsync(&bs->listCount[it & 1], 0, sizeof(unsigned long long), s);
     if (mode == GRIM_NEWTON_MIXED32)
-      k_batch_list_iter<C, V, float><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
+      k_batch_list_iter<C, V, F, float><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
     else
-      k_batch_list_iter<C, V, double><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
+      k_batch_list_iter<C, V, F, double><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
   }
 }
 void batch_newton(const DevCfg& c0, const BatchEntry* tbl, int nprob, long long total, int maxIter, int stage,
                   int mode, BatchState* bs, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c0, batch_newton_t, c0, tbl, nprob, total, maxIter, stage, mode, bs, s);
+  GRIM_GEO_DISPATCH(c0, batch_newton_t, c0, tbl, nprob, total, maxIter, stage, mode, bs, s);
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void residual_t(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* out,
                        cudaStream_t s) {
-  k_residual<C, V><<<nblk(c.Z, 128), 128, 0, s>>>(c, stage, b, pg, out);
+  k_residual<C, V, F><<<nblk(c.Z, 128), 128, 0, s>>>(c, stage, b, pg, out);
 }
 void residual(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* out, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, residual_t, c, stage, b, pg, out, s);
+  GRIM_GEO_DISPATCH(c, residual_t, c, stage, b, pg, out, s);
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void jacobian_t(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* jac, int tangent,
                        cudaStream_t s) {
-  k_jacobian<C, V><<<nblk(c.Z, 128), 128, 0, s>>>(c, stage, b, pg, jac, tangent);
+  k_jacobian<C, V, F><<<nblk(c.Z, 128), 128, 0, s>>>(c, stage, b, pg, jac, tangent);
 }
 void jacobian(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* jac, int tangent,
               cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, jacobian_t, c, stage, b, pg, jac, tangent, s);
+  GRIM_GEO_DISPATCH(c, jacobian_t, c, stage, b, pg, jac, tangent, s);
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void conserved_t(const DevCfg& c, const double* p, const double* geoC, double* out, int fdir, int dir,
                         double* mn, double* mx, cudaStream_t s) {
-  k_conserved<C, V><<<nblk(c.Z, 128), 128, 0, s>>>(c, p, geoC, out, fdir, dir, mn, mx);
+  k_conserved<C, V, F><<<nblk(c.Z, 128), 128, 0, s>>>(c, p, geoC, out, fdir, dir, mn, mx);
 }
 void conserved(const DevCfg& c, const double* p, const double* geoC, double* out, int fdir, int dir, double* mn,
                double* mx, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, conserved_t, c, p, geoC, out, fdir, dir, mn, mx, s);
+  GRIM_GEO_DISPATCH(c, conserved_t, c, p, geoC, out, fdir, dir, mn, mx, s);
 }
 void reconstruct(const DevCfg& c, int dir, const double* p, double* pl, double* pr, cudaStream_t s) {
   k_reconstruct<<<nblk(c.Z, 128), 128, 0, s>>>(c, dir, p, pl, pr);
@@ -2647,33 +2660,36 @@ static void torus_floor_t(const DevCfg& c, double* p, const double* geoC, const 
 void torus_floor(const DevCfg& c, double* p, const double* geoC, const unsigned long long* flag, cudaStream_t s) {
   GRIM_EMHD_DISPATCH(c, torus_floor_t, c, p, geoC, flag, s);
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void stage_finish_t(const DevCfg& c, const double* src, double* dst, const double* geoC, bool floors,
                            bool post, const unsigned long long* nanFlag, int dtOn, DevState* st, cudaStream_t s) {
   const TorusCfg t = torus_cfg(c);
   const unsigned nb = (unsigned)nblk(c.Z, 128);
-  if (floors && post)
-    k_stage_finish<C, V, true, true><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
-  else if (floors)
-    k_stage_finish<C, V, true, false><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
-  else if (post)
-    k_stage_finish<C, V, false, true><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
+  if constexpr (!F) {  // the torus floors: Kerr-Schild only
+    if (floors) {
+      if (post) k_stage_finish<C, V, F, true, true><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
+      else k_stage_finish<C, V, F, true, false><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
+      return;
+    }
+  }
+  if (post)
+    k_stage_finish<C, V, F, false, true><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
   else
-    k_stage_finish<C, V, false, false><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
+    k_stage_finish<C, V, F, false, false><<<nb, 128, 0, s>>>(c, t, src, dst, geoC, nanFlag, dtOn, st);
 }
 void stage_finish(const DevCfg& c, const double* src, double* dst, const double* geoC, bool floors, bool post,
                   const unsigned long long* nanFlag, int dtOn, DevState* st, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, stage_finish_t, c, src, dst, geoC, floors, post, nanFlag, dtOn, st, s);
+  GRIM_GEO_DISPATCH(c, stage_finish_t, c, src, dst, geoC, floors, post, nanFlag, dtOn, st, s);
 }
-template <int C, int V>
+template <int C, int V, bool F>
 static void torus_observe_t(const DevCfg& c, const double* p, const double* geoC, double volElem, double every,
                             DevState* st, double* partials, double* out, double* hist, int cap, cudaStream_t s) {
-  k_torus_obs_partial<C, V><<<kObsBlocks, 128, 0, s>>>(c, p, geoC, volElem, every, st, partials);
+  k_torus_obs_partial<C, V, F><<<kObsBlocks, 128, 0, s>>>(c, p, geoC, volElem, every, st, partials);
   k_torus_obs_final<<<1, 32, 0, s>>>(partials, kObsBlocks, every, st, out, hist, cap);
 }
 void torus_observe(const DevCfg& c, const double* p, const double* geoC, double volElem, double every, DevState* st,
                    double* partials, double* out, double* hist, int cap, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, torus_observe_t, c, p, geoC, volElem, every, st, partials, out, hist, cap, s);
+  GRIM_GEO_DISPATCH(c, torus_observe_t, c, p, geoC, volElem, every, st, partials, out, hist, cap, s);
 }
 void torus_nan_flag(const DevCfg& c, const double* p, unsigned long long* flag, cudaStream_t s) {
   k_nan_flag<<<nblk(c.Zint, 256), 256, 0, s>>>(c, p, flag);

@@ -79,7 +79,8 @@ namespace GRIM_KNS {
 //        epilogue centre work of one zone (element, conserved vector,
 //        geometric source contraction; CT and divergence not counted)};
 // the Jacobian is the closed form for ideal MHD and the forward tangent
-// otherwise
+// otherwise; the counts are the general metric's arithmetic also where the
+// step runs the Minkowski kernels
 template <int COND, int VISC>
 __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, double* out) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;

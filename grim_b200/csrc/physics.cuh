@@ -14,6 +14,7 @@ namespace grim {
 
 template <class R>
 struct ZoneGeo {
+  static constexpr bool flat = false;
   R gcov[4][4];
   R gcon[4][4];
   R g, alpha;
@@ -22,7 +23,52 @@ struct ZoneGeo {
   R dyn;     // x1^1.5 (torus closure)
 };
 
-// Minkowski at compile time; MKS from the stored per-location arrays
+// Minkowski as a type of its own: the element, the speeds, the residual and
+// the Jacobian drop the terms the metric's zeros and ones remove (adding a
+// zero and multiplying by one are exact, so the parity unit's results keep
+// the reference's bits; only the sign of a zero can differ).  A kernel
+// compiled for either metric holds no geometry array and runs a quarter to a
+// half of the general metric's FP64 instructions: with one kernel for both
+// metrics the 32 metric words stay live and every zero is multiplied.
+// Measured on one B200 (FP32-Jacobian Newton, us per step): Orszag-Tang
+// 512^2 WENO5/HLL 305 -> 240; 256^2 extended MHD, MP5/HLL
+// 363 -> 299.
+template <class R>
+struct FlatGeo {
+  static constexpr bool flat = true;
+  R g, alpha, ialpha;  // all one
+  R x1, x2;
+  R dyn;
+};
+template <bool FLAT, class R> struct GeoSel { typedef ZoneGeo<R> type; };
+template <class R> struct GeoSel<true, R> { typedef FlatGeo<R> type; };
+template <bool FLAT, class R> using Geo = typename GeoSel<FLAT, R>::type;
+
+// a^m lowered: g_mn a^n
+template <class R, class S>
+GRIM_D S lower(const ZoneGeo<R>& G, int m, const S* a) {
+  return G.gcov[m][0] * a[0] + G.gcov[m][1] * a[1] + G.gcov[m][2] * a[2] + G.gcov[m][3] * a[3];
+}
+template <class R, class S>
+GRIM_D S lower(const FlatGeo<R>&, int m, const S* a) {
+  return m == 0 ? -a[0] : a[m];
+}
+// the geometry in another precision (the FP32 Jacobian's)
+template <class T>
+GRIM_D void convert_geo(ZoneGeo<T>& Gt, const ZoneGeo<double>& G) {
+#pragma unroll
+  for (int m = 0; m < 4; m++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = (T)G.gcov[m][q]; Gt.gcon[m][q] = (T)G.gcon[m][q]; }
+  Gt.g = (T)G.g; Gt.alpha = (T)G.alpha; Gt.ialpha = (T)G.ialpha; Gt.x1 = (T)G.x1; Gt.x2 = (T)G.x2; Gt.dyn = (T)G.dyn;
+}
+template <class T>
+GRIM_D void convert_geo(FlatGeo<T>& Gt, const FlatGeo<double>& G) {
+  Gt.g = T(1); Gt.alpha = T(1); Gt.ialpha = T(1);
+  Gt.x1 = (T)G.x1; Gt.x2 = (T)G.x2; Gt.dyn = T(0);
+}
+
+// The general form at run time; MKS from the stored per-location arrays
 // (layout, SoA: 16 gCov, 16 gCon, g, alpha, then the auxiliary fields
 // x1, x2, x1^1.5, rhoFloor(x1), uFloor(x1) -> 39 words per zone).  The last
 // three depend on the geometry only and are evaluated once: the torus
@@ -87,6 +133,13 @@ GRIM_D void load_geo(ZoneGeo<R>& G, const DevCfg& c, const double* geo, long lon
   else
     geo_load<R>(G, geo, c.GZ, gidx(c, i, j));
 }
+template <class R>
+GRIM_D void load_geo(FlatGeo<R>& G, const DevCfg& c, const double*, long long, int i, int j, double o1, double o2) {
+  G.g = R(1); G.alpha = R(1); G.ialpha = R(1);
+  G.x1 = (R)zone_x1(c, i, o1);
+  G.x2 = (R)zone_x2(c, j, o2);
+  G.dyn = R(0);
+}
 
 template <class S, class R>
 struct ElemT {
@@ -124,8 +177,8 @@ template <class T, int N>
 GRIM_HD Dual<T, N> dcube(const Dual<T, N>& a) { return a * a * a; }
 
 // setFluidElementParameters (problem hook) -- closures
-template <class S, class R>
-GRIM_D void closure(ElemT<S, R>& e, const ZoneGeo<R>& G, const DevCfg& c) {
+template <class S, class R, class GT>
+GRIM_D void closure(ElemT<S, R>& e, const GT& G, const DevCfg& c) {
   const S cs = e.soundSpeed;
   if (c.closure == GRIM_CLOSURE_CONST_TAU) {
     // linear_modes/problem.cpp:3-8
@@ -172,10 +225,10 @@ GRIM_D void closure(ElemT<S, R>& e, const ZoneGeo<R>& G, const DevCfg& c) {
 
 // fluidElement::set (physics.cpp:53-183) minus T^mu_nu, which callers take
 // row by row with tmunu().
-template <int COND, int VISC, class S, class R>
+template <int COND, int VISC, class S, class R, class GT>
 GRIM_D void elem_set(ElemT<S, R>& e, const S& rho_in, const S& u_in, const S& v1, const S& v2,
                      const S& v3, R B1, R B2, R B3, const S& qT, const S& dPT,
-                     const ZoneGeo<R>& G, const DevCfg& c) {
+                     const GT& G, const DevCfg& c) {
   typedef typename Real<S>::type T;
   const T Gam = (T)c.Gam;
   e.rho = dmaxc(rho_in, (T)c.rhoFloor);
@@ -185,43 +238,72 @@ GRIM_D void elem_set(ElemT<S, R>& e, const S& rho_in, const S& u_in, const S& v1
   e.pressure = (Gam - T(1.)) * e.u;
   e.temperature = dmaxc(e.pressure / e.rho, (T)c.TFloor);
   e.soundSpeed = dsqrt(Gam * e.pressure / (e.rho + Gam * e.u));
+  if constexpr (GT::flat) {
 #ifdef GRIM_FAST_MATH
-  // gamma and 1 / gamma from one reciprocal square root: u^0 = gamma / alpha
-  // and 1 / u^0 = alpha / gamma without divisions
-  const S gsq = T(1) + G.gcov[1][1] * v1 * v1 + G.gcov[2][2] * v2 * v2 + G.gcov[3][3] * v3 * v3 +
-                T(2) * (G.gcov[1][2] * v1 * v2 + G.gcov[1][3] * v1 * v3 + G.gcov[2][3] * v2 * v3);
-  const S rgam = drsqrt(gsq);
-  e.gam = gsq * rgam;
-  e.uCon[0] = e.gam * G.ialpha;
+    const S gsq = T(1) + v1 * v1 + v2 * v2 + v3 * v3;
+    const S rgam = drsqrt(gsq);  // 0 at an infinite velocity: gamma is then NaN, as every row below
+    e.gam = gsq * rgam;
+    e.uCon[0] = e.gam;
 #else
-  e.gam = dsqrt(T(1) + G.gcov[1][1] * v1 * v1 + G.gcov[2][2] * v2 * v2 + G.gcov[3][3] * v3 * v3 +
-                T(2) * (G.gcov[1][2] * v1 * v2 + G.gcov[1][3] * v1 * v3 + G.gcov[2][3] * v2 * v3));
-  e.uCon[0] = e.gam / G.alpha;
+    e.gam = dsqrt(T(1) + v1 * v1 + v2 * v2 + v3 * v3);
+    // an infinite gamma makes every component NaN, as the metric's zeros do
+    // in the general form; a finite one is unchanged
+    e.uCon[0] = e.gam + T(0) * e.gam;
 #endif
-  e.uCon[1] = v1 - e.gam * G.gcon[0][1] * G.alpha;
-  e.uCon[2] = v2 - e.gam * G.gcon[0][2] * G.alpha;
-  e.uCon[3] = v3 - e.gam * G.gcon[0][3] * G.alpha;
-#pragma unroll
-  for (int mu = 0; mu < 4; mu++)
-    e.uCov[mu] = G.gcov[mu][0] * e.uCon[0] + G.gcov[mu][1] * e.uCon[1] + G.gcov[mu][2] * e.uCon[2] +
-                 G.gcov[mu][3] * e.uCon[3];
-  e.bCon[0] = B1 * e.uCov[1] + B2 * e.uCov[2] + B3 * e.uCov[3];
+    e.uCon[1] = v1; e.uCon[2] = v2; e.uCon[3] = v3;
+    e.uCov[0] = -e.uCon[0];
+    e.uCov[1] = v1; e.uCov[2] = v2; e.uCov[3] = v3;
+    e.bCon[0] = B1 * v1 + B2 * v2 + B3 * v3;
 #ifdef GRIM_FAST_MATH
-  {
-    const S iu0 = G.alpha * rgam;  // 1 / u^0
-    e.bCon[1] = (B1 + e.bCon[0] * e.uCon[1]) * iu0;
-    e.bCon[2] = (B2 + e.bCon[0] * e.uCon[2]) * iu0;
-    e.bCon[3] = (B3 + e.bCon[0] * e.uCon[3]) * iu0;
+    e.bCon[1] = (B1 + e.bCon[0] * v1) * rgam;
+    e.bCon[2] = (B2 + e.bCon[0] * v2) * rgam;
+    e.bCon[3] = (B3 + e.bCon[0] * v3) * rgam;
+#else
+    e.bCon[1] = (B1 + e.bCon[0] * v1) / e.uCon[0];
+    e.bCon[2] = (B2 + e.bCon[0] * v2) / e.uCon[0];
+    e.bCon[3] = (B3 + e.bCon[0] * v3) / e.uCon[0];
+#endif
+    e.bCov[0] = -e.bCon[0];
+    e.bCov[1] = e.bCon[1]; e.bCov[2] = e.bCon[2]; e.bCov[3] = e.bCon[3];
+  } else {
+#ifdef GRIM_FAST_MATH
+    // gamma and 1 / gamma from one reciprocal square root: u^0 = gamma / alpha
+    // and 1 / u^0 = alpha / gamma without divisions
+    const S gsq = T(1) + G.gcov[1][1] * v1 * v1 + G.gcov[2][2] * v2 * v2 + G.gcov[3][3] * v3 * v3 +
+                  T(2) * (G.gcov[1][2] * v1 * v2 + G.gcov[1][3] * v1 * v3 + G.gcov[2][3] * v2 * v3);
+    const S rgam = drsqrt(gsq);
+    e.gam = gsq * rgam;
+    e.uCon[0] = e.gam * G.ialpha;
+#else
+    e.gam = dsqrt(T(1) + G.gcov[1][1] * v1 * v1 + G.gcov[2][2] * v2 * v2 + G.gcov[3][3] * v3 * v3 +
+                  T(2) * (G.gcov[1][2] * v1 * v2 + G.gcov[1][3] * v1 * v3 + G.gcov[2][3] * v2 * v3));
+    e.uCon[0] = e.gam / G.alpha;
+#endif
+    e.uCon[1] = v1 - e.gam * G.gcon[0][1] * G.alpha;
+    e.uCon[2] = v2 - e.gam * G.gcon[0][2] * G.alpha;
+    e.uCon[3] = v3 - e.gam * G.gcon[0][3] * G.alpha;
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++)
+      e.uCov[mu] = G.gcov[mu][0] * e.uCon[0] + G.gcov[mu][1] * e.uCon[1] + G.gcov[mu][2] * e.uCon[2] +
+                   G.gcov[mu][3] * e.uCon[3];
+    e.bCon[0] = B1 * e.uCov[1] + B2 * e.uCov[2] + B3 * e.uCov[3];
+#ifdef GRIM_FAST_MATH
+    {
+      const S iu0 = G.alpha * rgam;  // 1 / u^0
+      e.bCon[1] = (B1 + e.bCon[0] * e.uCon[1]) * iu0;
+      e.bCon[2] = (B2 + e.bCon[0] * e.uCon[2]) * iu0;
+      e.bCon[3] = (B3 + e.bCon[0] * e.uCon[3]) * iu0;
+    }
+#else
+    e.bCon[1] = (B1 + e.bCon[0] * e.uCon[1]) / e.uCon[0];
+    e.bCon[2] = (B2 + e.bCon[0] * e.uCon[2]) / e.uCon[0];
+    e.bCon[3] = (B3 + e.bCon[0] * e.uCon[3]) / e.uCon[0];
+#endif
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++)
+      e.bCov[mu] = G.gcov[mu][0] * e.bCon[0] + G.gcov[mu][1] * e.bCon[1] + G.gcov[mu][2] * e.bCon[2] +
+                   G.gcov[mu][3] * e.bCon[3];
   }
-#else
-  e.bCon[1] = (B1 + e.bCon[0] * e.uCon[1]) / e.uCon[0];
-  e.bCon[2] = (B2 + e.bCon[0] * e.uCon[2]) / e.uCon[0];
-  e.bCon[3] = (B3 + e.bCon[0] * e.uCon[3]) / e.uCon[0];
-#endif
-#pragma unroll
-  for (int mu = 0; mu < 4; mu++)
-    e.bCov[mu] = G.gcov[mu][0] * e.bCon[0] + G.gcov[mu][1] * e.bCon[1] + G.gcov[mu][2] * e.bCon[2] +
-                 G.gcov[mu][3] * e.bCon[3];
   e.bSqr = e.bCon[0] * e.bCov[0] + e.bCon[1] * e.bCov[1] + e.bCon[2] * e.bCov[2] +
            e.bCon[3] * e.bCov[3] + (T)c.bSqrFloor;
   e.bNorm = dsqrt(e.bSqr);
@@ -278,8 +360,8 @@ GRIM_D void fluxes_B(const ElemT<S, R>& e, int dir, R g, S* out3) {
 
 // computeMinMaxCharSpeeds (riemannsolver.cpp:54-200), dir = 0,1,2
 // (templated on the scalar for the op-counting build; double in the kernels)
-template <int COND, int VISC, class S, class R>
-GRIM_D void char_speeds(const ElemT<S, R>& e, const ZoneGeo<R>& G, int dir, const DevCfg& c, S& minSpeed,
+template <int COND, int VISC, class S, class R, class GT>
+GRIM_D void char_speeds(const ElemT<S, R>& e, const GT& G, int dir, const DevCfg& c, S& minSpeed,
                         S& maxSpeed) {
   const S Gam = S(c.Gam);
 #ifdef GRIM_FAST_MATH
@@ -318,14 +400,21 @@ GRIM_D void char_speeds(const ElemT<S, R>& e, const ZoneGeo<R>& G, int dir, cons
   csSqr = csSqr + cAlvenSqr - csSqr * cAlvenSqr;
   if (csSqr > S(1.)) csSqr = S(1.);
   const int s = dir + 1;
-  const S ASqr = G.gcon[s][s];
-  const S BSqr = G.gcon[0][0];
   const S ADotU = e.uCon[s];
   const S BDotU = e.uCon[0];
-  const S ADotB = G.gcon[s][0];
-  S A = (BDotU * BDotU) - (BSqr + BDotU * BDotU) * csSqr;
-  S B = S(2.) * (ADotU * BDotU - (ADotB + ADotU * BDotU) * csSqr);
-  S C = ADotU * ADotU - (ASqr + ADotU * ADotU) * csSqr;
+  S A, B, C;
+  if constexpr (GT::flat) {
+    A = (BDotU * BDotU) - (S(-1.) + BDotU * BDotU) * csSqr;
+    B = S(2.) * (ADotU * BDotU - ADotU * BDotU * csSqr);
+    C = ADotU * ADotU - (S(1.) + ADotU * ADotU) * csSqr;
+  } else {
+    const S ASqr = G.gcon[s][s];
+    const S BSqr = G.gcon[0][0];
+    const S ADotB = G.gcon[s][0];
+    A = (BDotU * BDotU) - (BSqr + BDotU * BDotU) * csSqr;
+    B = S(2.) * (ADotU * BDotU - (ADotB + ADotU * BDotU) * csSqr);
+    C = ADotU * ADotU - (ASqr + ADotU * ADotU) * csSqr;
+  }
   S discr = dsqrt(dmax2(B * B - S(4.) * A * C, S(1.e-16)));
 #ifdef GRIM_FAST_MATH
   const S i2a = S(0.5) / A;
@@ -355,8 +444,8 @@ GRIM_D void char_speeds(const ElemT<S, R>& e, const ZoneGeo<R>& G, int dir, cons
 // and a floored rho or u (af::max with the floor) has a zero column, as in
 // the forward tangent.  About a third of the flops of the 5-lane tangent.
 // ---------------------------------------------------------------------------
-template <class T, class KC>
-GRIM_D void ideal_jacobian(const double* P, const KC& K, const ZoneGeo<T>& G, const DevCfg& c, T J[5][5]) {
+template <class T, class KC, class GT>
+GRIM_D void ideal_jacobian(const double* P, const KC& K, const GT& G, const DevCfg& c, T J[5][5]) {
   const T Gam = (T)c.Gam;
   const T rhoIn = (T)P[0], uIn = (T)P[1];
   const T rhoF = (T)c.rhoFloor, uF = (T)c.uFloor;
@@ -368,7 +457,10 @@ GRIM_D void ideal_jacobian(const double* P, const KC& K, const ZoneGeo<T>& G, co
   const T B[3] = {(T)K.B[0], (T)K.B[1], (T)K.B[2]};
   T gv[3];
 #pragma unroll
-  for (int j = 0; j < 3; j++) gv[j] = G.gcov[j + 1][1] * v[0] + G.gcov[j + 1][2] * v[1] + G.gcov[j + 1][3] * v[2];
+  for (int j = 0; j < 3; j++) {
+    if constexpr (GT::flat) gv[j] = v[j];
+    else gv[j] = G.gcov[j + 1][1] * v[0] + G.gcov[j + 1][2] * v[1] + G.gcov[j + 1][3] * v[2];
+  }
   // gamma and 1 / gamma from one reciprocal square root
   const T gsq = T(1.) + v[0] * gv[0] + v[1] * gv[1] + v[2] * gv[2];
   const T rgam = drsqrt(gsq);
@@ -376,17 +468,18 @@ GRIM_D void ideal_jacobian(const double* P, const KC& K, const ZoneGeo<T>& G, co
   T uCon[4], uCov[4], bCon[4], bCov[4];
   uCon[0] = gam * G.ialpha;
 #pragma unroll
-  for (int i = 1; i < 4; i++) uCon[i] = v[i - 1] - gam * G.gcon[0][i] * G.alpha;
+  for (int i = 1; i < 4; i++) {
+    if constexpr (GT::flat) uCon[i] = v[i - 1];
+    else uCon[i] = v[i - 1] - gam * G.gcon[0][i] * G.alpha;
+  }
 #pragma unroll
-  for (int m = 0; m < 4; m++)
-    uCov[m] = G.gcov[m][0] * uCon[0] + G.gcov[m][1] * uCon[1] + G.gcov[m][2] * uCon[2] + G.gcov[m][3] * uCon[3];
+  for (int m = 0; m < 4; m++) uCov[m] = lower(G, m, uCon);
   const T iu0 = G.alpha * rgam;  // 1 / u^0
   bCon[0] = B[0] * uCov[1] + B[1] * uCov[2] + B[2] * uCov[3];
 #pragma unroll
   for (int i = 1; i < 4; i++) bCon[i] = (B[i - 1] + bCon[0] * uCon[i]) * iu0;
 #pragma unroll
-  for (int m = 0; m < 4; m++)
-    bCov[m] = G.gcov[m][0] * bCon[0] + G.gcov[m][1] * bCon[1] + G.gcov[m][2] * bCon[2] + G.gcov[m][3] * bCon[3];
+  for (int m = 0; m < 4; m++) bCov[m] = lower(G, m, bCon);
   const T bsq = bCon[0] * bCov[0] + bCon[1] * bCov[1] + bCon[2] * bCov[2] + bCon[3] * bCov[3] + (T)c.bSqrFloor;
   const T w = rho + u + p + bsq;
   const T gi = G.g / (T)K.dtp;  // sqrt(-g) / dt'
@@ -413,20 +506,32 @@ GRIM_D void ideal_jacobian(const double* P, const KC& K, const ZoneGeo<T>& G, co
     T du[4], duCov[4], db[4];
     du[0] = dg * G.ialpha;
 #pragma unroll
-    for (int i = 1; i < 4; i++) du[i] = ((i == j + 1) ? T(1.) : T(0.)) - dg * G.gcon[0][i] * G.alpha;
+    for (int i = 1; i < 4; i++) {
+      du[i] = (i == j + 1) ? T(1.) : T(0.);
+      if constexpr (!GT::flat) du[i] = du[i] - dg * G.gcon[0][i] * G.alpha;
+    }
 #pragma unroll
-    for (int m = 0; m < 4; m++)
-      duCov[m] = G.gcov[m][0] * du[0] + G.gcov[m][1] * du[1] + G.gcov[m][2] * du[2] + G.gcov[m][3] * du[3];
-    db[0] = B[0] * duCov[1] + B[1] * duCov[2] + B[2] * duCov[3];
+    for (int m = 0; m < 4; m++) duCov[m] = lower(G, m, du);
+    if constexpr (GT::flat) db[0] = B[j];
+    else db[0] = B[0] * duCov[1] + B[1] * duCov[2] + B[2] * duCov[3];
 #pragma unroll
-    for (int i = 1; i < 4; i++) db[i] = (db[0] * uCon[i] + bCon[0] * du[i] - bCon[i] * du[0]) * iu0;
+    for (int i = 1; i < 4; i++) {
+      if constexpr (GT::flat) {
+        db[i] = db[0] * uCon[i] - bCon[i] * du[0];
+        if (i == j + 1) db[i] = db[i] + bCon[0];
+        db[i] = db[i] * iu0;
+      } else {
+        db[i] = (db[0] * uCon[i] + bCon[0] * du[i] - bCon[i] * du[0]) * iu0;
+      }
+    }
     const T dbsq = T(2.) * (bCov[0] * db[0] + bCov[1] * db[1] + bCov[2] * db[2] + bCov[3] * db[3]);
     T dT[4];
 #pragma unroll
     for (int n = 0; n < 4; n++) {
-      const T dbCov = G.gcov[n][0] * db[0] + G.gcov[n][1] * db[1] + G.gcov[n][2] * db[2] + G.gcov[n][3] * db[3];
-      dT[n] = dbsq * uCon[0] * uCov[n] + w * (du[0] * uCov[n] + uCon[0] * duCov[n]) -
-              (db[0] * bCov[n] + bCon[0] * dbCov);
+      const T dbCov = lower(G, n, db);
+      T dw = du[0] * uCov[n];
+      if (!GT::flat || n == 0 || n == j + 1) dw = dw + uCon[0] * duCov[n];  // flat: u_n, n > 0, is v^n itself
+      dT[n] = dbsq * uCon[0] * uCov[n] + w * dw - (db[0] * bCov[n] + bCon[0] * dbCov);
     }
     dT[0] = dT[0] + T(0.5) * dbsq;
     const T d0 = gi * rho * du[0];
@@ -474,8 +579,8 @@ GRIM_D double newton_tol(const DevCfg& c, double l2first, const K_& K) {
   return fmax(fmax(c.atol, c.rtol * c.rtol * l2first), K.tolFloor2);
 }
 
-template <int COND, int VISC, class S, class R>
-GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, const ZoneGeo<R>& G,
+template <int COND, int VISC, class S, class R, class GT>
+GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, const GT& G,
                           const DevCfg& c, S* Rout) {
   typedef typename Real<S>::type T;
   constexpr int NF = 5 + COND + VISC;
@@ -510,7 +615,13 @@ GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, cons
     for (int mu = 0; mu < 4; mu++) dtuCov[mu] = (e.uCov[mu] - (T)K.uCovOld[mu]) / dtp;
     S div = S(T(0.));
 #pragma unroll
-    for (int mu = 0; mu < 4; mu++) div = div + G.gcon[0][mu] * dtuCov[mu];
+    for (int mu = 0; mu < 4; mu++) {
+      if constexpr (GT::flat) {
+        if (mu == 0) div = -dtuCov[0];
+      } else {
+        div = div + G.gcon[0][mu] * dtuCov[mu];
+      }
+    }
     const T rr = (T)K.refRho, rnu = (T)K.refNu, rchi = (T)K.refChi, rtau = (T)K.refTau, rT = (T)K.refT;
     const T rbn = (T)K.refBNorm, rbs = (T)K.refBSqr;
     if (VISC) {

@@ -18,9 +18,8 @@ struct TorusCfg {
   double BsqrOverRhoMax, BsqrOverUMax;
 };
 
-template <int COND, int VISC>
-GRIM_D void load_elem(ElemT<double, double>& e, const DevCfg& c, const double* p, long long z,
-                      const ZoneGeo<double>& G) {
+template <int COND, int VISC, class GT>
+GRIM_D void load_elem(ElemT<double, double>& e, const DevCfg& c, const double* p, long long z, const GT& G) {
   const long long Z = c.Z;
   elem_set<COND, VISC>(e, p[z], p[Z + z], p[2 * Z + z], p[3 * Z + z], p[4 * Z + z], p[(long long)c.B1 * Z + z],
                        p[(long long)(c.B1 + 1) * Z + z], p[(long long)(c.B1 + 2) * Z + z],
@@ -29,8 +28,8 @@ GRIM_D void load_elem(ElemT<double, double>& e, const DevCfg& c, const double* p
 
 // the element of one zone's primitives q (rows: fluid, then B1..B3); S is
 // double, or the forward-tangent scalar of the adjoint's local Jacobians
-template <int COND, int VISC, class S>
-GRIM_D void elem_of(ElemT<S, S>& e, const DevCfg& c, const S* q, const ZoneGeo<S>& G) {
+template <int COND, int VISC, class S, class GT>
+GRIM_D void elem_of(ElemT<S, S>& e, const DevCfg& c, const S* q, const GT& G) {
   constexpr int NFT = 5 + COND + VISC;
   elem_set<COND, VISC>(e, q[RHO], q[UU], q[U1], q[U2], q[U3], q[NFT], q[NFT + 1], q[NFT + 2], COND ? q[5] : S(0.),
                        VISC ? q[5 + COND] : S(0.), G, c);
