@@ -864,6 +864,9 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
 #pragma unroll
   for (int v = 0; v < NF; v++) S[v] = 0.;
   constexpr bool needS = !FLAT || COND || VISC;
+  // fast path, extended MHD: Gamma^la_(ka nu) u_la (symmetric), formed from
+  // the connection words the geometric source loads
+  [[maybe_unused]] double gu0[4][4];
   if constexpr (!FLAT) {
     double T[4][4];
 #pragma unroll
@@ -881,9 +884,11 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
         for (int ka = 0; ka < 4; ka++)
 #pragma unroll
           for (int nu = ka; nu < 4; nu++) {
-            const double gv = G.g * __ldg(gam + (long long)(la * 16 + ka * 4 + nu) * c.GZ);
+            const double gw = __ldg(gam + (long long)(la * 16 + ka * 4 + nu) * c.GZ);
+            const double gv = G.g * gw;
             acc[nu] -= T[ka][la] * gv;
             if (nu != ka) acc[ka] -= T[nu][la] * gv;
+            if constexpr (COND || VISC) gu0[ka][nu] = (la == 0) ? gw * e.uCov[0] : gu0[ka][nu] + gw * e.uCov[la];
           }
 #pragma unroll
       for (int nu = 0; nu < 4; nu++) S[UU + nu] = acc[nu];
@@ -915,7 +920,10 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
       gu[1][mu] = st(mu, 0, c.dX[0]);
       gu[2][mu] = (c.dim > 1) ? st(mu, 1, c.dX[1]) : 0.;
       gu[3][mu] = (c.dim > 2) ? st(mu, 2, c.dX[2]) : 0.;
-      if constexpr (!FLAT) {
+      if constexpr (!FLAT && kFastMath) {
+#pragma unroll
+        for (int nu = 0; nu < 4; nu++) gu[nu][mu] -= nu <= mu ? gu0[nu][mu] : gu0[mu][nu];
+      } else if constexpr (!FLAT) {
 #pragma unroll
         for (int nu = 0; nu < 4; nu++)
 #pragma unroll
@@ -940,6 +948,35 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
 #pragma unroll
         for (int nu = 0; nu < 4; nu++) dv += G.gcon[mu][nu] * gu[mu][nu];
     }
+#ifdef GRIM_FAST_MATH
+    // the common factors outside the sums; h^mu = b^nu D_mu u_nu serves both
+    const double igt = G.g / e.tau;
+    double h[4];
+#pragma unroll
+    for (int mu = FLAT ? 1 : 0; mu < 4; mu++)
+      h[mu] = e.bCon[0] * gu[mu][0] + e.bCon[1] * gu[mu][1] + e.bCon[2] * gu[mu][2] + e.bCon[3] * gu[mu][3];
+    if (VISC) {
+      double bh = 0.;
+#pragma unroll
+      for (int mu = FLAT ? 1 : 0; mu < 4; mu++) bh += e.bCon[mu] * h[mu];
+      const double rn = e.rho * e.nu;
+      double s = -igt * rn * (3. * bh * e.ibSqr - dv);
+      if (c.hoVisc == 1) s = s * sqrt(e.tau / (rn * e.temperature)) - 0.5 * G.g * dv * e.deltaPTilde;
+      S[5 + COND] = s;
+    }
+    if (COND) {
+      double x = 0., y = 0.;
+#pragma unroll
+      for (int mu = FLAT ? 1 : 0; mu < 4; mu++) {
+        x += e.bCon[mu] * gT[mu];
+        y += e.uCon[mu] * h[mu];
+      }
+      const double rc = e.rho * e.chi;
+      double s = igt * rc * e.ibNorm * (x + e.temperature * y);
+      if (c.hoCond == 1) s = s * (sqrt(e.tau / rc) / e.temperature) - 0.5 * G.g * dv * e.qTilde;
+      S[5] = s;
+    }
+#else
     if (VISC) {
       double d0 = -dv * e.rho * e.nu;
 #pragma unroll
@@ -949,7 +986,7 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
       double d0t = (c.hoVisc == 1) ? d0 * sqrt(e.tau / e.rho / e.nu / e.temperature) : d0;
       double s = -G.g * (d0t) / e.tau;
       if (c.hoVisc == 1) s -= 0.5 * G.g * dv * e.deltaPTilde;
-      S[c.DP] = s;
+      S[5 + COND] = s;
     }
     if (COND) {
       double qq = 0.;
@@ -962,8 +999,9 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
       double qt = (c.hoCond == 1) ? qq * sqrt(e.tau / e.rho / e.chi) / e.temperature : qq;
       double s = -G.g * (qt) / e.tau;
       if (c.hoCond == 1) s -= 0.5 * G.g * dv * e.qTilde;
-      S[c.Q] = s;
+      S[5] = s;
     }
+#endif
   }
   // ---- outputs: stage constants for the Newton kernels
   if (needS)
@@ -1303,6 +1341,50 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
                            ph[(long long)(c.B1 + 2) * Z + z], COND ? ph[(long long)c.Q * Z + z] : 0.,
                            VISC ? ph[(long long)c.DP * Z + z] : 0., G, c);
     }
+#ifdef GRIM_FAST_MATH
+    // the q and deltaP rows' coefficients (see StageConst): with
+    // d_mu = (u_mu - uOld_mu) / dt', div = g^0mu d_mu,
+    //   deltaP: -sqrt(-g) f / tau (-rho nu div + 3 rho nu b^0 b^mu / b^2 d_mu)
+    //           - sqrt(-g) deltaP~ div / 2,      f = sqrt(tau / (rho nu T))
+    //   q:      sqrt(-g) f / tau rho chi / |b| (b^0 (T - TOld) / dt' + T u^0 b^mu d_mu)
+    //           - sqrt(-g) q~ div / 2,           f = sqrt(tau / (rho chi)) / T
+    // (without high-order terms f = 1 and no div / 2 term), and half of the
+    // implicit sources sqrt(-g) x~ / tau of the old and the new state
+    const double gt = G.g / er.tau;
+    double g0[4];
+    if constexpr (GT::flat) {
+      g0[0] = -1.; g0[1] = g0[2] = g0[3] = 0.;
+    } else {
+#pragma unroll
+      for (int m = 0; m < 4; m++) g0[m] = G.gcon[0][m];
+    }
+    K.rowT = 0.;
+    if (COND) {
+      const double norm = (c.hoCond) ? er.temperature * sqrt(er.rho * er.chi * er.tau) : er.tau;
+      const double f = (c.hoCond == 1) ? sqrt(er.tau / (er.rho * er.chi)) / er.temperature : 1.;
+      const double half = (c.hoCond == 1) ? 0.5 * G.g * er.qTilde : 0.;
+      const double s = gt * f * er.rho * er.chi * er.ibNorm, ni = norm * K.idtp;
+      K.rowU[0] = ni;
+      K.rowP[0] = 0.5 * gt * norm;
+      K.rowK[0] = (K.Kc[5] + 0.5 * gt * eo.qTilde) * norm;
+      K.rowT = s * er.bCon[0] * ni;
+#pragma unroll
+      for (int m = 0; m < 4; m++)
+        K.rowA[0][m] = (s * er.temperature * er.uCon[0] * er.bCon[m] - half * g0[m]) * ni;
+    }
+    if (VISC) {
+      const double norm = (c.hoVisc) ? sqrt(er.rho * er.nu * er.temperature * er.tau) : er.tau;
+      const double f = (c.hoVisc == 1) ? sqrt(er.tau / (er.rho * er.nu * er.temperature)) : 1.;
+      const double half = (c.hoVisc == 1) ? 0.5 * G.g * er.deltaPTilde : 0.;
+      const double s = gt * f * er.rho * er.nu, ni = norm * K.idtp;
+      const double sb = 3. * s * er.bCon[0] * er.ibSqr;
+      K.rowU[1] = ni;
+      K.rowP[1] = 0.5 * gt * norm;
+      K.rowK[1] = (K.Kc[5 + COND] + 0.5 * gt * eo.deltaPTilde) * norm;
+#pragma unroll
+      for (int m = 0; m < 4; m++) K.rowA[1][m] = ((s - half) * g0[m] - sb * er.bCon[m]) * ni;
+    }
+#else
     K.refRho = er.rho; K.refNu = VISC ? er.nu : 0.; K.refChi = COND ? er.chi : 0.;
     K.refTau = er.tau; K.refT = er.temperature;
 #pragma unroll
@@ -1316,6 +1398,7 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
     // residual normalisation (residual.cpp:291-323, :366-399)
     if (COND) K.normQ = (c.hoCond) ? er.temperature * sqrt(er.rho * er.chi * er.tau) : er.tau;
     if (VISC) K.normDP = (c.hoVisc) ? sqrt(er.rho * er.nu * er.temperature * er.tau) : er.tau;
+  #endif
   }
 }
 

@@ -147,6 +147,12 @@ struct ElemT {
   R B1, B2, B3;
   S uCon[4], uCov[4], bCon[4], bCov[4], bSqr, bNorm;
   S qTilde, deltaPTilde, q, deltaP, tau, chi, nu;
+#ifdef GRIM_FAST_MATH
+  // extended MHD, fast path: 1 / |b|, 1 / b^2, c_s^2, chi / tau and nu / tau
+  // (each closure sets chi and nu to a multiple of tau; the speeds need the
+  // multiple only, so a face evaluates none of the closure's exponentials)
+  S ibNorm, ibSqr, csSqr, chiTau, nuTau;
+#endif
 };
 
 // --- scalar helpers for the torus closure ---------------------------------
@@ -179,24 +185,39 @@ GRIM_HD Dual<T, N> dcube(const Dual<T, N>& a) { return a * a * a; }
 // setFluidElementParameters (problem hook) -- closures
 template <class S, class R, class GT>
 GRIM_D void closure(ElemT<S, R>& e, const GT& G, const DevCfg& c) {
+#ifdef GRIM_FAST_MATH
+  const S cs2 = e.csSqr;
+#else
   const S cs = e.soundSpeed;
+  const S cs2 = cs * cs;
+#endif
   if (c.closure == GRIM_CLOSURE_CONST_TAU) {
     // linear_modes/problem.cpp:3-8
     e.tau = Lift<S>::of(c.tau0);
-    e.chi = cs * cs * e.tau;
-    e.nu = cs * cs * e.tau;
+    e.chi = cs2 * e.tau;
+    e.nu = cs2 * e.tau;
+#ifdef GRIM_FAST_MATH
+    e.chiTau = e.nuTau = cs2;
+#endif
   } else if (c.closure == GRIM_CLOSURE_TAU_PROFILE) {
     R s = (G.x2 - (R)c.X2Start) / ((R)c.X2End - (R)c.X2Start);
     e.tau = Lift<S>::of((double)val_of((R)c.tau0 + ((R)c.tau1 - (R)c.tau0) * s));
-    e.chi = cs * cs * e.tau;
-    e.nu = cs * cs * e.tau;
+    e.chi = cs2 * e.tau;
+    e.nu = cs2 * e.tau;
+#ifdef GRIM_FAST_MATH
+    e.chiTau = e.nuTau = cs2;
+#endif
   } else {
     // torus/problem.cpp:7-55
     typedef typename Real<S>::type T;
     const T Dyn = (T)val_of(G.dyn);
     S t = Lift<S>::of((double)Dyn);
     if (c.conduction) {
+#ifdef GRIM_FAST_MATH
+      S Qmax = (T)c.CondClosure * e.rho * (cs2 * dsqrt(cs2));
+#else
       S Qmax = (T)c.CondClosure * e.rho * dcube(cs);
+#endif
       const T lambda = (T)0.01;
       S yCon = dfabs(e.q) / Qmax;
       yCon = dexp(-(yCon - T(1.)) / lambda);
@@ -217,9 +238,17 @@ GRIM_D void closure(ElemT<S, R>& e, const GT& G, const DevCfg& c) {
       t = dmin2(t, Dyn * fdVis);
     }
     e.tau = t;
+#ifdef GRIM_FAST_MATH
+    const S maxAlpha = (T(1.) - cs2) / (T(2.) * cs2 + T(1.e-12));
+    e.chiTau = dmin2(maxAlpha, Lift<S>::of(c.CondAlpha)) * cs2;
+    e.nuTau = dmin2(maxAlpha, Lift<S>::of(c.ViscAlpha)) * cs2;
+    e.chi = e.chiTau * t;
+    e.nu = e.nuTau * t;
+#else
     S maxAlpha = (T(1.) - cs * cs) / (T(2.) * cs * cs + T(1.e-12));
     e.chi = dmin2(maxAlpha, Lift<S>::of(c.CondAlpha)) * cs * cs * t;
     e.nu = dmin2(maxAlpha, Lift<S>::of(c.ViscAlpha)) * cs * cs * t;
+#endif
   }
 }
 
@@ -237,7 +266,12 @@ GRIM_D void elem_set(ElemT<S, R>& e, const S& rho_in, const S& u_in, const S& v1
   e.B1 = B1; e.B2 = B2; e.B3 = B3;
   e.pressure = (Gam - T(1.)) * e.u;
   e.temperature = dmaxc(e.pressure / e.rho, (T)c.TFloor);
+#ifdef GRIM_FAST_MATH
+  e.csSqr = Gam * e.pressure / (e.rho + Gam * e.u);
+  e.soundSpeed = dsqrt(e.csSqr);
+#else
   e.soundSpeed = dsqrt(Gam * e.pressure / (e.rho + Gam * e.u));
+#endif
   if constexpr (GT::flat) {
 #ifdef GRIM_FAST_MATH
     const S gsq = T(1) + v1 * v1 + v2 * v2 + v3 * v3;
@@ -306,6 +340,23 @@ GRIM_D void elem_set(ElemT<S, R>& e, const S& rho_in, const S& u_in, const S& v1
   }
   e.bSqr = e.bCon[0] * e.bCov[0] + e.bCon[1] * e.bCov[1] + e.bCon[2] * e.bCov[2] +
            e.bCon[3] * e.bCov[3] + (T)c.bSqrFloor;
+#ifdef GRIM_FAST_MATH
+  if constexpr (COND || VISC) {
+    // |b|, 1 / |b| and 1 / b^2 from one reciprocal square root; c_s^2 in
+    // place of the squared square root
+    e.ibNorm = drsqrt(e.bSqr);
+    e.ibSqr = e.ibNorm * e.ibNorm;
+    e.bNorm = e.bSqr * e.ibNorm;
+    if (COND) {
+      e.qTilde = qT;
+      e.q = (c.hoCond == 1) ? qT * e.temperature * dsqrt(e.rho * (T)c.CondAlpha * e.csSqr) : qT;
+    }
+    if (VISC) {
+      e.deltaPTilde = dPT;
+      e.deltaP = (c.hoVisc == 1) ? dPT * dsqrt(e.temperature * e.rho * (T)c.ViscAlpha * e.csSqr) : dPT;
+    }
+  }
+#else
   e.bNorm = dsqrt(e.bSqr);
   const S cs = e.soundSpeed;
   if (COND) {
@@ -322,6 +373,7 @@ GRIM_D void elem_set(ElemT<S, R>& e, const S& rho_in, const S& u_in, const S& v1
     else
       e.deltaP = dPT;
   }
+#endif
   if constexpr (COND || VISC) closure(e, G, c);
 }
 
@@ -333,8 +385,13 @@ GRIM_D S tmunu(const ElemT<S, R>& e, int mu, int nu) {
   S w = e.rho + e.u + e.pressure + e.bSqr;
   S pt = e.pressure + T(0.5) * e.bSqr;
   S r = w * e.uCon[mu] * e.uCov[nu] + pt * d - e.bCon[mu] * e.bCov[nu];
+#ifdef GRIM_FAST_MATH
+  if (COND) r += e.q * e.ibNorm * (e.uCon[mu] * e.bCov[nu] + e.bCon[mu] * e.uCov[nu]);
+  if (VISC) r -= e.deltaP * (e.bCon[mu] * (e.bCov[nu] * e.ibSqr) - T(1. / 3.) * (d + e.uCon[mu] * e.uCov[nu]));
+#else
   if (COND) r += e.q / e.bNorm * (e.uCon[mu] * e.bCov[nu] + e.bCon[mu] * e.uCov[nu]);
   if (VISC) r += (-e.deltaP) * (e.bCon[mu] * e.bCov[nu] / e.bSqr - T(1. / 3.) * (d + e.uCon[mu] * e.uCov[nu]));
+#endif
   return r;
 }
 
@@ -371,7 +428,7 @@ GRIM_D void char_speeds(const ElemT<S, R>& e, const GT& G, int dir, const DevCfg
   S cAlvenSqr, csSqr;
   if constexpr (COND || VISC) {
     cAlvenSqr = e.bSqr / (e.rho + Gam * e.u + e.bSqr);
-    csSqr = e.soundSpeed * e.soundSpeed;
+    csSqr = e.csSqr;
   } else {
     const S w1 = e.rho + Gam * e.u, w2 = w1 + e.bSqr;
     const S r = S(1.) / (w1 * w2);
@@ -383,9 +440,14 @@ GRIM_D void char_speeds(const ElemT<S, R>& e, const GT& G, int dir, const DevCfg
   S csSqr = e.soundSpeed * e.soundSpeed;
 #endif
   S cVisSqr = S(0.);
-  if (VISC) cVisSqr = S(4.) / S(3.) / (e.rho + Gam * e.u) * e.rho * e.nu / e.tau;
   S cConSqr = S(0.);
+#ifdef GRIM_FAST_MATH
+  if (VISC) cVisSqr = S(4. / 3.) * e.rho * e.nuTau / (e.rho + Gam * e.u);
+  if (COND) cConSqr = (Gam - S(1.)) * e.chiTau;
+#else
+  if (VISC) cVisSqr = S(4.) / S(3.) / (e.rho + Gam * e.u) * e.rho * e.nu / e.tau;
   if (COND) cConSqr = (Gam - S(1.)) * e.chi / e.tau;
+#endif
 #ifdef GRIM_FAST_MATH
   // with no conduction the combination is (cs^2 + |cs^2|) / 2 = cs^2
   // (cs^2 >= 0: a square root of a square is the magnitude exactly)
@@ -563,9 +625,19 @@ struct StageConst {
   double sImpOldQ, sImpOldDP;  // 0.5*(...) partner of the implicit source
   double normQ, normDP;        // EMHD row normalisation
   double dtp;                  // dt' (dt/2 or dt)
-  // fast path, ideal MHD: R = U / dt' + Kc, Kc = divF + Sexp - Uold / dt'
+  // fast path: R = U / dt' + Kc, Kc = divF + Sexp - Uold / dt'
   double idtp;
   double Kc[NF];
+  // fast path, extended MHD: the q and deltaP rows are affine in U, the
+  // unknown itself, u_mu - u_mu(old) and T - T(old); everything else in them
+  // is fixed for the stage, so it is folded into these once per zone:
+  //   R_q  = rowU U_q + rowP q~  + rowK + sum_mu rowA_mu (u_mu - uOld_mu) + rowT (T - TOld)
+  // (row 0: q, row 1: deltaP, whose rowT is zero).  A residual then has no
+  // division or square root of these rows, and the FP32 tangent pass
+  // neither.  With the speeds' and the sources' divisions hoisted the same
+  // way (us per step, one B200): EMHD torus 96x64x32 1735 -> 915, 256^2
+  // stratified 299 -> 224.
+  double rowU[2], rowP[2], rowK[2], rowA[2][4], rowT;
   // square of the Newton test's rounding floor: (tolUlps eps max_v |Kc_v|)^2
   // over the conserved rows (|Kc_v| = |U_v| / dt' at the solution, the
   // residual's largest term), 0 when tolUlps = 0
@@ -597,9 +669,25 @@ GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, cons
     const T idtp = (T)K.idtp;
 #pragma unroll
     for (int v = 0; v < NF; v++) Rout[v] = U[v] * idtp + (T)K.Kc[v];
-    return;
+  } else {
+    const T idtp = (T)K.idtp;
+#pragma unroll
+    for (int v = 0; v < 5; v++) Rout[v] = U[v] * idtp + (T)K.Kc[v];
+    S du[4];
+#pragma unroll
+    for (int mu = 0; mu < 4; mu++) du[mu] = e.uCov[mu] - (T)K.uCovOld[mu];
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      if ((r == 0 && !COND) || (r == 1 && !VISC)) continue;
+      const int v = r == 0 ? Q : DP;
+      S x = U[v] * (T)K.rowU[r] + P[v] * (T)K.rowP[r] + (T)K.rowK[r];
+#pragma unroll
+      for (int mu = 0; mu < 4; mu++) x = x + du[mu] * (T)K.rowA[r][mu];
+      if (r == 0) x = x + (e.temperature - (T)K.TOld) * (T)K.rowT;
+      Rout[v] = x;
+    }
   }
-#endif
+#else
   const T dtp = (T)K.dtp;
 #pragma unroll
   for (int v = 0; v < NF; v++) {
@@ -648,6 +736,7 @@ GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, cons
       Rout[Q] = r * (T)K.normQ;
     }
   }
+#endif
 }
 
 }  // namespace grim
