@@ -35,6 +35,8 @@
 // atomics), so a gradient is the same bits run to run.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "launch.h"
 #include "physics.cuh"
 #include "recon.cuh"
@@ -146,15 +148,16 @@ GRIM_D void geo_const(ZoneGeo<D>& Gd, const ZoneGeo<double>& G) {
 
 // the element of one zone's primitives p in grid row order (fluid rows,
 // then B1..B3)
-template <int C, int V, class S>
-GRIM_D void elem_rows(ElemT<S, S>& e, const DevCfg& c, const S* p, const ZoneGeo<S>& G) {
+template <int C, int V, class S, class GT>
+GRIM_D void elem_rows(ElemT<S, S>& e, const DevCfg& c, const S* p, const GT& G) {
   constexpr int NF = 5 + C + V;
   elem_set<C, V>(e, p[0], p[1], p[2], p[3], p[4], p[NF], p[NF + 1], p[NF + 2], C ? p[5] : S(0.),
                  V ? p[5 + C] : S(0.), G, c);
 }
 
 // the centre geometry of zone z
-GRIM_D void centre_geo(const DevCfg& c, const double* geoC, long long z, ZoneGeo<double>& G) {
+template <class GT>
+GRIM_D void centre_geo(const DevCfg& c, const double* geoC, long long z, GT& G) {
   int i, j, k;
   zijk(c, z, i, j, k);
   load_geo(G, c, geoC, z, i, j, 0.5, 0.5);
@@ -162,15 +165,13 @@ GRIM_D void centre_geo(const DevCfg& c, const double* geoC, long long z, ZoneGeo
 
 // conserved fluid rows U (nf = 5) of one zone and their Jacobian with
 // respect to the 8 primitives (5 fluid, then B)
-GRIM_D void cons_jacobian(const DevCfg& c, const double* p, long long z, const ZoneGeo<double>& G0,
-                          double J[5][8]) {
+template <class GT>
+GRIM_D void cons_jacobian(const DevCfg& c, const double* p, long long z, const GT& G, double J[5][8]) {
   typedef Dual<double, 8> D;
   const long long Z = c.Z;
   D q[8];
   for (int v = 0; v < 5; v++) q[v] = D::var(p[(long long)v * Z + z], v);
   for (int v = 0; v < 3; v++) q[5 + v] = D::var(p[(long long)(c.B1 + v) * Z + z], 5 + v);
-  ZoneGeo<D> G;
-  geo_const(G, G0);
   ElemT<D, D> e;
   elem_set<0, 0>(e, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7], D(0.), D(0.), G, c);
   D U[5];
@@ -181,6 +182,7 @@ GRIM_D void cons_jacobian(const DevCfg& c, const double* p, long long z, const Z
 
 // Stage adjoint at the stage's solution P (interior zones): lam -> g (dL/d
 // divF, dof rows), ubar (+)= mu / dt', bacc (+)= beta
+template <bool FLAT>
 __global__ void k_stage(DevCfg c, const double* __restrict__ geoC, const double* __restrict__ P, double dtp,
                         const double* __restrict__ lam, double* __restrict__ g, double* __restrict__ ubar,
                         double* __restrict__ bacc, int accumulate) {
@@ -200,7 +202,7 @@ __global__ void k_stage(DevCfg c, const double* __restrict__ geoC, const double*
     }
     return;
   }
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   centre_geo(c, geoC, z, G);
   double J[5][8];
   cons_jacobian(c, P, z, G, J);
@@ -225,6 +227,7 @@ __global__ void k_stage(DevCfg c, const double* __restrict__ geoC, const double*
 }
 
 // out(P0) += dU/dP(P0)^T ubar + [0 ; bacc] (interior zones)
+template <bool FLAT>
 __global__ void k_cons(DevCfg c, const double* __restrict__ geoC, const double* __restrict__ P,
                        const double* __restrict__ ubar, const double* __restrict__ bacc, double* __restrict__ lam) {
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -235,7 +238,7 @@ __global__ void k_cons(DevCfg c, const double* __restrict__ geoC, const double* 
   for (int r = 0; r < 5; r++) any |= ubar[(long long)r * Z + z] != 0.;
   for (int k = 0; k < 3; k++) any |= bacc[(long long)k * Z + z] != 0.;
   if (!any) return;
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   centre_geo(c, geoC, z, G);
   double J[5][8];
   cons_jacobian(c, P, z, G, J);
@@ -265,12 +268,10 @@ __global__ void k_src_t(DevCfg c, const double* __restrict__ geoC, const double*
   zijk(c, z, i, j, k);
   ZoneGeo<double> G0;
   load_geo(G0, c, geoC, z, i, j, 0.5, 0.5);
-  ZoneGeo<D> G;
-  geo_const(G, G0);
   D q[DOF];
   for (int v = 0; v < DOF; v++) q[v] = D::var(P[(long long)v * Z + z], v);
   ElemT<D, D> e;
-  elem_rows<C, V>(e, c, q, G);
+  elem_rows<C, V>(e, c, q, G0);
   D T[4][4];
   for (int ka = 0; ka < 4; ka++)
     for (int la = 0; la < 4; la++) T[ka][la] = tmunu<C, V>(e, ka, la);
@@ -302,6 +303,7 @@ __global__ void k_div_t(DevCfg c, const double* __restrict__ g, double* __restri
   int i, j, k;
   zijk(c, z, i, j, k);
   const long long Z = c.Z;
+  const int v = (int)blockIdx.y;  // one row per block of threads
   for (int d = 0; d < c.dim; d++) {
     const int im = d == 0 ? i - 1 : i, jm = d == 1 ? j - 1 : j, km = d == 2 ? k - 1 : k;
     const bool in0 = is_interior(c, i, j, k), in1 = is_interior(c, im, jm, km);
@@ -310,11 +312,9 @@ __global__ void k_div_t(DevCfg c, const double* __restrict__ g, double* __restri
     // the torus flux filter zeroes every row of the faces at the poles
     // (problem.cpp:1243-1285): only the zone beside each pole face uses it
     const bool pole = c.problem == GRIM_PROBLEM_TORUS && d == 1 && (j == c.g2 || j == c.N2 + c.g2);
-    for (int v = 0; v < c.dof; v++) {
-      const double a = in1 ? g[(long long)v * Z + zm] : 0.;
-      const double b = in0 ? g[(long long)v * Z + z] : 0.;
-      Ft[((long long)d * c.dof + v) * Z + z] = pole ? 0. : (a - b) * idx;
-    }
+    const double a = in1 ? g[(long long)v * Z + zm] : 0.;
+    const double b = in0 ? g[(long long)v * Z + z] : 0.;
+    Ft[((long long)d * c.dof + v) * Z + z] = pole ? 0. : (a - b) * idx;
   }
 }
 
@@ -385,38 +385,85 @@ __global__ void k_ct_t_raw(DevCfg c, const double* __restrict__ ebar, double* __
   row(2, 2) = 0.;
 }
 
-// the Riemann flux of one face (riemannsolver.cpp:202-328) on any scalar
-template <int C, int V, class S>
-GRIM_D void riemann_flux(const DevCfg& c, int dir, const ZoneGeo<double>& G0, const S* pl, const S* pr, S* F) {
+// One tangent lane of the flux of a face (riemannsolver.cpp:202-328):
+// (dF / d state[lane]) . fb, the state on side LEFT (left) or right seeded
+// in its variable `lane` (ps), the other (po) plain values.  The rows enter
+// only through their products with fb, so five sums replace the flux
+// vectors; a row whose adjoint is zero is left out (its flux need not be
+// finite).
+template <int C, int V, int DIR, bool LEFT, class GT>
+GRIM_D double face_lane(const DevCfg& c, int x, const GT& G, const double* ps, const double* po, int lane,
+                        const double* fbIn) {
   constexpr int NF = 5 + C + V, DOF = NF + 3;
-  ZoneGeo<S> G;
-  geo_const(G, G0);
-  const int fd = dir + 1;
-  S FL[DOF], UL[DOF], FR[DOF], UR[DOF], mnL, mxL, mnR, mxR;
+  constexpr int fd = DIR + 1;  // at compile time: the element stays in registers
+  typedef Dual<double, 1> D;
+  double Uo[DOF], Fo[DOF], mno, mxo;
   {
-    ElemT<S, S> e;
-    elem_rows<C, V>(e, c, pl, G);
-    fluxes_fluid<C, V>(e, fd, G.g, FL, 5, 5 + C);
-    fluxes_B(e, fd, G.g, FL + NF);
-    fluxes_fluid<C, V>(e, 0, G.g, UL, 5, 5 + C);
-    fluxes_B(e, 0, G.g, UL + NF);
-    char_speeds<C, V>(e, G, dir, c, mnL, mxL);
+    ElemT<double, double> e;
+    elem_rows<C, V>(e, c, po, G);
+    fluxes_fluid<C, V>(e, fd, G.g, Fo, 5, 5 + C);
+    fluxes_B(e, fd, G.g, Fo + NF);
+    fluxes_fluid<C, V>(e, 0, G.g, Uo, 5, 5 + C);
+    fluxes_B(e, 0, G.g, Uo + NF);
+    char_speeds<C, V>(e, G, DIR, c, mno, mxo);
   }
-  {
-    ElemT<S, S> e;
-    elem_rows<C, V>(e, c, pr, G);
-    fluxes_fluid<C, V>(e, fd, G.g, FR, 5, 5 + C);
-    fluxes_B(e, fd, G.g, FR + NF);
-    fluxes_fluid<C, V>(e, 0, G.g, UR, 5, 5 + C);
-    fluxes_B(e, 0, G.g, UR + NF);
-    char_speeds<C, V>(e, G, dir, c, mnR, mxR);
+  D q[DOF];
+#pragma unroll
+  for (int v = 0; v < DOF; v++) {
+    q[v].v = ps[v];
+    q[v].d[0] = (v == lane) ? 1. : 0.;
   }
-  const S cmin = dmin2(mnL, mnR), cmax = dmax2(mxL, mxR);
-  if (c.riemann == GRIM_HLL) {
-    for (int v = 0; v < DOF; v++) F[v] = (cmax * FL[v] - cmin * FR[v] + cmin * cmax * (UR[v] - UL[v])) / (cmax - cmin);
+  ElemT<D, D> e;
+  elem_rows<C, V>(e, c, q, G);
+  D mns, mxs;
+  char_speeds<C, V>(e, G, DIR, c, mns, mxs);
+  // the argument order decides which state a tie follows: (left, right)
+  const D cmin = LEFT ? dmin2(mns, D(mno)) : dmin2(D(mno), mns);
+  const D cmax = LEFT ? dmax2(mxs, D(mxo)) : dmax2(D(mxo), mxs);
+  D Fs[DOF], Us[DOF];
+  fluxes_fluid<C, V>(e, 0, G.g, Us, 5, 5 + C);
+  fluxes_B(e, 0, G.g, Us + NF);
+  fluxes_fluid<C, V>(e, fd, G.g, Fs, 5, 5 + C);
+  fluxes_B(e, fd, G.g, Fs + NF);
+  const bool hll = c.riemann == GRIM_HLL;
+  const D cm = dmax2(cmax, -cmin);
+  double fb[DOF];
+#pragma unroll
+  for (int r = 0; r < DOF; r++) fb[r] = fbIn[r];
+  if constexpr (!GT::flat && DIR == 0) {
+    // the torus flux filter on the density flux of the inner / outer X1
+    // faces: min(F, 0) / max(F, 0), so its derivative is 1 or 0
+    if (c.problem == GRIM_PROBLEM_TORUS && (x == c.g1 || x == c.N1 + c.g1)) {
+      const double FL = LEFT ? Fs[0].v : Fo[0], FR = LEFT ? Fo[0] : Fs[0].v;
+      const double dU = LEFT ? Uo[0] - Us[0].v : Us[0].v - Uo[0];
+      const double F0 = hll ? (cmax.v * FL - cmin.v * FR + cmin.v * cmax.v * dU) / (cmax.v - cmin.v)
+                            : 0.5 * (FL + FR - cm.v * dU);
+      if ((x == c.g1 && F0 > 0.) || (x == c.N1 + c.g1 && F0 < 0.)) fb[0] = 0.;
+    }
+  }
+  double sFo = 0., sFs = 0., dFs = 0., sdU = 0., dUs = 0.;
+#pragma unroll
+  for (int r = 0; r < DOF; r++)
+    if (fb[r] != 0.) {
+      sFo += fb[r] * Fo[r];
+      sFs += fb[r] * Fs[r].v;
+      dFs += fb[r] * Fs[r].d[0];
+      sdU += fb[r] * (Uo[r] - Us[r].v);
+      dUs += fb[r] * Us[r].d[0];
+    }
+  if (!hll) {
+    const double j = cm.v * dUs - cm.d[0] * sdU;
+    return 0.5 * (LEFT ? dFs + j : dFs - j);
+  }
+  const D cc = cmin * cmax;
+  const double iw = 1. / (cmax.v - cmin.v), dw = cmax.d[0] - cmin.d[0];
+  const double j = cc.d[0] * sdU - cc.v * dUs;
+  if constexpr (LEFT) {
+    const double num = cmax.v * sFs - cmin.v * sFo + cc.v * sdU;
+    return (cmax.d[0] * sFs + cmax.v * dFs - cmin.d[0] * sFo + j - num * iw * dw) * iw;
   } else {
-    const S cm = dmax2(cmax, -cmin);
-    for (int v = 0; v < DOF; v++) F[v] = S(0.5) * (FL[v] + FR[v] - cm * (UR[v] - UL[v]));
+    const double num = cmax.v * sFo - cmin.v * sFs - cc.v * sdU;
+    return (cmax.d[0] * sFo - cmin.d[0] * sFs - cmin.v * dFs - j - num * iw * dw) * iw;
   }
 }
 
@@ -425,63 +472,69 @@ GRIM_D void riemann_flux(const DevCfg& c, int dir, const ZoneGeo<double>& G0, co
 // reconstructed states, gl = (dF/dpl)^T Fbar (pl: the right-face state of a)
 // and gr = (dF/dpr)^T Fbar (pr: the left-face state of b), into gface
 // (rows 0..dof-1 gl, dof..2 dof-1 gr; zero on the faces the stencil does
-// not use)
-template <int C, int V>
-__global__ void k_faces_t(DevCfg c, int dir, const double* __restrict__ geoF, const double* __restrict__ P,
-                          const double* __restrict__ Ft, double* __restrict__ gface) {
-  constexpr int DOF = 8 + C + V;
-  long long z = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (z >= c.Z) return;
-  int i, j, k;
-  zijk(c, z, i, j, k);
-  const int x = dir == 0 ? i : (dir == 1 ? j : k);
-  const int NT = dir == 0 ? c.N1T : (dir == 1 ? c.N2T : c.N3T);
+// not use).
+// A block takes 32 faces with one warp per variable: warp v reconstructs
+// variable v's two states into shared memory, then runs the tangent lane of
+// variable v on each side (one-lane tangents: the element, its fluxes and
+// the speeds fit in registers; the other state is plain values).  Bound by
+// FP64 latency at the occupancy of its registers (206 in 2D ideal MHD, one
+// block per SM).  One thread per face with all dof lanes together kept its
+// tangents in local memory and took 357 us per launch at 192^2, three
+// quarters of a gradient; a gradient through 10 steps there went from 22.8
+// to 7.7 ms with this split and the row-parallel gathers below.
+template <int C, int V, bool FLAT, int DIR>
+__global__ void __launch_bounds__(32 * (8 + C + V)) k_faces_t(DevCfg c, const double* __restrict__ geoF,
+                                                               const double* __restrict__ P,
+                                                               const double* __restrict__ Ft,
+                                                               double* __restrict__ gface) {
+  constexpr int DOF = 8 + C + V, dir = DIR;
+  __shared__ double sl[DOF][32], sr[DOF][32], sf[DOF][32];
+  const int t = threadIdx.x & 31, v = threadIdx.x >> 5;
+  const long long z = (long long)blockIdx.x * 32 + t;
   const long long Z = c.Z, s = stride_of(c, dir);
+  int i = 0, j = 0, k = 0, x = 0;
+  bool in = false;
+  double f = 0.;
+  if (z < Z) {
+    zijk(c, z, i, j, k);
+    x = dir == 0 ? i : (dir == 1 ? j : k);
+    const int NT = dir == 0 ? c.N1T : (dir == 1 ? c.N2T : c.N3T);
+    in = x >= 3 && x <= NT - 3;
+    if (in) f = Ft[((long long)dir * DOF + v) * Z + z];
+  }
+  sf[v][t] = f;
+  // the face states, where any of the face's adjoints is nonzero
+  const bool anyBlock = __syncthreads_or(f != 0.);
+  if (anyBlock && in) {
+    const double* a = P + (long long)v * Z + z;
+    double lo, ro, lo2, ro2;
+    recon_faces<double>(c.reconstruction, c.theta, a[-3 * s], a[-2 * s], a[-s], a[0], a[s], lo, ro);
+    recon_faces<double>(c.reconstruction, c.theta, a[-2 * s], a[-s], a[0], a[s], a[2 * s], lo2, ro2);
+    sl[v][t] = ro;
+    sr[v][t] = lo2;
+  }
+  __syncthreads();
+  if (z >= Z) return;
   double fb[DOF];
   bool any = false;
-  for (int v = 0; v < DOF; v++) {
-    fb[v] = (x < 3 || x > NT - 3) ? 0. : Ft[((long long)dir * c.dof + v) * Z + z];
-    any |= fb[v] != 0.;
+#pragma unroll
+  for (int r = 0; r < DOF; r++) {
+    fb[r] = sf[r][t];
+    any |= fb[r] != 0.;
   }
-  if (!any) {
-    for (int v = 0; v < 2 * DOF; v++) gface[(long long)v * Z + z] = 0.;
-    return;
+  double gl = 0., gr = 0.;
+  if (any) {
+    double pl[DOF], pr[DOF];
+#pragma unroll
+    for (int r = 0; r < DOF; r++) { pl[r] = sl[r][t]; pr[r] = sr[r][t]; }
+    // the face metric (the X3 faces of the axisymmetric metrics: the centre's)
+    Geo<FLAT, double> G;
+    load_geo(G, c, geoF, z, i, j, dir == 0 ? 0. : 0.5, dir == 1 ? 0. : 0.5);
+    gl = face_lane<C, V, DIR, true>(c, x, G, pl, pr, v, fb);
+    gr = face_lane<C, V, DIR, false>(c, x, G, pr, pl, v, fb);
   }
-  // the face states
-  double pl[DOF], pr[DOF];
-  for (int v = 0; v < DOF; v++) {
-    const double* a = P + (long long)v * Z;
-    double lo, ro, lo2, ro2;
-    recon_faces<double>(c.reconstruction, c.theta, a[z - 3 * s], a[z - 2 * s], a[z - s], a[z], a[z + s], lo, ro);
-    recon_faces<double>(c.reconstruction, c.theta, a[z - 2 * s], a[z - s], a[z], a[z + s], a[z + 2 * s], lo2, ro2);
-    pl[v] = ro;
-    pr[v] = lo2;
-  }
-  // the face metric (the X3 faces of the axisymmetric metrics: the centre's)
-  ZoneGeo<double> G;
-  load_geo(G, c, geoF, z, i, j, dir == 0 ? 0. : 0.5, dir == 1 ? 0. : 0.5);
-  // dF/dpl and dF/dpr, dof tangent lanes each
-  typedef Dual<double, DOF> D8;
-  for (int side = 0; side < 2; side++) {
-    D8 L[DOF], R[DOF], F[DOF];
-    for (int v = 0; v < DOF; v++) {
-      L[v] = side == 0 ? D8::var(pl[v], v) : D8(pl[v]);
-      R[v] = side == 1 ? D8::var(pr[v], v) : D8(pr[v]);
-    }
-    riemann_flux<C, V, D8>(c, dir, G, L, R, F);
-    // the torus flux filter on the density flux of the inner / outer X1
-    // faces: min(F, 0) / max(F, 0), so its derivative is 1 or 0
-    double fr0 = fb[0];
-    if (c.problem == GRIM_PROBLEM_TORUS && dir == 0 &&
-        ((x == c.g1 && F[0].v > 0.) || (x == c.N1 + c.g1 && F[0].v < 0.)))
-      fr0 = 0.;
-    for (int k2 = 0; k2 < DOF; k2++) {
-      double acc = fr0 * F[0].d[k2];
-      for (int r = 1; r < DOF; r++)
-        if (fb[r] != 0.) acc += fb[r] * F[r].d[k2];
-      gface[(long long)(side * DOF + k2) * Z + z] = acc;
-    }
-  }
+  gface[(long long)v * Z + z] = gl;
+  gface[(long long)(DOF + v) * Z + z] = gr;
 }
 
 // Reconstruction transpose along dir, as a gather: zone x collects, in a
@@ -491,6 +544,20 @@ __global__ void k_faces_t(DevCfg c, int dir, const double* __restrict__ geoF, co
 // (the right state of face y, adjoint gr), each times its derivative with
 // respect to x from a forward-tangent pass of y's reconstruction.  One
 // thread per zone and direction, so the sums are the same run to run.
+// One tangent lane per neighbour: only the derivative with respect to x is
+// used.
+template <int M>
+GRIM_D double recon_t_term(const DevCfg& c, const double* __restrict__ a, long long s, double gl, double gr) {
+  typedef Dual<double, 1> D;
+  D y[5], lo, ro;
+#pragma unroll
+  for (int m = 0; m < 5; m++) {
+    y[m] = D(a[(m - 2) * s]);
+    if (m == M) y[m].d[0] = 1.;
+  }
+  recon_faces<D>(c.reconstruction, c.theta, y[0], y[1], y[2], y[3], y[4], lo, ro);
+  return gl * ro.d[0] + gr * lo.d[0];
+}
 __global__ void k_recon_t(DevCfg c, int dir, const double* __restrict__ P, const double* __restrict__ gface,
                           double* __restrict__ q) {
   long long z = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -500,26 +567,28 @@ __global__ void k_recon_t(DevCfg c, int dir, const double* __restrict__ P, const
   const int x = dir == 0 ? i : (dir == 1 ? j : k);
   const int NT = dir == 0 ? c.N1T : (dir == 1 ? c.N2T : c.N3T);
   const long long Z = c.Z, s = stride_of(c, dir);
-  typedef Dual<double, 5> D5;
-  for (int v = 0; v < c.dof; v++) {
-    const double* a = P + (long long)v * Z;
-    double acc = 0.;
-    for (int m = 4; m >= 0; m--) {
-      // x is point m of the stencil of y = x + 2 - m
-      const int y = x + 2 - m;
-      if (y < 2 || y > NT - 3) continue;
-      const long long zy = z + (long long)(2 - m) * s;
-      const double gl = (y + 1 <= NT - 1) ? gface[(long long)v * Z + zy + s] : 0.;
-      const double gr = gface[(long long)(c.dof + v) * Z + zy];
-      if (gl == 0. && gr == 0.) continue;
-      D5 yb[5];
-      for (int mm = 0; mm < 5; mm++) yb[mm] = D5::var(a[zy + (mm - 2) * s], mm);
-      D5 lo, ro;
-      recon_faces<D5>(c.reconstruction, c.theta, yb[0], yb[1], yb[2], yb[3], yb[4], lo, ro);
-      acc += gl * ro.d[m] + gr * lo.d[m];
-    }
-    q[(long long)v * Z + z] += acc;
-  }
+  const int v = (int)blockIdx.y;  // one variable per block of threads
+  const double* a = P + (long long)v * Z + z;
+  const double* gL = gface + (long long)v * Z + z;
+  const double* gR = gface + (long long)(c.dof + v) * Z + z;
+  double acc = 0.;
+  // x is point m of the stencil of y = x + 2 - m
+  auto term = [&](auto mc) {
+    constexpr int m = decltype(mc)::value;
+    const int y = x + 2 - m;
+    if (y < 2 || y > NT - 3) return;
+    const long long o = (long long)(2 - m) * s;
+    const double gl = (y + 1 <= NT - 1) ? gL[o + s] : 0.;
+    const double gr = gR[o];
+    if (gl == 0. && gr == 0.) return;
+    acc += recon_t_term<m>(c, a + o, s, gl, gr);
+  };
+  term(std::integral_constant<int, 4>{});
+  term(std::integral_constant<int, 3>{});
+  term(std::integral_constant<int, 2>{});
+  term(std::integral_constant<int, 1>{});
+  term(std::integral_constant<int, 0>{});
+  q[(long long)v * Z + z] += acc;
 }
 
 // The ghost fill's transpose: every ghost zone copies the interior zone
@@ -560,17 +629,22 @@ __global__ void k_fold(DevCfg c, const double* __restrict__ q, double* __restric
   const long long z = interior_to_z(c, n);
   int i, j, k;
   zijk(c, z, i, j, k);
+  const bool edge = i < 2 * c.g1 || i >= c.N1 || (c.dim >= 2 && (j < 2 * c.g2 || j >= c.N2)) ||
+                    (c.dim >= 3 && (k < 2 * c.g3 || k >= c.N3));
+  if (!edge) {  // no ghost copies a zone this far inside
+    out[(long long)blockIdx.y * Z + z] = 0. + q[(long long)blockIdx.y * Z + z];
+    return;
+  }
   int ys1[8], ys2[8], ys3[8];
   const int n1 = preimages(i, c.g1, c.N1, c.N1T, c.bc[0], c.bc[1], ys1);
   const int n2 = c.dim >= 2 ? preimages(j, c.g2, c.N2, c.N2T, c.bc[2], c.bc[3], ys2) : (ys2[0] = j, 1);
   const int n3 = c.dim >= 3 ? preimages(k, c.g3, c.N3, c.N3T, c.bc[4], c.bc[5], ys3) : (ys3[0] = k, 1);
-  for (int v = 0; v < c.dof; v++) {
-    double s = 0.;
-    for (int a = 0; a < n1; a++)
-      for (int b = 0; b < n2; b++)
-        for (int m = 0; m < n3; m++) s += q[(long long)v * Z + zidx(c, ys1[a], ys2[b], ys3[m])];
-    out[(long long)v * Z + z] = s;
-  }
+  const long long v = blockIdx.y;  // one row per block of threads
+  double s = 0.;
+  for (int a = 0; a < n1; a++)
+    for (int b = 0; b < n2; b++)
+      for (int m = 0; m < n3; m++) s += q[v * Z + zidx(c, ys1[a], ys2[b], ys3[m])];
+  out[v * Z + z] = s;
 }
 
 
@@ -1115,23 +1189,36 @@ static void stencil_q(const DevCfg& c, const AdjointGeo& geo, const double* P, c
                       double* ebar, double* q, double* gface, cudaStream_t s) {
   using namespace adj;
   const size_t bZ = (size_t)c.Z * sizeof(double);
-  k_div_t<<<nblk(c.Z, 128), 128, 0, s>>>(c, g, Ft);
+  k_div_t<<<dim3(nblk(c.Z, 128), c.dof), 128, 0, s>>>(c, g, Ft);
   k_ct_t_emf<<<nblk(c.Z, 256), 256, 0, s>>>(c, Ft, ebar);
   k_ct_t_raw<<<nblk(c.Z, 256), 256, 0, s>>>(c, ebar, Ft);
   cudaMemsetAsync(q, 0, (size_t)c.dof * bZ, s);
+  const bool flat = c.metric == GRIM_MINKOWSKI;
+  const unsigned nb = nblk(c.Z, 32);
   for (int d = 0; d < c.dim; d++) {
-    if (c.conduction && c.viscosity) k_faces_t<1, 1><<<nblk(c.Z, 32), 32, 0, s>>>(c, d, geo.geoF[d], P, Ft, gface);
-    else if (c.conduction) k_faces_t<1, 0><<<nblk(c.Z, 32), 32, 0, s>>>(c, d, geo.geoF[d], P, Ft, gface);
-    else if (c.viscosity) k_faces_t<0, 1><<<nblk(c.Z, 32), 32, 0, s>>>(c, d, geo.geoF[d], P, Ft, gface);
-    else k_faces_t<0, 0><<<nblk(c.Z, 64), 64, 0, s>>>(c, d, geo.geoF[d], P, Ft, gface);
-    k_recon_t<<<nblk(c.Z, 64), 64, 0, s>>>(c, d, P, gface, q);
+#define GRIM_FACES_T(C, V)                                                                 \
+  do {                                                                                     \
+    auto kernel = flat ? (d == 0   ? &k_faces_t<C, V, true, 0>                             \
+                          : d == 1 ? &k_faces_t<C, V, true, 1>                             \
+                                   : &k_faces_t<C, V, true, 2>)                            \
+                       : (d == 0   ? &k_faces_t<C, V, false, 0>                            \
+                          : d == 1 ? &k_faces_t<C, V, false, 1>                            \
+                                   : &k_faces_t<C, V, false, 2>);                          \
+    kernel<<<nb, 32 * (8 + C + V), 0, s>>>(c, geo.geoF[d], P, Ft, gface);                  \
+  } while (0)
+    if (c.conduction && c.viscosity) GRIM_FACES_T(1, 1);
+    else if (c.conduction) GRIM_FACES_T(1, 0);
+    else if (c.viscosity) GRIM_FACES_T(0, 1);
+    else GRIM_FACES_T(0, 0);
+#undef GRIM_FACES_T
+    k_recon_t<<<dim3(nblk(c.Z, 64), c.dof), 64, 0, s>>>(c, d, P, gface, q);
   }
 }
 
 void adjoint_stencil_t(const DevCfg& c, const AdjointGeo& geo, const double* P, const double* g, double* Ft,
                        double* ebar, double* q, double* gface, double* out, cudaStream_t s) {
   stencil_q(c, geo, P, g, Ft, ebar, q, gface, s);
-  adj::k_fold<<<adj::nblk(c.Zint, 128), 128, 0, s>>>(c, q, out);
+  adj::k_fold<<<dim3(adj::nblk(c.Zint, 128), c.dof), 128, 0, s>>>(c, q, out);
 }
 
 template <int C, int V>
@@ -1139,6 +1226,9 @@ static void adjoint_step_t(const DevCfg& c, const AdjointGeo& geo, double dt, co
                            const AdjointBufs& w, cudaStream_t s) {
   using namespace adj;
   constexpr bool emhd = C || V;
+  const bool flat = c.metric == GRIM_MINKOWSKI;
+  auto stage = flat ? &k_stage<true> : &k_stage<false>;
+  auto cons = flat ? &k_cons<true> : &k_cons<false>;
   const bool torus = c.problem == GRIM_PROBLEM_TORUS;
   const size_t rows = (size_t)c.dof * c.Z * sizeof(double);
   // the start-of-stage hooks' and the ghost fill's transposes: q -> out
@@ -1147,7 +1237,7 @@ static void adjoint_step_t(const DevCfg& c, const AdjointGeo& geo, double dt, co
       k_poles_t<<<nblk(2LL * c.N1T * c.N3T, 128), 128, 0, s>>>(c, geo.geoC, w.q);
       k_inflow_t<<<nblk(2LL * c.ng * c.N2T * c.N3T, 64), 64, 0, s>>>(c, geo.geoC, Pfill, w.q);
     }
-    k_fold<<<nblk(c.Zint, 128), 128, 0, s>>>(c, w.q, out);
+    k_fold<<<dim3(nblk(c.Zint, 128), c.dof), 128, 0, s>>>(c, w.q, out);
   };
   // the explicit sources' transposes at the stage input Ps, into q
   auto sources = [&](const double* Ps) {
@@ -1166,7 +1256,7 @@ static void adjoint_step_t(const DevCfg& c, const AdjointGeo& geo, double dt, co
     k_stage_emhd<C, V><<<nblk(c.Zint, 32), 32, 0, s>>>(c, geo.geoC, GRIM_FULL_STEP, dt, st.P1Sol, st.P0eff, st.PhEff,
                                                       st.divF1, st.Sexp1, lam, w.g, w.p0bar, w.psl);
   } else {
-    k_stage<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.P1Sol, dt, lam, w.g, w.ubar, w.bacc, 0);
+    stage<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.P1Sol, dt, lam, w.g, w.ubar, w.bacc, 0);
   }
   stencil_q(c, geo, st.PhEff, w.g, w.Ft, w.ebar, w.q, w.gface, s);
   sources(st.PhEff);
@@ -1178,12 +1268,12 @@ static void adjoint_step_t(const DevCfg& c, const AdjointGeo& geo, double dt, co
     k_stage_emhd<C, V><<<nblk(c.Zint, 32), 32, 0, s>>>(c, geo.geoC, GRIM_HALF_STEP, 0.5 * dt, st.PhSol, st.P0eff,
                                                       st.P0eff, st.divFh, st.Sexph, w.lamh, w.g, w.p0bar, w.psl);
   } else {
-    k_stage<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.PhSol, 0.5 * dt, w.lamh, w.g, w.ubar, w.bacc, 1);
+    stage<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.PhSol, 0.5 * dt, w.lamh, w.g, w.ubar, w.bacc, 1);
   }
   stencil_q(c, geo, st.P0eff, w.g, w.Ft, w.ebar, w.q, w.gface, s);
   sources(st.P0eff);
   if constexpr (emhd) k_add_interior<<<nblk(c.Zint, 128), 128, 0, s>>>(c, w.p0bar, w.q);
-  else k_cons<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.P0eff, w.ubar, w.bacc, w.q);
+  else cons<<<nblk(c.Zint, 128), 128, 0, s>>>(c, geo.geoC, st.P0eff, w.ubar, w.bacc, w.q);
   hooks_fold(st.P0fill, lam);
 }
 

@@ -396,8 +396,8 @@ GRIM_D S tmunu(const ElemT<S, R>& e, int mu, int nu) {
 }
 
 // computeFluxes(dir) for the fluid rows (physics.cpp:185-217): out[0..nf)
-template <int COND, int VISC, class S, class R>
-GRIM_D void fluxes_fluid(const ElemT<S, R>& e, int dir, R g, S* out, int Q, int DP) {
+template <int COND, int VISC, class S, class R, class RG>
+GRIM_D void fluxes_fluid(const ElemT<S, R>& e, int dir, RG g, S* out, int Q, int DP) {
   S fr = g * (e.rho * e.uCon[dir]);
   out[0] = fr;
   out[1] = g * tmunu<COND, VISC>(e, dir, 0) + fr;
@@ -408,8 +408,8 @@ GRIM_D void fluxes_fluid(const ElemT<S, R>& e, int dir, R g, S* out, int Q, int 
   if (VISC) out[DP] = g * (e.uCon[dir] * e.deltaPTilde);
 }
 // induction rows of computeFluxes
-template <class S, class R>
-GRIM_D void fluxes_B(const ElemT<S, R>& e, int dir, R g, S* out3) {
+template <class S, class R, class RG>
+GRIM_D void fluxes_B(const ElemT<S, R>& e, int dir, RG g, S* out3) {
   out3[0] = g * (e.bCon[1] * e.uCon[dir] - e.bCon[dir] * e.uCon[1]);
   out3[1] = g * (e.bCon[2] * e.uCon[dir] - e.bCon[dir] * e.uCon[2]);
   out3[2] = g * (e.bCon[3] * e.uCon[dir] - e.bCon[dir] * e.uCon[3]);
@@ -470,9 +470,9 @@ GRIM_D void char_speeds(const ElemT<S, R>& e, const GT& G, int dir, const DevCfg
     B = S(2.) * (ADotU * BDotU - ADotU * BDotU * csSqr);
     C = ADotU * ADotU - (S(1.) + ADotU * ADotU) * csSqr;
   } else {
-    const S ASqr = G.gcon[s][s];
-    const S BSqr = G.gcon[0][0];
-    const S ADotB = G.gcon[s][0];
+    const auto ASqr = G.gcon[s][s];
+    const auto BSqr = G.gcon[0][0];
+    const auto ADotB = G.gcon[s][0];
     A = (BDotU * BDotU) - (BSqr + BDotU * BDotU) * csSqr;
     B = S(2.) * (ADotU * BDotU - (ADotB + ADotU * BDotU) * csSqr);
     C = ADotU * ADotU - (ASqr + ADotU * ADotU) * csSqr;
