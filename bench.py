@@ -382,8 +382,8 @@ def batch_problems(seed=5, count=16):
 
 def run_batch(args, local_rank):
     """The ragged-batch workload: value = all problems' zone-cycles/s stepped
-    as one batch (one graph per step, one compacted Newton launch per
-    iteration for all problems); beside it the same problems as separate
+    as one batch (one graph per step, the problems' chains side by side);
+    beside it the same problems as separate
     steppers (fast form and FD64 form) and the adjoint of the largest."""
     import torch
     from grim_b200.timestepper import Batch, timeStepper
@@ -772,7 +772,7 @@ def main():
     ap.add_argument("--decomp", default=None, choices=[None, "x3"],
                     help="x3: split the grid into X3 slabs over the GPUs (strong scaling) instead of replicas")
     ap.add_argument("--per-zone", type=int, default=1,
-                    help="fast Newton: 1 = per-zone loop in one kernel, 2 = compacted worklists")
+                    help="fast Newton: 1 or 2 = per-zone loop in one kernel, 3 = last update deferred")
     args = ap.parse_args()
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))

@@ -1707,17 +1707,21 @@ GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>
   return !(l2 >= 0. && l2 <= newton_tol(c, l2first, K));
 }
 
+// One thread iterates its zone to convergence.  A launch per iteration over a
+// compacted worklist of the unconverged zones, which re-reads each zone's
+// stage constants and state, was 1.5 to 4 times as long on every workload
+// (us per step, both stages: 64^2 wave 76 against 19, Orszag-Tang 512^2 155
+// against 66, EMHD torus 550 against 368, torus 256x128x64 1121 against 547).
 constexpr int kNewtonMinBlocks = 3;  // blocks per SM of the ideal FP32-Jacobian Newton
 template <int COND, int VISC, bool FLAT, class T>
-__global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b,
-                                                              const int* __restrict__ list, long long nlist) {
+__global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int unconv = 0, itsMax = 0;
   bool nanZone = false;
-  if (n < nlist) {
+  if (n < c.Zint) {
     const long long Z = c.Z;
-    const long long z = list ? (long long)list[n] : interior_to_z(c, n);
+    const long long z = interior_to_z(c, n);
     int i, j, k;
     zijk(c, z, i, j, k);
     Geo<FLAT, double> G;
@@ -1743,7 +1747,7 @@ __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kN
       for (int v = 0; v < 3; v++) nanZone |= isnan(K.B[v]);
     }
   }
-  hist_add(b.st->itHist[stage], min(itsMax, 15), n < nlist);
+  hist_add(b.st->itHist[stage], min(itsMax, 15), n < c.Zint);
   // warp-level tallies: no block barrier, so a warp whose zones converged
   // early retires without waiting for the rest of its block
   const int nUnconv = __popc(__ballot_sync(0xffffffffu, unconv != 0));
@@ -1899,227 +1903,6 @@ __global__ void __launch_bounds__(32 * kDeferWarps, kNewtonMinBlocks) k_newton_d
   }
 }
 #endif  // GRIM_FAST_MATH
-
-// ---------------------------------------------------------------------------
-// Compacted fast Newton: one launch per iteration over a worklist of the
-// zones still above tolerance, so no warp carries converged lanes.  The
-// state between launches (P in prim, R, l2first) lives in HBM; worklists are
-// appended with warp-aggregated atomics.  Launch 0 floors, evaluates the
-// residual and lists the unconverged zones; launch it >= 1 does Newton
-// iteration it-1 on list[(it-1)&1] and lists the zones still unconverged.
-// ---------------------------------------------------------------------------
-GRIM_D void list_append(int* list, unsigned long long* count, int zone, bool take) {
-  const unsigned m = __ballot_sync(0xffffffffu, take);
-  if (m == 0) return;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(m) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) base = atomicAdd(count, (unsigned long long)__popc(m));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (take) list[base + __popc(m & ((1u << lane) - 1))] = zone;
-}
-
-// Launch 0, one zone: floors, residual, stored state; true when the zone
-// is above tolerance (goes on the worklist).
-template <int COND, int VISC, bool FLAT>
-GRIM_D bool list_init_zone(const DevCfg& c, int stage, const StageBufs& b, long long z) {
-  constexpr int NF = 5 + COND + VISC;
-  const long long Z = c.Z;
-  int i, j, k;
-  zijk(c, z, i, j, k);
-  Geo<FLAT, double> G;
-  load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
-  StageConst<NF> K;
-  load_stage_const<COND, VISC>(K, c, stage, b, z, G);
-  double P[NF], R[NF];
-#pragma unroll
-  for (int v = 0; v < NF; v++) P[v] = b.prim[(long long)v * Z + z];
-  P[0] = fmax(P[0], c.rhoFloor);
-  P[1] = fmax(P[1], c.uFloor);
-  b.prim[z] = P[0];
-  b.prim[Z + z] = P[1];
-  zone_residual<COND, VISC, double, double>(P, K, G, c, R);
-  const double l2 = l2sum<NF>(R);
-#pragma unroll
-  for (int v = 0; v < NF; v++) b.R[(long long)v * Z + z] = R[v];
-  b.l2[Z + z] = l2;
-  return l2 > newton_tol(c, l2, K);
-}
-
-// Launch it >= 1, one zone on the worklist: one Newton update from the
-// stored state; true when the zone stays above tolerance (and it is not
-// the last iteration).
-template <int COND, int VISC, bool FLAT, class T>
-GRIM_D bool list_iter_zone(const DevCfg& c, int stage, int it, const StageBufs& b, long long z) {
-  constexpr int NF = 5 + COND + VISC;
-  const long long Z = c.Z;
-  const bool last = (it == c.maxIter);
-  int i, j, k;
-  zijk(c, z, i, j, k);
-  Geo<FLAT, double> G;
-  load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
-  Geo<FLAT, T> Gt;
-  convert_geo(Gt, G);
-  StageConst<NF> K;
-  load_stage_const<COND, VISC>(K, c, stage, b, z, G);
-  double P[NF], R[NF];
-#pragma unroll
-  for (int v = 0; v < NF; v++) {
-    P[v] = b.prim[(long long)v * Z + z];
-    R[v] = b.R[(long long)v * Z + z];
-  }
-  const double l2 = l2sum<NF>(R);
-  const double l2first = b.l2[Z + z];
-  T J[NF][NF];
-  tangent_jacobian<COND, VISC, T>(P, K, Gt, c, J);
-  T bv[NF], xv[NF];
-#pragma unroll
-  for (int v = 0; v < NF; v++) bv[v] = (T)(-R[v]);
-  gauss_solve<T, NF>(J, bv, xv);
-  double dPv[NF];
-#pragma unroll
-  for (int v = 0; v < NF; v++) dPv[v] = (double)xv[v];
-  const double f0 = 0.5 * l2, fPrime0 = -2. * f0;
-  double lam = 1.;
-  bool haveR = false;
-  double Rt[NF];
-  for (int ls = 0; ls < c.maxLS; ls++) {
-    double Pt[NF];
-#pragma unroll
-    for (int v = 0; v < NF; v++) Pt[v] = P[v] + lam * dPv[v];
-    zone_residual<COND, VISC, double, double>(Pt, K, G, c, Rt);
-    const double f1 = 0.5 * l2sum<NF>(Rt);
-    if (!(f1 > (f0 * (1. - 1e-4 * lam) + c.lsFloor))) { haveR = true; break; }
-    const double denom = (f1 - f0 - fPrime0 * lam);
-    lam = -fPrime0 * lam * lam / denom / 2.;
-  }
-#pragma unroll
-  for (int v = 0; v < NF; v++) P[v] = P[v] + lam * dPv[v];
-  const bool floored = (P[0] < c.rhoFloor) || (P[1] < c.uFloor);
-  if (!last) {
-    P[0] = fmax(P[0], c.rhoFloor);
-    P[1] = fmax(P[1], c.uFloor);
-  }
-  if (!haveR || floored) zone_residual<COND, VISC, double, double>(P, K, G, c, Rt);
-  const double l2n = l2sum<NF>(Rt);
-  const bool conv = l2n <= newton_tol(c, l2first, K);
-  if (!conv && last) atomicAdd(&b.st->finalUnconv[stage], 1ULL);
-#pragma unroll
-  for (int v = 0; v < NF; v++) {
-    b.prim[(long long)v * Z + z] = P[v];
-    b.R[(long long)v * Z + z] = Rt[v];
-  }
-  return !conv && !last;
-}
-
-template <int COND, int VISC, bool FLAT>
-__global__ void __launch_bounds__(128) k_newton_list_init(DevCfg c, int stage, StageBufs b) {
-  for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < c.Zint; n0 += (long long)gridDim.x * blockDim.x) {
-    const long long n = n0 + threadIdx.x;
-    bool take = false;
-    long long z = 0;
-    if (n < c.Zint) {
-      z = interior_to_z(c, n);
-      take = list_init_zone<COND, VISC, FLAT>(c, stage, b, z);
-    }
-    hist_add(b.st->itHist[stage], 0, n < c.Zint && !take);
-    list_append(b.list[0], &b.st->listCount[0], (int)z, take);
-  }
-}
-
-template <int COND, int VISC, bool FLAT, class T>
-__global__ void __launch_bounds__(128) k_newton_list_iter(DevCfg c, int stage, int it, StageBufs b) {
-  const int in = (it - 1) & 1, out = it & 1;
-  const long long count = (long long)b.st->listCount[in];
-  const bool last = (it == c.maxIter);
-  for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < count; n0 += (long long)gridDim.x * blockDim.x) {
-    const long long n = n0 + threadIdx.x;
-    bool take = false;
-    int zone = 0;
-    if (n < count) {
-      zone = b.list[in][n];
-      take = list_iter_zone<COND, VISC, FLAT, T>(c, stage, it, b, zone);
-    }
-    hist_add(b.st->itHist[stage], min(it, 15), n < count && !take);
-    if (!last) list_append(b.list[out], &b.st->listCount[out], zone, take);
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0 && count > 0) atomicMax(&b.st->itersDone[stage], (unsigned long long)it);
-}
-
-// ---------------------------------------------------------------------------
-// Ragged batch: the compacted Newton of several independent problems (grid
-// sizes may differ) in one launch per iteration.  Worklist entries are
-// global interior indices over the concatenated problems; each lane finds
-// its problem in the offset table and runs the same per-zone code with that
-// problem's configuration and buffers.
-// ---------------------------------------------------------------------------
-GRIM_D int batch_problem(const BatchEntry* tbl, int nprob, long long g) {
-  int lo = 0, hi = nprob - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tbl[mid].offset <= g) lo = mid;
-    else hi = mid - 1;
-  }
-  return lo;
-}
-// histogram add keyed by (problem, bin): one atomic per distinct key in a warp
-GRIM_D void batch_hist_add(const BatchEntry* tbl, int stage, int p, int bin, bool active) {
-  const unsigned act = __ballot_sync(0xffffffffu, active);
-  if (!active) return;
-  const unsigned peers = __match_any_sync(act, p * 16 + bin);
-  if ((threadIdx.x & 31) == __ffs(peers) - 1)
-    atomicAdd(&tbl[p].b[stage].st->itHist[stage][bin], (unsigned long long)__popc(peers));
-}
-
-template <int COND, int VISC, bool FLAT>
-__global__ void __launch_bounds__(128) k_batch_list_init(const BatchEntry* __restrict__ tbl, int nprob,
-                                                         long long total, int stage, BatchState* bs) {
-  for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < total; n0 += (long long)gridDim.x * blockDim.x) {
-    const long long gidx_ = n0 + threadIdx.x;
-    bool take = false;
-    int p = 0;
-    if (gidx_ < total) {
-      p = batch_problem(tbl, nprob, gidx_);
-      const DevCfg& c = tbl[p].c;
-      const long long z = interior_to_z(c, gidx_ - tbl[p].offset);
-      take = list_init_zone<COND, VISC, FLAT>(c, stage, tbl[p].b[stage], z);
-    }
-    batch_hist_add(tbl, stage, p, 0, gidx_ < total && !take);
-    list_append(bs->list[0], &bs->listCount[0], (int)gidx_, take);
-  }
-}
-
-template <int COND, int VISC, bool FLAT, class T>
-__global__ void __launch_bounds__(128) k_batch_list_iter(const BatchEntry* __restrict__ tbl, int nprob, int stage,
-                                                         int it, int lastIt, BatchState* bs) {
-  const int in = (it - 1) & 1, out = it & 1;
-  const long long count = (long long)bs->listCount[in];
-  for (long long n0 = (long long)blockIdx.x * blockDim.x; n0 < count; n0 += (long long)gridDim.x * blockDim.x) {
-    const long long n = n0 + threadIdx.x;
-    bool take = false;
-    int gidx_ = 0, p = 0;
-    if (n < count) {
-      gidx_ = bs->list[in][n];
-      p = batch_problem(tbl, nprob, gidx_);
-      const DevCfg& c = tbl[p].c;
-      const long long z = interior_to_z(c, gidx_ - tbl[p].offset);
-      // a problem past its own maxIter leaves the list (its last update
-      // was counted there)
-      if (it <= c.maxIter) take = list_iter_zone<COND, VISC, FLAT, T>(c, stage, it, tbl[p].b[stage], z);
-    }
-    batch_hist_add(tbl, stage, p, min(it, 15), n < count && !take);
-    {
-      // iterations done, per problem: one atomic per problem in the warp
-      const unsigned act = __ballot_sync(0xffffffffu, n < count);
-      if (n < count) {
-        const unsigned peers = __match_any_sync(act, p);
-        if ((threadIdx.x & 31) == __ffs(peers) - 1)
-          atomicMax(&tbl[p].b[stage].st->itersDone[stage], (unsigned long long)it);
-      }
-    }
-    if (it < lastIt) list_append(bs->list[out], &bs->listCount[out], gidx_, take);
-  }
-}
 
 // ---------------------------------------------------------------------------
 // kernels behind the test entry points
@@ -2605,17 +2388,14 @@ void newton_fd_iter(const DevCfg& c, int stage, int it, const StageBufs& b, cuda
 }
 
 template <int C, int V, bool F>
-static void newton_fast_t(const DevCfg& c, int stage, const StageBufs& b, int mode, const int* list,
-                          long long nlist, cudaStream_t s) {
-  if (nlist <= 0) return;
+static void newton_fast_t(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
   if (mode == GRIM_NEWTON_MIXED32)
-    k_newton_fast<C, V, F, float><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
+    k_newton_fast<C, V, F, float><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
   else
-    k_newton_fast<C, V, F, double><<<nblk(nlist, 128), 128, 0, s>>>(c, stage, b, list, nlist);
+    k_newton_fast<C, V, F, double><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
 }
-void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, const int* list, long long nlist,
-                 cudaStream_t s) {
-  GRIM_GEO_DISPATCH(c, newton_fast_t, c, stage, b, mode, list, nlist, s);
+void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
+  GRIM_GEO_DISPATCH(c, newton_fast_t, c, stage, b, mode, s);
 }
 
 #ifdef GRIM_FAST_MATH
@@ -2636,54 +2416,6 @@ bool newton_defer(const DevCfg& c, int stage, const StageBufs& b, int mode, cuda
   return true;
 }
 #endif
-
-static int persistent_blocks() {
-  static int nb = 0;
-  if (!nb) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    nb = sms * 8;
-  }
-  return nb;
-}
-template <int C, int V, bool F>
-static void newton_list_t(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
-  const int nb = persistent_blocks();
-  cudaMemsetAsync(b.st->listCount, 0, sizeof(b.st->listCount), s);
-  k_newton_list_init<C, V, F><<<nb, 128, 0, s>>>(c, stage, b);
-  for (int it = 1; it <= c.maxIter; it++) {
-    // the list this launch appends to starts empty
-    cudaMemsetAsync(&b.st->listCount[it & 1], 0, sizeof(unsigned long long), s);
-    if (mode == GRIM_NEWTON_MIXED32)
-      k_newton_list_iter<C, V, F, float><<<nb, 128, 0, s>>>(c, stage, it, b);
-    else
-      k_newton_list_iter<C, V, F, double><<<nb, 128, 0, s>>>(c, stage, it, b);
-  }
-}
-void newton_list(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
-  GRIM_GEO_DISPATCH(c, newton_list_t, c, stage, b, mode, s);
-}
-
-template <int C, int V, bool F>
-static void batch_newton_t(const DevCfg& c0, const BatchEntry* tbl, int nprob, long long total, int maxIter, int stage,
-                           int mode, BatchState* bs, cudaStream_t s) {
-  (void)c0;
-  const int nb = persistent_blocks();
-  cudaMemsetAsync(bs->listCount, 0, sizeof(bs->listCount), s);
-  k_batch_list_init<C, V, F><<<nb, 128, 0, s>>>(tbl, nprob, total, stage, bs);
-  for (int it = 1; it <= maxIter; it++) {
-    cudaMemsetAsync(&bs->listCount[it & 1], 0, sizeof(unsigned long long), s);
-    if (mode == GRIM_NEWTON_MIXED32)
-      k_batch_list_iter<C, V, F, float><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
-    else
-      k_batch_list_iter<C, V, F, double><<<nb, 128, 0, s>>>(tbl, nprob, stage, it, maxIter, bs);
-  }
-}
-void batch_newton(const DevCfg& c0, const BatchEntry* tbl, int nprob, long long total, int maxIter, int stage,
-                  int mode, BatchState* bs, cudaStream_t s) {
-  GRIM_GEO_DISPATCH(c0, batch_newton_t, c0, tbl, nprob, total, maxIter, stage, mode, bs, s);
-}
 
 template <int C, int V, bool F>
 static void residual_t(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* out,

@@ -20,9 +20,7 @@
   void advance_time(DevState* st, cudaStream_t s);                                                      \
   void newton_fd_init(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s);                  \
   void newton_fd_iter(const DevCfg& c, int stage, int it, const StageBufs& b, cudaStream_t s);          \
-  void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, const int* list,           \
-                   long long nlist, cudaStream_t s);                                                    \
-  void newton_list(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s);          \
+  void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s);           \
   void residual(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* out,         \
                 cudaStream_t s);                                                                        \
   void jacobian(const DevCfg& c, int stage, const StageBufs& b, const double* pg, double* jac,         \
@@ -101,10 +99,6 @@ void adjoint_stencil_t(const DevCfg& c, const AdjointGeo& geo, const double* P, 
 
 namespace grim {
 namespace fast {
-// the compacted Newton of a ragged batch: one launch per iteration over
-// all problems' unconverged zones (tbl, bs in device memory)
-void batch_newton(const DevCfg& c0, const BatchEntry* tbl, int nprob, long long total, int maxIter, int stage,
-                  int mode, BatchState* bs, cudaStream_t s);
 // the deferred-tail Newton (ideal MHD, mixed form, maxIter >= 2): one
 // persistent launch per stage; false when the configuration is not one it
 // runs (the caller then runs newton_fast)

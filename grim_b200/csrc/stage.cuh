@@ -17,7 +17,6 @@ struct DevState {
   unsigned long long finalUnconv[2];
   unsigned long long nanFlag;
   unsigned long long itHist[2][16];  // zones by Newton iterations used (fast path)
-  unsigned long long listCount[2];   // compacted worklists: entries per ping-pong list
   unsigned long long waitTimeouts;   // bounded waits on asynchronous copies that gave up
   unsigned long long obsCount;       // torus observer records written (ring index = count % capacity)
   unsigned long long drainTimeouts;  // give-up paths whose wait for their own copies in flight gave up too
@@ -51,21 +50,6 @@ struct StageBufs {
   DevState* st;
   unsigned long long* nanCount;  // non-null: the per-zone Newton adds the zones whose result (fluid and field
                                  // rows) holds a NaN (fullStepDiagnostics' count of the full stage)
-  int* list[2];           // compacted Newton worklists (interior zone indices)
-};
-
-// one problem of a ragged batch: its configuration, its stage buffers
-// (half, full) and the offset of its first interior zone in the batch's
-// concatenated index space
-struct BatchEntry {
-  DevCfg c;
-  StageBufs b[2];
-  long long offset;
-};
-// the batch's shared worklists (global interior indices) and their counts
-struct BatchState {
-  unsigned long long listCount[2];
-  int* list[2];
 };
 
 }  // namespace grim

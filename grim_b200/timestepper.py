@@ -450,9 +450,9 @@ class timeStepper:
 
 
 class Batch:
-    """Independent problems stepped together (grim_batch_*): per problem the
-    stencil launches, per stage one compacted Newton launch per iteration
-    over all problems' unconverged zones.  problems[p] is a timeStepper view
+    """Independent problems stepped together (grim_batch_*): each problem's
+    step is one chain of launches, and the chains run side by side on the
+    GPU.  problems[p] is a timeStepper view
     of problem p (state, time, statistics); the batch owns it."""
 
     def __init__(self, cfgs, device=0):

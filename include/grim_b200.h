@@ -85,7 +85,7 @@ typedef struct grim_config {
   int problem;              /* problem hooks: BCs, flux filter, floors */
   int elemOldFromFullStep;  /* 1: fullStepDiagnostics re-sets elemOld */
   int newtonMode;           /* GRIM_NEWTON_* */
-  int perZoneConvergence;   /* 0: global break (reference), 1: per zone, 2: compacted,
+  int perZoneConvergence;   /* 0: global break (reference), 1: per zone, 2: as 1,
                                3: per zone with the last update deferred */
   int N3Global;             /* > 0: the handle holds N3 of N3Global X3 planes of a slab
                                decomposition; X3Start / X3End are the global extent */
@@ -362,8 +362,7 @@ int grim_set_geometry(grim_handle* h, int location, const double* in,
 
 /* ---- options, statistics, graphs ------------------------------------- */
 /* mode: GRIM_NEWTON_*; perZoneConvergence for the tangent / mixed modes:
- * 1 = one kernel, each thread iterates its zone to convergence; 2 = one
- * launch per iteration over a compacted worklist of unconverged zones;
+ * 1 = one kernel, each thread iterates its zone to convergence; 2 = as 1;
  * 3 = one persistent kernel whose warps run the first maxIter - 1 updates
  * of 32 zones together and gather the zones still unconverged, 32 at a
  * time, for the last update (ideal MHD in the mixed mode with
@@ -482,10 +481,10 @@ int grim_set_face_variant(grim_handle* h, int dir, int variant);
 int grim_set_dt_mode(grim_handle* h, int fixed);
 
 /* ---- ragged batch.  No counterpart in the reference (one problem per
- *      run).  Independent problems, grid sizes free, step together on one
- *      stream: per problem the stencil launches of timeStep, and for each
- *      stage ONE compacted Newton launch per iteration over the unconverged
- *      zones of all problems (tangent or mixed mode).  The problems share
+ *      run).  Independent problems, grid sizes free, step together: each
+ *      problem's timeStep (tangent or mixed mode) is one chain of launches
+ *      and the chains run side by side, forked from and joined to the
+ *      batch's stream.  The problems share
  *      the conduction / viscosity flags; each keeps its own dt, time,
  *      boundaries, metric and reconstruction.  grim_batch_problem returns
  *      problem p's handle for set/get of its state and its statistics;
