@@ -1113,7 +1113,7 @@ __global__ void k_dt_speeds(DevCfg c, const double* __restrict__ p, const double
 // grid.cpp:306-360), then per zone
 //   FLOOR: the torus floors (halfStepDiagnostics / fullStepDiagnostics,
 //          torus/problem.cpp:714-746; with POST the NaN reset first),
-//   POST:  after the full step, the zone's term of the next computeDt from
+//   POST:  after the full step, the time advance, the zone's term of the next computeDt from
 //          the stored result (all zones, as k_dt_speeds mode 0; when
 //          dtOn) and the non-finite count over the interior.
 // Every step of the reference's sequence acts on one zone at a time, so the
@@ -1162,6 +1162,7 @@ __global__ void __launch_bounds__(128) k_stage_finish(DevCfg c, TorusCfg t, cons
     }
   }
   if constexpr (POST) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) st->time += st->dt;  // nothing in this kernel reads it
     block_max_to(best, &st->maxInvDt);
     bad = __syncthreads_count(bad);
     if (threadIdx.x == 0 && bad) atomicAdd(&st->nonFinite, (unsigned long long)bad);
@@ -1276,17 +1277,33 @@ static __global__ void k_torus_obs_final(const double* __restrict__ partials, in
 }
 
 // dt = Courant / maxInvDt, capped at maxDtIncrement * dt (timestep.cpp:393-399)
-static __global__ void k_dt_update(DevState* st, double courant, double maxInc) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double newDt = courant / st->maxInvDt;
-    if (newDt > maxInc * st->dt) newDt = maxInc * st->dt;
-    st->dtOld = st->dt;
-    st->dt = newDt;
-  }
+GRIM_D void new_dt(DevState* st, double courant, double maxInc) {
+  double newDt = courant / st->maxInvDt;
+  if (newDt > maxInc * st->dt) newDt = maxInc * st->dt;
+  st->dtOld = st->dt;
+  st->dt = newDt;
 }
-
-static __global__ void k_advance_time(DevState* st) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) st->time += st->dt;
+static __global__ void k_dt_update(DevState* st, double courant, double maxInc) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) new_dt(st, courant, maxInc);
+}
+// The start of a step, one warp: computeDt (unless dt is held) and every
+// counter the step accumulates set to zero, the next maxInvDt among them
+// (its last value has just been used).  One launch for what were a kernel
+// and six memsets, each a node on the critical path of a captured step.
+static __global__ void k_step_begin(DevState* st, double courant, double maxInc, int holdDt) {
+  const int t = threadIdx.x;  // 32 threads
+  if (t == 0) {
+    if (!holdDt) new_dt(st, courant, maxInc);
+    st->maxInvDt = 0.;
+    st->nonFinite = 0;
+    st->nanFlag = 0;
+  }
+  if (t < 2) {
+    st->itersDone[t] = 0;
+    st->finalUnconv[t] = 0;
+  }
+  st->count[t >> 4][t & 15] = 0;
+  st->itHist[t >> 4][t & 15] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -2344,19 +2361,21 @@ int face_variants(const DevCfg& c, int dir) {
 #endif  // !GRIM_SKIP_FACES
 
 #if !defined(GRIM_ONLY_FACES)
+// With explicit sources (Kerr-Schild, extended MHD) the epilogue is two
+// kernels: the centre half, which reads no face flux and may run beside the
+// face kernels, and the flux half, whose induction reads the centre half's
+// consOld.  Without them it is one kernel, launched as the flux half.
 template <int C, int V, bool F>
-static void stage_epilogue_t(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
+static void stage_epilogue_t(const DevCfg& c, int stage, const StageBufs& b, bool centre, cudaStream_t s) {
   if constexpr (!F || C || V) {
-    // centre half first: the flux half's induction reads its consOld
-    k_stage_epilogue<C, V, F, 1><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
-    k_stage_epilogue<C, V, F, 2><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    if (centre) k_stage_epilogue<C, V, F, 1><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    else k_stage_epilogue<C, V, F, 2><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
   } else {
-    // no explicit sources: one kernel
-    k_stage_epilogue<C, V, F, 0><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+    if (!centre) k_stage_epilogue<C, V, F, 0><<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
   }
 }
-void stage_epilogue(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {
-  GRIM_GEO_DISPATCH(c, stage_epilogue_t, c, stage, b, s);
+void stage_epilogue(const DevCfg& c, int stage, const StageBufs& b, bool centre, cudaStream_t s) {
+  GRIM_GEO_DISPATCH(c, stage_epilogue_t, c, stage, b, centre, s);
 }
 
 template <int C, int V, bool F>
@@ -2370,7 +2389,9 @@ void dt_speeds(const DevCfg& c, const double* p, const double* geoC, int mode, D
 void dt_update(DevState* st, double courant, double maxInc, cudaStream_t s) {
   k_dt_update<<<1, 32, 0, s>>>(st, courant, maxInc);
 }
-void advance_time(DevState* st, cudaStream_t s) { k_advance_time<<<1, 32, 0, s>>>(st); }
+void step_begin(DevState* st, double courant, double maxInc, bool holdDt, cudaStream_t s) {
+  k_step_begin<<<1, 32, 0, s>>>(st, courant, maxInc, holdDt ? 1 : 0);
+}
 
 template <int C, int V, bool F>
 static void newton_fd_init_t(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s) {

@@ -13,11 +13,11 @@
   void face_flux(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,    \
                  double* flux, int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s);    \
   int face_variants(const DevCfg& c, int dir);                                                          \
-  void stage_epilogue(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s);                  \
+  void stage_epilogue(const DevCfg& c, int stage, const StageBufs& b, bool centre, cudaStream_t s);     \
   void dt_speeds(const DevCfg& c, const double* p, const double* geoC, int mode, DevState* st,          \
                  cudaStream_t s);                                                                       \
   void dt_update(DevState* st, double courant, double maxInc, cudaStream_t s);                          \
-  void advance_time(DevState* st, cudaStream_t s);                                                      \
+  void step_begin(DevState* st, double courant, double maxInc, bool holdDt, cudaStream_t s);            \
   void newton_fd_init(const DevCfg& c, int stage, const StageBufs& b, cudaStream_t s);                  \
   void newton_fd_iter(const DevCfg& c, int stage, int it, const StageBufs& b, cudaStream_t s);          \
   void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s);           \

@@ -154,7 +154,8 @@ extern "C" int grim_div_fluxes_noalloc(const grim_config* cfg, const double* pri
   if (cudaMemsetAsync(b.st, 0, sizeof(DevState), s) != cudaSuccess) return GRIM_ECUDA;
   if (emhd) exact::emhd_prepass(c, prim, nullptr, b.uT, s);
   for (int d = 0; d < c.dim; d++) exact::face_flux(c, d, prim, nullptr, nullptr, b.flux[d], 0, nullptr, nullptr, s);
-  exact::stage_epilogue(c, GRIM_HALF_STEP, b, s);
+  exact::stage_epilogue(c, GRIM_HALF_STEP, b, true, s);
+  exact::stage_epilogue(c, GRIM_HALF_STEP, b, false, s);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     set_error_message(cudaGetErrorString(e));

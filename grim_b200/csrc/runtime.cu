@@ -80,6 +80,7 @@ struct grim_handle {
   cudaEvent_t ev[8];
   bool graphOn = false;
   cudaGraphExec_t graph = nullptr;
+  bool capturing = false;  // the step being enqueued is captured: it may branch (GraphFork)
   grim_stats stats;
   long long launchesPerStep = 0;
   size_t bytesZ = 0;
@@ -351,24 +352,100 @@ static long long g_launch_counter = 0;
 // primOld; the stand-alone stage pieces (grim_stage_setup and
 // grim_newton_solve) keep it in prim
 static bool step_guess_old(const grim_handle* h) { return !is_fd(h); }
+
+// Parallel branches of a graph being captured on one stream: each branch's
+// first launch depends on what the fork's did, and what follows join()
+// depends on every branch's last launches.  Works on the capture's
+// dependency set directly, so a first step needs no side streams or events
+// (making three streams and four events took 0.35 ms of a new handle's first
+// pass).  Inactive (one stream, in order) when the stream is not capturing.
+class GraphFork {
+ public:
+  GraphFork(cudaStream_t s, bool on) : s_(s), on_(on) {
+    if (on_) on_ = deps(root_);
+    open_ = false;
+  }
+  void branch() {
+    if (!on_) return;
+    if (open_) collect();
+    cudaStreamUpdateCaptureDependencies(s_, root_.data(), root_.size(), cudaStreamSetCaptureDependencies);
+    open_ = true;
+  }
+  void join() {
+    if (!on_ || !open_) return;
+    collect();
+    cudaStreamUpdateCaptureDependencies(s_, tails_.data(), tails_.size(), cudaStreamSetCaptureDependencies);
+    on_ = false;
+  }
+
+ private:
+  bool deps(std::vector<cudaGraphNode_t>& out) const {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t* d = nullptr;
+    size_t n = 0;
+    if (cudaStreamGetCaptureInfo_v2(s_, &st, nullptr, nullptr, &d, &n) != cudaSuccess ||
+        st != cudaStreamCaptureStatusActive)
+      return false;
+    out.insert(out.end(), d, d + n);
+    return true;
+  }
+  void collect() { deps(tails_); }
+  cudaStream_t s_;
+  bool on_, open_;
+  std::vector<cudaGraphNode_t> root_, tails_;
+};
+
+// whether direction d's face kernel is one of the TMA-staged variants, whose
+// persistent grid divides the faces over the whole GPU's resident blocks
+static bool persistent_faces(const grim_handle* h, const double* ps, int d) {
+  const DevCfg& c = h->dc;
+  const int v = h->faceVariant[use_exact(h) ? 0 : 1][d];
+  if (!tmap_for(h, ps, d)) return false;
+  if (c.conduction || c.viscosity) return v == 1;
+  return d == 0 ? (v == 2 || v == 3 || v == 5) : v >= 8;
+}
+
+// The face kernels of the directions and the epilogue's centre half read
+// the same primitives and write arrays of their own: in a captured step
+// they are parallel branches of the graph, joined before the flux half (each
+// fills the GPU for one to a few waves only, one after another, on all but
+// the largest grids).  Measured on one B200, us per step in order / side by
+// side: 64^2 wave 16.1 / 14.0, Orszag-Tang 512^2 236 / 219, extended MHD
+// 256^2 228 / 209, torus 64x48x24 144 / 137, EMHD torus 96x64x32 907 / 862;
+// torus 256x128x64, whose kernels each run many waves, 2465 / 2467.  Past a
+// million zones there is nothing left to gain, and a persistent grid that has
+// to share the GPU finishes late (its blocks' shares are fixed): 2390 / 2500
+// on that torus with two such kernels, so those stay in order.
+constexpr long long kForkPersistentMax = 1LL << 20;
 static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false) {
   const DevCfg& c = h->dc;
   cudaStream_t s = h->stream;
   StageBufs b = stage_bufs(h, stage, guessOld);
-  if (c.conduction || c.viscosity) {
-    PROF(GRIM_PROF_EMHD_PREPASS);
-    KNS_CALL(h, emhd_prepass, c, b.ps, b.geoC, h->uT, s);
-    g_launch_counter++;
-  }
+  const bool emhd = c.conduction || c.viscosity, split = emhd || c.metric != GRIM_MINKOWSKI;
+  bool persistent = false;
+  for (int d = 0; d < c.dim; d++) persistent = persistent || persistent_faces(h, b.ps, d);
+  GraphFork fork(s, h->capturing && !(persistent && c.Zint > kForkPersistentMax));
   for (int d = 0; d < c.dim; d++) {
+    fork.branch();
     PROF(GRIM_PROF_FACES_X1 + d);
     KNS_CALL(h, face_flux, c, d, b.ps, b.geoF[d], b.geoC, h->flux[d], h->faceVariant[use_exact(h) ? 0 : 1][d],
              tmap_for(h, b.ps, d), h->st, s);
     g_launch_counter++;
   }
+  if (split) fork.branch();
+  if (emhd) {
+    PROF(GRIM_PROF_EMHD_PREPASS);
+    KNS_CALL(h, emhd_prepass, c, b.ps, b.geoC, h->uT, s);
+    g_launch_counter++;
+  }
   PROF(GRIM_PROF_EPILOGUE);
-  KNS_CALL(h, stage_epilogue, c, stage, b, s);
-  g_launch_counter += (c.metric != GRIM_MINKOWSKI || c.conduction || c.viscosity) ? 2 : 1;
+  if (split) {
+    KNS_CALL(h, stage_epilogue, c, stage, b, true, s);
+    g_launch_counter++;
+  }
+  fork.join();
+  KNS_CALL(h, stage_epilogue, c, stage, b, false, s);
+  g_launch_counter++;
 }
 
 // the torus step's per-zone fast Newton counts, as it writes the full
@@ -387,10 +464,7 @@ static bool enqueue_newton(grim_handle* h, int stage, bool guessOld = false, boo
   StageBufs b = stage_bufs(h, stage, guessOld);
   PROF(GRIM_PROF_NEWTON);
   countNan = countNan && newton_counts_nan(h);
-  if (countNan) {
-    cudaMemsetAsync(&h->st->nanFlag, 0, sizeof(unsigned long long), s);
-    b.nanCount = &h->st->nanFlag;
-  }
+  if (countNan) b.nanCount = &h->st->nanFlag;  // zero since the step began
   if (h->cfg.newtonMode == GRIM_NEWTON_PARITY_FD64) {
     grim::exact::newton_fd_init(c, stage, b, s);
     g_launch_counter++;
@@ -441,31 +515,38 @@ static void enqueue_full_diagnostics(grim_handle* h) {
   g_launch_counter += 2;
 }
 
+// the stage-start boundary fill; with no outflow or mirror side (a periodic
+// side leaves its whole direction to grid::communicate) it would change
+// nothing and is not launched
+static void enqueue_ghost_fill(grim_handle* h, double* p) {
+  const DevCfg& c = h->dc;
+  PROF(GRIM_PROF_BOUNDARY);
+  bool fills = false;
+  for (int d = 0; d < c.dim; d++) {
+    const int lo = c.bc[2 * d], hi = c.bc[2 * d + 1];
+    if (lo == GRIM_PERIODIC || hi == GRIM_PERIODIC) continue;
+    fills = fills || lo != GRIM_EXCHANGE || hi != GRIM_EXCHANGE;
+  }
+  if (!fills) return;
+  KNS_CALL(h, ghost_fill, c, p, c.dof, h->stream);
+  g_launch_counter++;
+}
+
 // The step in segments around the two stencil + Newton pairs, so that a
 // batch of problems can interleave its problems around one shared Newton
 // launch: pre_half -> stencil(half) -> Newton(half) -> mid -> stencil(full)
 // -> Newton(full) -> post.
 static void enqueue_pre_half(grim_handle* h, bool timed) {
-  const DevCfg& c = h->dc;
   cudaStream_t s = h->stream;
   if (timed) cudaEventRecord(h->ev[0], s);
   // computeDt (timestep.cpp:8): dt from the last elemOld state
-  if (!h->fixedDt) {
-    PROF(GRIM_PROF_DT);
-    KNS_CALL(h, dt_update, h->st, h->cfg.CourantFactor, h->cfg.maxDtIncrement, s);
-    g_launch_counter++;
-  }
-  cudaMemsetAsync(h->st->count, 0, sizeof(h->st->count), s);
-  cudaMemsetAsync(h->st->itersDone, 0, sizeof(h->st->itersDone), s);
-  cudaMemsetAsync(h->st->finalUnconv, 0, sizeof(h->st->finalUnconv), s);
-  cudaMemsetAsync(h->st->itHist, 0, sizeof(h->st->itHist), s);
-  cudaMemsetAsync(&h->st->nonFinite, 0, sizeof(unsigned long long), s);
-  // ---- half stage
   {
-    PROF(GRIM_PROF_BOUNDARY);
-    KNS_CALL(h, ghost_fill, c, h->primOld, c.dof, s);
+    PROF(GRIM_PROF_DT);
+    KNS_CALL(h, step_begin, h->st, h->cfg.CourantFactor, h->cfg.maxDtIncrement, h->fixedDt, s);
     g_launch_counter++;
   }
+  // ---- half stage
+  enqueue_ghost_fill(h, h->primOld);
   enqueue_problem_bcs(h, h->primOld);
   if (!h->cfg.elemOldFromFullStep) enqueue_dt_speeds(h, h->primOld, 0);
   if (timed) cudaEventRecord(h->ev[1], s);
@@ -482,11 +563,7 @@ static void enqueue_mid_finish(grim_handle* h) {
 }
 // the full stage's boundaries on primHalfStep
 static void enqueue_mid_fill(grim_handle* h) {
-  {
-    PROF(GRIM_PROF_BOUNDARY);
-    KNS_CALL(h, ghost_fill, h->dc, h->primHalf, h->dc.dof, h->stream);
-    g_launch_counter++;
-  }
+  enqueue_ghost_fill(h, h->primHalf);
   enqueue_problem_bcs(h, h->primHalf);
 }
 static void enqueue_mid(grim_handle* h) {
@@ -511,20 +588,13 @@ static void enqueue_observers(grim_handle* h, double every, double* out, bool to
 // floors), the next computeDt's speeds when the element is re-set from the
 // full step (linear_modes/problem.cpp:287) and the non-finite count, as one
 // pass after the NaN count
-// time advance and the NaN count of fullStepDiagnostics (on the Newton
-// result, whose interior the finish copies unchanged), unless the full
-// stage's Newton counted it
+// the NaN count of fullStepDiagnostics (on the Newton result, whose interior
+// the finish copies unchanged), unless the full stage's Newton counted it
 static void enqueue_post_count(grim_handle* h, bool nanCounted) {
   const DevCfg& c = h->dc;
   cudaStream_t s = h->stream;
-  {
-    PROF(GRIM_PROF_DT);
-    grim::exact::advance_time(h->st, s);
-    g_launch_counter++;
-  }
   if (h->cfg.problem == GRIM_PROBLEM_TORUS && !nanCounted) {
     PROF(GRIM_PROF_DIAGNOSTICS);
-    cudaMemsetAsync(&h->st->nanFlag, 0, sizeof(unsigned long long), s);
     KNS_CALL(h, torus_nan_flag, c, h->prim, &h->st->nanFlag, s);
     g_launch_counter++;
   }
@@ -535,8 +605,7 @@ static void enqueue_post_finish(grim_handle* h, bool timed) {
   const bool torus = h->cfg.problem == GRIM_PROBLEM_TORUS;
   {
     PROF(GRIM_PROF_COPY);
-    const int dtOn = h->cfg.elemOldFromFullStep ? 1 : 0;
-    if (dtOn) cudaMemsetAsync(&h->st->maxInvDt, 0, sizeof(double), s);
+    const int dtOn = h->cfg.elemOldFromFullStep ? 1 : 0;  // maxInvDt: zero since the step began
     const double* geoC = h->cfg.metric == GRIM_MINKOWSKI ? nullptr : h->geo[GRIM_CENTER];
     KNS_CALL(h, stage_finish, c, h->prim, h->primOld, geoC, torus, true, &h->st->nanFlag, dtOn, h->st, s);
     g_launch_counter++;
@@ -873,7 +942,9 @@ static int run_steps(grim_handle* h, int nsteps) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         long long before = g_launch_counter;
+        h->capturing = true;
         enqueue_step(h, false);
+        h->capturing = false;
         h->launchesPerStep = g_launch_counter - before;
         CK(cudaStreamEndCapture(h->stream, &g));
         cudaError_t e = cudaGraphInstantiate(&h->graph, g, 0);
@@ -1139,7 +1210,8 @@ int grim_compute_div_fluxes(grim_handle* h, const double* prim, double* divF, do
              tmap_for(h, b.ps, d), h->st, h->stream);
   // divergence of all dof rows (the time step needs the fluid rows only)
   b.divFB = 1;
-  KNS_CALL(h, stage_epilogue, c, GRIM_HALF_STEP, b, h->stream);
+  KNS_CALL(h, stage_epilogue, c, GRIM_HALF_STEP, b, true, h->stream);
+  KNS_CALL(h, stage_epilogue, c, GRIM_HALF_STEP, b, false, h->stream);
   CK(cudaGetLastError());
   if (divF) {
     rc = stage_out(h, divF, h->divF, (size_t)c.dof * h->bytesZ, memKind);
@@ -1937,14 +2009,15 @@ int grim_adjoint_backward(grim_handle* h, const double* lambda, double* grad, in
 // ragged batch: independent problems (grid sizes may differ) stepped
 // together, each as one chain of launches beside the others
 // ---------------------------------------------------------------------------
-constexpr int kBatchStreams = 16;  // parallel chains of a batch step, at most
+constexpr int kBatchStreams = 16;  // streams of an eager batch step, at most
 
 struct grim_batch {
   int device = 0;
   std::vector<grim_handle*> h;
   cudaStream_t stream = nullptr;
-  // the chains of a step: problems are dealt to them, largest first, so that
-  // each carries about the same number of zones
+  // the chains of a step: one per problem in a captured step; launched
+  // eagerly, streams made at the first such step, the problems dealt to them
+  // largest first so that each carries about the same number of zones
   std::vector<cudaStream_t> chain;
   std::vector<int> chainOf;  // per problem
   std::vector<int> order;    // problems, largest first
@@ -1984,10 +2057,6 @@ static int batch_chains(grim_batch* B) {
     B->join.push_back(e);
   }
   CK(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
-  B->order.resize(n);
-  for (int p = 0; p < n; p++) B->order[p] = p;
-  std::stable_sort(B->order.begin(), B->order.end(),
-                   [&](int a, int b) { return B->h[a]->dc.Zint > B->h[b]->dc.Zint; });
   std::vector<long long> load(m, 0);
   B->chainOf.resize(n);
   for (int p : B->order) {
@@ -2027,8 +2096,10 @@ int grim_batch_create(const grim_config* cfgs, int n, int device, grim_batch** o
   long long total = 0;
   for (grim_handle* h : B->h) total += h->dc.Zint;
   if (total >= (1LL << 31)) { set_err("grim_batch_create: more than 2^31 zones"); batch_free(B); return GRIM_EINVAL; }
-  const int rc = batch_chains(B);
-  if (rc) { batch_free(B); return rc; }
+  B->order.resize(n);
+  for (int p = 0; p < n; p++) B->order[p] = p;
+  std::stable_sort(B->order.begin(), B->order.end(),
+                   [&](int a, int b) { return B->h[a]->dc.Zint > B->h[b]->dc.Zint; });
   *out = B;
   return GRIM_OK;
 }
@@ -2069,7 +2140,22 @@ int grim_batch_set_newton_mode(grim_batch* B, int mode, double rtol) {
 // one; side by side they fill it.  Measured on the 16-problem family (2.04 M
 // zones, one B200), us per step: problem after problem with one worklist
 // Newton per stage over all of them 1951, chains with the per-zone Newton 1192.
-static int enqueue_batch_step(grim_batch* B) {
+static int enqueue_batch_step(grim_batch* B, bool capturing) {
+  if (capturing) {
+    GraphFork fork(B->stream, true);
+    for (int p : B->order) {
+      fork.branch();
+      B->h[p]->capturing = true;
+      enqueue_step(B->h[p], false);
+      B->h[p]->capturing = false;
+    }
+    fork.join();
+    return GRIM_OK;
+  }
+  if (B->chain.empty()) {
+    const int rc = batch_chains(B);
+    if (rc) return rc;
+  }
   CK(cudaEventRecord(B->fork, B->stream));
   for (cudaStream_t s : B->chain) CK(cudaStreamWaitEvent(s, B->fork, 0));
   for (int p : B->order) {
@@ -2102,7 +2188,7 @@ int grim_batch_time_steps(grim_batch* B, int nsteps) {
       if (!B->graph) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = enqueue_batch_step(B);
+        const int rc = enqueue_batch_step(B, true);
         CK(cudaStreamEndCapture(B->stream, &g));
         if (rc) { cudaGraphDestroy(g); return rc; }
         cudaError_t e = cudaGraphInstantiate(&B->graph, g, 0);
@@ -2111,7 +2197,7 @@ int grim_batch_time_steps(grim_batch* B, int nsteps) {
       }
       CK(cudaGraphLaunch(B->graph, B->stream));
     } else {
-      const int rc = enqueue_batch_step(B);
+      const int rc = enqueue_batch_step(B, false);
       if (rc) return rc;
     }
   }
