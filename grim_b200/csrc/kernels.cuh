@@ -220,6 +220,31 @@ GRIM_D void recon_zone(const DevCfg& c, const double* __restrict__ ps, long long
   }
 }
 
+#ifdef GRIM_FAST_MATH
+// the weights a and signal speeds s of flux = aL (F_L - sL U_L) + aR (F_R -
+// sR U_R), sqrt(-g) included: HLL, or LLF as HLL with the speeds -c, c
+struct FaceWeights {
+  double aL, sL, aR, sR;
+};
+GRIM_D FaceWeights face_weights(const DevCfg& c, double g, double cmin, double cmax) {
+  FaceWeights f;
+  if (c.riemann == GRIM_HLL) {
+    const double id = g / (cmax - cmin);
+    f.aL = cmax * id;
+    f.sL = cmin;
+    f.aR = -cmin * id;
+    f.sR = cmax;
+  } else {
+    const double cm = fmax(cmax, -cmin);
+    f.aL = f.aR = 0.5 * g;
+    f.sL = -cm;
+    f.sR = cm;
+  }
+  return f;
+}
+template <int COND, int VISC, class GT>
+GRIM_D void riemann_face(const DevCfg&, int, const double*, const GT&, double*, long long, double*);  // parity path only
+#else
 // Shared memory holds what waits: the right face state (slot 2, put there
 // by the caller) while the left element is evaluated, then the left
 // state's fluxes (slots 0, 1) while the right element is; slot [v][thread],
@@ -230,7 +255,7 @@ GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const GT& G
   constexpr int NF = 5 + COND + VISC;
   constexpr int DOF = NF + 3;
   const long long Z = c.Z;
-  const int fd = dir + 1;
+  [[maybe_unused]] const int fd = dir + 1;
   const int nt = blockDim.x, t = threadIdx.x;
   double minL, maxL;
   {
@@ -266,12 +291,11 @@ GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const GT& G
   const double cmin = fmin(minL, minR);
   const double cmax = fmax(maxL, maxR);
   if (c.riemann == GRIM_HLL) {
-    const double id = 1. / (cmax - cmin);
 #pragma unroll
     for (int v = 0; v < DOF; v++) {
       const double FL = park[v * nt + t], UL = park[(DOF + v) * nt + t];
       const double num = cmax * FL - cmin * F[v] + cmin * cmax * (U[v] - UL);
-      flux[(long long)v * Z + z] = kFastMath ? num * id : num / (cmax - cmin);
+      flux[(long long)v * Z + z] = num / (cmax - cmin);
     }
   } else {
     const double cm = fmax(cmax, -cmin);
@@ -282,18 +306,22 @@ GRIM_D void riemann_face(const DevCfg& c, int dir, const double* pl, const GT& G
     }
   }
 }
+#endif
 
 // The same face flux with both states' elements evaluated side by side
-// (no shared-memory parking): twice the independent arithmetic per thread
-// for more registers, which the autotuner weighs against occupancy.
+// (no shared-memory parking): twice the independent arithmetic per thread.
+// In the parity path the autotuner weighs it against the parked form; the
+// fast path, whose side_flux needs the speeds of both states first, has this
+// form only (torus 256x128x64, us per step: X1 358 parked / 333 side by side,
+// X2 422 / 378, X3 424 / 409; with F and U of both sides formed apart it was
+// 395 / 389, 459 / 467, 451 / 478).
 template <int COND, int VISC, class GT>
 GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const double* pr,
                               const GT& G, double* __restrict__ flux, long long z) {
   constexpr int NF = 5 + COND + VISC;
   constexpr int DOF = NF + 3;
   const long long Z = c.Z;
-  const int fd = dir + 1;
-  double F[2][DOF], U[2][DOF], mn[2], mx[2];
+  [[maybe_unused]] const int fd = dir + 1;
   ElemT<double, double> e[2];
 #pragma unroll
   for (int sd = 0; sd < 2; sd++) {
@@ -301,6 +329,17 @@ GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const 
     elem_set<COND, VISC>(e[sd], q[0], q[1], q[2], q[3], q[4], q[NF], q[NF + 1], q[NF + 2], COND ? q[5] : 0.,
                          VISC ? q[5 + COND] : 0., G, c);
   }
+#ifdef GRIM_FAST_MATH
+  double mn[2], mx[2], L[DOF], R[DOF];
+#pragma unroll
+  for (int sd = 0; sd < 2; sd++) char_speeds<COND, VISC>(e[sd], G, dir, c, mn[sd], mx[sd]);
+  const FaceWeights fw = face_weights(c, G.g, fmin(mn[0], mn[1]), fmax(mx[0], mx[1]));
+  side_flux<COND, VISC>(e[0], dir, fw.sL, L);
+  side_flux<COND, VISC>(e[1], dir, fw.sR, R);
+#pragma unroll
+  for (int v = 0; v < DOF; v++) flux[(long long)v * Z + z] = fw.aL * L[v] + fw.aR * R[v];
+#else
+  double F[2][DOF], U[2][DOF], mn[2], mx[2];
 #pragma unroll
   for (int sd = 0; sd < 2; sd++) {
     fluxes_fluid<COND, VISC>(e[sd], fd, G.g, F[sd], 5, 5 + COND);
@@ -312,17 +351,17 @@ GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const 
   const double cmin = fmin(mn[0], mn[1]);
   const double cmax = fmax(mx[0], mx[1]);
   if (c.riemann == GRIM_HLL) {
-    const double id = 1. / (cmax - cmin);
 #pragma unroll
     for (int v = 0; v < DOF; v++) {
       const double num = cmax * F[0][v] - cmin * F[1][v] + cmin * cmax * (U[1][v] - U[0][v]);
-      flux[(long long)v * Z + z] = kFastMath ? num * id : num / (cmax - cmin);
+      flux[(long long)v * Z + z] = num / (cmax - cmin);
     }
   } else {
     const double cm = fmax(cmax, -cmin);
 #pragma unroll
     for (int v = 0; v < DOF; v++) flux[(long long)v * Z + z] = 0.5 * (F[0][v] + F[1][v] - cm * (U[1][v] - U[0][v]));
   }
+#endif
 }
 
 // X1 faces: warp w of a row covers faces i0 .. i0+30; lane l reconstructs
@@ -442,8 +481,8 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_x1_tma(const __grid_con
   extern __shared__ __align__(128) double smem_x1[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double* rows = smem_x1 + (size_t)w * 2 * ROW;
-  double* park = smem_x1 + (size_t)nw * 2 * ROW;
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(park + 3 * DOF * blockDim.x) + 2 * w;
+  [[maybe_unused]] double* park = smem_x1 + (size_t)nw * 2 * ROW;
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(park + (PAIR ? 0 : 3 * DOF * blockDim.x)) + 2 * w;
   const int nfaces = c.N1T - 5;  // faces i = 3 .. N1T-3
   const int wpr = (nfaces + 30) / 31;
   const long long nitems = (long long)c.nfj * c.nfk * wpr;
@@ -538,8 +577,8 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_strip_tma(const __grid_
   extern __shared__ __align__(128) double smem_st[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double* bufs = smem_st + (size_t)w * 2 * BOX;
-  double* park = smem_st + (size_t)nw * 2 * BOX;
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(park + 3 * DOF * blockDim.x) + 2 * w;
+  [[maybe_unused]] double* park = smem_st + (size_t)nw * 2 * BOX;
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(park + (PAIR ? 0 : 3 * DOF * blockDim.x)) + 2 * w;
   const int NT = (DIR == 1) ? c.N2T : c.N3T;
   const unsigned nq = (unsigned)(c.N1T + QI - 1) / QI;
   const unsigned nch = (unsigned)(NT - 5 + FPW - 1) / FPW;  // faces 3 .. NT-3
@@ -912,7 +951,10 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
     auto st = [&](int m, int dir, double dx) -> double {
       const long long sd = stride_of(c, dir);
       const double* a = uT + (long long)m * Z + z;
-      return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], dx);
+      if constexpr (kFastMath)
+        return recon_slope_fast(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.invdX[dir]);
+      else
+        return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], dx);
     };
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) {
@@ -1381,7 +1423,7 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
       const double f = (c.hoCond == 1) ? sqrt(er.tau / (er.rho * er.chi)) / er.temperature : 1.;
       const double half = (c.hoCond == 1) ? 0.5 * G.g * er.qTilde : 0.;
       const double s = gt * f * er.rho * er.chi * er.ibNorm, ni = norm * K.idtp;
-      K.rowU[0] = ni;
+      K.rowU[0] = G.g * ni;
       K.rowP[0] = 0.5 * gt * norm;
       K.rowK[0] = (K.Kc[5] + 0.5 * gt * eo.qTilde) * norm;
       K.rowT = s * er.bCon[0] * ni;
@@ -1395,7 +1437,7 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
       const double half = (c.hoVisc == 1) ? 0.5 * G.g * er.deltaPTilde : 0.;
       const double s = gt * f * er.rho * er.nu, ni = norm * K.idtp;
       const double sb = 3. * s * er.bCon[0] * er.ibSqr;
-      K.rowU[1] = ni;
+      K.rowU[1] = G.g * ni;
       K.rowP[1] = 0.5 * gt * norm;
       K.rowK[1] = (K.Kc[5 + COND] + 0.5 * gt * eo.deltaPTilde) * norm;
 #pragma unroll
@@ -2168,13 +2210,13 @@ void emhd_prepass(const DevCfg& c, const double* ps, const double* geoC, double*
 
 #if !defined(GRIM_SKIP_FACES)
 // Launch-shape variants of the face kernels, chosen per direction by the
-// autotuner (grim_autotune): X1 faces by the register budget (3 or 4
-// resident 128-thread blocks per SM), X2 / X3 faces by that budget and by
-// the lane split QI (i per warp).  EMHD has one shape (2 resident blocks).
+// autotuner (grim_autotune): X1 faces by the register budget (resident
+// 128-thread blocks per SM), X2 / X3 faces by that budget and by the lane
+// split QI (i per warp); see face_variants.
 // the reconstruction scheme is a compile-time constant of the X1 kernels
 // as of the TMA ones: one scheme's code per kernel keeps the instruction
 // footprint small
-template <int C, int V, bool F, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = kFastMath>
 static void face_x1_launch(const DevCfg& c, const double* ps, const double* geoF, double* flux, cudaStream_t s) {
   const long long warps = (long long)c.nfj * c.nfk * ((c.N1T - 5 + 30) / 31);
   const size_t park = PAIR ? 0 : 3 * (8 + C + V) * 128 * sizeof(double);
@@ -2186,7 +2228,7 @@ static void face_x1_launch(const DevCfg& c, const double* ps, const double* geoF
     default: k_face_flux_x1<C, V, F, MINB, PAIR, GRIM_MINMOD><<<nb, 128, park, s>>>(c, ps, geoF, flux); break;
   }
 }
-template <int C, int V, bool F, int QI, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int QI, int MINB, bool PAIR = kFastMath>
 static void face_strip_launch(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,
                               double* flux, cudaStream_t s) {
   const int NT = (dir == 1) ? c.N2T : c.N3T;
@@ -2223,7 +2265,7 @@ static void face_x1_tma_launch_rs(const DevCfg& c, const CUtensorMap* tmap, cons
                                   DevState* st, cudaStream_t s) {
   constexpr int DOF = 8 + C + V;
   const int nw = 4;
-  const size_t smem = ((size_t)nw * 2 * DOF * kX1Box + 3 * DOF * 128) * sizeof(double) + 2 * nw * 8;
+  const size_t smem = ((size_t)nw * 2 * DOF * kX1Box + (PAIR ? 0 : 3 * DOF * 128)) * sizeof(double) + 2 * nw * 8;
   // the attribute belongs to the function on each device that launches it
   static unsigned long long attrDevices = 0;
   int dev = 0;
@@ -2237,7 +2279,7 @@ static void face_x1_tma_launch_rs(const DevCfg& c, const CUtensorMap* tmap, cons
 }
 // the reconstruction scheme becomes a compile-time constant of the TMA
 // kernels: one scheme's code per kernel keeps the instruction footprint small
-template <int C, int V, bool F, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = kFastMath>
 static void face_x1_tma_launch(const DevCfg& c, const CUtensorMap* tmap, const double* geoF, double* flux,
                                DevState* st, cudaStream_t s) {
   switch (c.reconstruction) {
@@ -2252,7 +2294,7 @@ static void face_strip_tma_launch_rs(const DevCfg& c, int dir, const CUtensorMap
                                      const double* geoC, double* flux, DevState* st, cudaStream_t s) {
   constexpr int DOF = 8 + C + V;
   const int nw = 4;
-  const size_t smem = ((size_t)nw * 2 * 4 * kStripRows * DOF + 3 * DOF * 128) * sizeof(double) + 2 * nw * 8;
+  const size_t smem = ((size_t)nw * 2 * 4 * kStripRows * DOF + (PAIR ? 0 : 3 * DOF * 128)) * sizeof(double) + 2 * nw * 8;
   static unsigned long long attrDevices = 0;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -2270,7 +2312,7 @@ static void face_strip_tma_launch_rs(const DevCfg& c, int dir, const CUtensorMap
     k_face_flux_strip_tma<C, V, F, MINB, 2, RS, PAIR>
         <<<sm_count() * MINB, 32 * nw, smem, s>>>(tmap[2], c, geoF, geoC, flux, st);
 }
-template <int C, int V, bool F, int MINB, bool PAIR = false>
+template <int C, int V, bool F, int MINB, bool PAIR = kFastMath>
 static void face_strip_tma_launch(const DevCfg& c, int dir, const CUtensorMap* tmap, const double* geoF,
                                   const double* geoC, double* flux, DevState* st, cudaStream_t s) {
   switch (c.reconstruction) {
@@ -2287,7 +2329,39 @@ static void face_strip_tma_launch(const DevCfg& c, int dir, const CUtensorMap* t
 template <int C, int V, bool F>
 static void face_flux_t(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,
                         double* flux, int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s) {
-  if constexpr (C == 0 && V == 0) {
+  if constexpr (kFastMath && C == 0 && V == 0) {
+    const bool tma = tmap && st;
+    if (dir == 0) {
+      if ((variant == 2 || variant == 5) && tma) face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s);
+      else if (variant == 3 && tma) face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s);
+      else if (variant == 1 || variant == 3) face_x1_launch<C, V, F, 5>(c, ps, geoF, flux, s);
+      else face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s);
+      return;
+    }
+    if (variant >= 8 && tma) {
+      if (variant & 1) face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s);
+      return;
+    }
+    switch (variant) {
+      case 1: face_strip_launch<C, V, F, 4, 5>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 2: face_strip_launch<C, V, F, 2, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 3: face_strip_launch<C, V, F, 2, 5>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 4: case 6: face_strip_launch<C, V, F, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 5: face_strip_launch<C, V, F, 8, 5>(c, dir, ps, geoF, geoC, flux, s); break;
+      default: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+    }
+  } else if constexpr (kFastMath) {
+    constexpr int MB = F ? 4 : 3;  // resident blocks: 110 registers in Minkowski, 158 in Kerr-Schild
+    const bool tma = variant == 1 && tmap && st;
+    if (dir == 0) {
+      if (tma) face_x1_tma_launch<C, V, F, MB>(c, &tmap[0], geoF, flux, st, s);
+      else face_x1_launch<C, V, F, MB>(c, ps, geoF, flux, s);
+    } else {
+      if (tma) face_strip_tma_launch<C, V, F, MB>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else face_strip_launch<C, V, F, 4, MB>(c, dir, ps, geoF, geoC, flux, s);
+    }
+  } else if constexpr (C == 0 && V == 0) {
     if (dir == 0) {
       if ((variant == 2 || variant == 3 || variant == 5) && tmap && st) {
         if (variant == 5) face_x1_tma_launch<C, V, F, 3, true>(c, &tmap[0], geoF, flux, st, s);
@@ -2341,21 +2415,26 @@ void face_flux(const DevCfg& c, int dir, const double* ps, const double* geoF, c
                int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s) {
   GRIM_GEO_DISPATCH(c, face_flux_t, c, dir, ps, geoF, geoC, flux, variant, tmap, st, s);
 }
-// X1: 0, 1 = register budget 3 / 4 blocks; 2, 3 = the same with TMA-staged
-// rows (when the caller has a tensor map of the primitives); 4 = both face
-// states evaluated side by side; 5 = TMA-staged rows with both states side
-// by side, 3 blocks per SM; 6 = both states side by side, 4 blocks per SM.
-// X2 / X3: 0-5 = lane split x register budget;
-// 6, 7 = side by side with 8 / 4 i per warp; 8, 9 = TMA-staged chunks, 3 / 4
-// blocks per SM; 10, 11 = TMA-staged chunks side by side, 3 / 4 blocks per
-// SM.
-// EMHD (10 dof), every direction: 0 = plain, 1 = TMA-staged, 2 blocks per SM.
+// Parity path, X1: 0, 1 = register budget 3 / 4 blocks; 2, 3 = the same with
+// TMA-staged rows (when the caller has a tensor map of the primitives); 4 =
+// both face states evaluated side by side; 5 = TMA-staged rows with both
+// states side by side, 3 blocks per SM; 6 = both states side by side, 4
+// blocks per SM.
+// X2 / X3: 0-5 = lane split x register budget; 6, 7 = side by side with 8 / 4
+// i per warp; 8, 9 = TMA-staged chunks, 3 / 4 blocks per SM; 10, 11 =
+// TMA-staged chunks side by side, 3 / 4 blocks per SM.
+// Fast path (always side by side; about 120 registers in Kerr-Schild, 76-90
+// in Minkowski), X1: 0 = 4 blocks, 1 = 5 (a few spills in Kerr-Schild), 2 / 3
+// = TMA-staged, 3 / 4 blocks; 4, 6 run 0 and 5 runs 2.  X2 / X3: 0-5 = 4, 2, 8
+// i per warp x 4 / 5 blocks; 8, 9 = TMA-staged, 3 / 4 blocks; 7 runs 0, 6
+// runs 4, 10 and 11 run 8 and 9.
+// EMHD (9 or 10 dof), every direction: 0 = plain, 1 = TMA-staged.
 // tmap points at the caller's three tensor maps (X1, X2, X3 box shapes) of
 // the prim array, or is null (the TMA variants then run their plain
 // counterparts).
 int face_variants(const DevCfg& c, int dir) {
   (void)dir;
-  if (c.conduction || c.viscosity) return 2;  // plain / TMA-staged, 2 blocks per SM
+  if (c.conduction || c.viscosity) return 2;  // plain / TMA-staged
   return dir == 0 ? 7 : 12;
 }
 #endif  // !GRIM_SKIP_FACES
