@@ -1461,66 +1461,69 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
   }
 }
 
-// pivoted Gaussian elimination (the oracle's; af::solve at solve.cpp:220)
-template <class T, int N>
-GRIM_D void gauss_solve(T A[N][N], T b[N], T x[N]) {
+// pivoted Gaussian elimination (the oracle's; af::solve at solve.cpp:220).
+// One template step per column: every index is a constant whatever the size,
+// so the matrix stays in registers (nested loops of the 7 x 7 extended-MHD
+// system were left partly rolled, its augmented matrix in local memory).
+template <class T, int N, int K>
+GRIM_D void gauss_column(T A[N][N], T b[N]) {
+  if constexpr (K < N) {
+    int p = K;
+    T best = fabs(A[K][K]);
 #pragma unroll
-  for (int kk = 0; kk < N; kk++) {
-    int p = kk;
-    T best = fabs(A[kk][kk]);
-#pragma unroll
-    for (int r = kk + 1; r < N; r++) {
-      T v = fabs(A[r][kk]);
+    for (int r = K + 1; r < N; r++) {
+      T v = fabs(A[r][K]);
       if (v > best) { best = v; p = r; }
     }
     // row exchange as selects over compile-time indices, so the matrix
     // stays in registers (a conditional swap sends it to local memory);
-    // columns left of kk are not read again
+    // columns left of K are not read again
 #pragma unroll
-    for (int r = kk + 1; r < N; r++) {
+    for (int r = K + 1; r < N; r++) {
       const bool sw = (r == p);
 #pragma unroll
-      for (int cc = kk; cc < N; cc++) {
-        const T a0 = A[kk][cc], a1 = A[r][cc];
-        A[kk][cc] = sw ? a1 : a0;
+      for (int cc = K; cc < N; cc++) {
+        const T a0 = A[K][cc], a1 = A[r][cc];
+        A[K][cc] = sw ? a1 : a0;
         A[r][cc] = sw ? a0 : a1;
       }
-      const T b0 = b[kk], b1 = b[r];
-      b[kk] = sw ? b1 : b0;
+      const T b0 = b[K], b1 = b[r];
+      b[K] = sw ? b1 : b0;
       b[r] = sw ? b0 : b1;
     }
-    const T akk = A[kk][kk];
-    if constexpr (kFastMath) {
-      // one reciprocal per pivot, kept for the back substitution
-      const T ia = T(1) / akk;
-      A[kk][kk] = ia;
+    const T akk = A[K][K];
+    // fast path: one reciprocal per pivot, kept for the back substitution
+    [[maybe_unused]] const T ia = kFastMath ? T(1) / akk : T(0);
+    if constexpr (kFastMath) A[K][K] = ia;
 #pragma unroll
-      for (int r = kk + 1; r < N; r++) {
-        T l = A[r][kk] * ia;
+    for (int r = K + 1; r < N; r++) {
+      T l;
+      if constexpr (kFastMath) l = A[r][K] * ia;
+      else l = A[r][K] / akk;
 #pragma unroll
-        for (int cc = kk + 1; cc < N; cc++) A[r][cc] -= l * A[kk][cc];
-        b[r] -= l * b[kk];
-      }
-    } else {
-#pragma unroll
-      for (int r = kk + 1; r < N; r++) {
-        T l = A[r][kk] / akk;
-#pragma unroll
-        for (int cc = kk + 1; cc < N; cc++) A[r][cc] -= l * A[kk][cc];
-        b[r] -= l * b[kk];
-      }
+      for (int cc = K + 1; cc < N; cc++) A[r][cc] -= l * A[K][cc];
+      b[r] -= l * b[K];
     }
+    gauss_column<T, N, K + 1>(A, b);
   }
+}
+template <class T, int N, int R>
+GRIM_D void gauss_back(T A[N][N], T b[N], T x[N]) {
+  if constexpr (R >= 0) {
+    T s = b[R];
 #pragma unroll
-  for (int r = N - 1; r >= 0; r--) {
-    T s = b[r];
-#pragma unroll
-    for (int cc = r + 1; cc < N; cc++) s -= A[r][cc] * x[cc];
+    for (int cc = R + 1; cc < N; cc++) s -= A[R][cc] * x[cc];
     if constexpr (kFastMath)
-      x[r] = s * A[r][r];  // the stored reciprocal
+      x[R] = s * A[R][R];  // the stored reciprocal
     else
-      x[r] = s / A[r][r];
+      x[R] = s / A[R][R];
+    gauss_back<T, N, R - 1>(A, b, x);
   }
+}
+template <class T, int N>
+GRIM_D void gauss_solve(T A[N][N], T b[N], T x[N]) {
+  gauss_column<T, N, 0>(A, b);
+  gauss_back<T, N, N - 1>(A, b, x);
 }
 
 // histogram of per-zone iteration counts, one atomic per distinct value in
@@ -1771,7 +1774,10 @@ GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>
 // stage constants and state, was 1.5 to 4 times as long on every workload
 // (us per step, both stages: 64^2 wave 76 against 19, Orszag-Tang 512^2 155
 // against 66, EMHD torus 550 against 368, torus 256x128x64 1121 against 547).
-constexpr int kNewtonMinBlocks = 3;  // blocks per SM of the ideal FP32-Jacobian Newton
+// Blocks per SM of the ideal FP32-Jacobian Newton: 4 (128 registers, 84 bytes
+// of spills in Kerr-Schild, none in Minkowski) takes 495 us per torus step, 3
+// (168, none) 525.
+constexpr int kNewtonMinBlocks = 4;
 template <int COND, int VISC, bool FLAT, class T>
 __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
