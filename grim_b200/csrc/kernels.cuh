@@ -777,10 +777,8 @@ static __global__ void k_emf(DevCfg c, const double* __restrict__ F1, const doub
 // 3D torus: 64 registers with a few spills beat 85 and 98 without)
 constexpr int kEpiMinBlocks[3] = {4, 5, 8};
 template <int COND, int VISC, bool FLAT, int PART>
-__global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(DevCfg c, int stage, StageBufs b) {
+GRIM_D void epilogue_zone(const DevCfg& c, int stage, const StageBufs& b, long long n) {
   constexpr int NF = 5 + COND + VISC;
-  long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= c.Zint) return;
   const long long Z = c.Z;
   const long long z = interior_to_z(c, n);
   int i, j, k;
@@ -1067,6 +1065,12 @@ __global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(Dev
 #pragma unroll
     for (int v = 0; v < NF; v++) b.prim[(long long)v * Z + z] = b.pold[(long long)v * Z + z];
   }  // PART != 1
+}
+
+template <int COND, int VISC, bool FLAT, int PART>
+__global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(DevCfg c, int stage, StageBufs b) {
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < c.Zint) epilogue_zone<COND, VISC, FLAT, PART>(c, stage, b, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1779,7 +1783,7 @@ GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>
 // (168, none) 525.
 constexpr int kNewtonMinBlocks = 4;
 template <int COND, int VISC, bool FLAT, class T>
-__global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b) {
+GRIM_D void newton_block(const DevCfg& c, int stage, const StageBufs& b) {
   constexpr int NF = 5 + COND + VISC;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int unconv = 0, itsMax = 0;
@@ -1823,6 +1827,20 @@ __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kN
     if (nUnconv) atomicAdd(&b.st->finalUnconv[stage], (unsigned long long)nUnconv);
     if (nNan) atomicAdd(b.nanCount, (unsigned long long)nNan);
   }
+}
+
+template <int COND, int VISC, bool FLAT, class T>
+__global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kNewtonMinBlocks) k_newton_fast(DevCfg c, int stage, StageBufs b) {
+  newton_block<COND, VISC, FLAT, T>(c, stage, b);
+}
+// The flux half of the epilogue and the Newton of the same zone in one
+// launch: nothing of a zone's solve depends on another zone's epilogue, and a
+// thread reads back only what it wrote itself.
+template <bool FLAT, class T>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 1 : kNewtonMinBlocks) k_stage_solve(DevCfg c, int stage, StageBufs b) {
+  const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (n < c.Zint) epilogue_zone<0, 0, FLAT, FLAT ? 0 : 2>(c, stage, b, n);
+  newton_block<0, 0, FLAT, T>(c, stage, b);
 }
 
 #ifdef GRIM_FAST_MATH
@@ -2503,6 +2521,14 @@ static void newton_fast_t(const DevCfg& c, int stage, const StageBufs& b, int mo
 void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
   GRIM_GEO_DISPATCH(c, newton_fast_t, c, stage, b, mode, s);
 }
+#ifdef GRIM_FAST_MATH
+void stage_solve(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
+  auto kernel = mode == GRIM_NEWTON_MIXED32
+                    ? (c.metric == GRIM_MINKOWSKI ? &k_stage_solve<true, float> : &k_stage_solve<false, float>)
+                    : (c.metric == GRIM_MINKOWSKI ? &k_stage_solve<true, double> : &k_stage_solve<false, double>);
+  kernel<<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+}
+#endif
 
 #ifdef GRIM_FAST_MATH
 bool newton_defer(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {

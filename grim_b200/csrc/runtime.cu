@@ -417,7 +417,7 @@ static bool persistent_faces(const grim_handle* h, const double* ps, int d) {
 // to share the GPU finishes late (its blocks' shares are fixed): 2390 / 2500
 // on that torus with two such kernels, so those stay in order.
 constexpr long long kForkPersistentMax = 1LL << 20;
-static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false) {
+static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false, bool fluxHalf = true) {
   const DevCfg& c = h->dc;
   cudaStream_t s = h->stream;
   StageBufs b = stage_bufs(h, stage, guessOld);
@@ -444,6 +444,7 @@ static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false) {
     g_launch_counter++;
   }
   fork.join();
+  if (!fluxHalf) return;
   KNS_CALL(h, stage_epilogue, c, stage, b, false, s);
   g_launch_counter++;
 }
@@ -485,6 +486,36 @@ static bool enqueue_newton(grim_handle* h, int stage, bool guessOld = false, boo
     grim::fast::newton_fast(c, stage, b, h->cfg.newtonMode, s);
     g_launch_counter++;
   }
+  return countNan;
+}
+
+// A stage's flux half and Newton as one launch (k_stage_solve) on grids of
+// about a wave of the Newton's blocks, where a launch less on the step's
+// critical path is what counts; the flux half is a memory stream that wants
+// twice the Newton's resident warps, so larger grids keep the two apart.
+// Measured on one B200, us per step apart / together: 64^2 wave 14.6 / 13.1,
+// PPM vortex 301x187 36.2 / 34.8, torus 64x48x24 118.6 / 114.3; Orszag-Tang
+// 512^2 193 / 192, torus 256x128x64 2267 / 2373, EMHD 256^2 167 / 170.
+constexpr long long kFuseMax = 1LL << 17;
+static bool stage_fused(const grim_handle* h) {
+  const DevCfg& c = h->dc;
+  return !is_fd(h) && h->cfg.perZoneConvergence != 3 && !h->profOn && !c.conduction && !c.viscosity &&
+         c.Zint <= kFuseMax;
+}
+// between: recorded between the stencil and the solve (null: not)
+static bool enqueue_stage(grim_handle* h, int stage, bool guessOld, bool countNan, cudaEvent_t between) {
+  if (!stage_fused(h)) {
+    enqueue_stencil(h, stage, guessOld);
+    if (between) cudaEventRecord(between, h->stream);
+    return enqueue_newton(h, stage, guessOld, countNan);
+  }
+  enqueue_stencil(h, stage, guessOld, false);
+  if (between) cudaEventRecord(between, h->stream);
+  StageBufs b = stage_bufs(h, stage, guessOld);
+  countNan = countNan && newton_counts_nan(h);
+  if (countNan) b.nanCount = &h->st->nanFlag;
+  grim::fast::stage_solve(h->dc, stage, b, h->cfg.newtonMode, h->stream);
+  g_launch_counter++;
   return countNan;
 }
 
@@ -645,15 +676,11 @@ static void enqueue_segment(grim_handle* h, int seg) {
 static void enqueue_step(grim_handle* h, bool timed) {
   cudaStream_t s = h->stream;
   enqueue_pre_half(h, timed);
-  enqueue_stencil(h, GRIM_HALF_STEP, step_guess_old(h));
-  if (timed) cudaEventRecord(h->ev[2], s);
-  enqueue_newton(h, GRIM_HALF_STEP, step_guess_old(h));
+  enqueue_stage(h, GRIM_HALF_STEP, step_guess_old(h), false, timed ? h->ev[2] : nullptr);
   if (timed) cudaEventRecord(h->ev[3], s);
   enqueue_mid(h);
   if (timed) cudaEventRecord(h->ev[4], s);
-  enqueue_stencil(h, GRIM_FULL_STEP);
-  if (timed) cudaEventRecord(h->ev[5], s);
-  const bool nanCounted = enqueue_newton(h, GRIM_FULL_STEP, false, true);
+  const bool nanCounted = enqueue_stage(h, GRIM_FULL_STEP, false, true, timed ? h->ev[5] : nullptr);
   if (timed) cudaEventRecord(h->ev[6], s);
   enqueue_post(h, timed, nanCounted);
 }
