@@ -393,12 +393,15 @@ __global__ void k_ct_t_raw(DevCfg c, const double* __restrict__ ebar, double* __
 // finite).
 template <int C, int V, int DIR, bool LEFT, class GT>
 GRIM_D double face_lane(const DevCfg& c, int x, const GT& G, const double* ps, const double* po, int lane,
-                        const double* fbIn) {
+                        const double* fb) {
   constexpr int NF = 5 + C + V, DOF = NF + 3;
   constexpr int fd = DIR + 1;  // at compile time: the element stays in registers
   typedef Dual<double, 1> D;
-  double Uo[DOF], Fo[DOF], mno, mxo;
+  // the other state, reduced at once to its speeds, its sums over the rows
+  // from 1 on, and its row 0 (which the flux filter below may drop)
+  double mno, mxo, Fo0, Uo0, sFo = 0., sUo = 0.;
   {
+    double Uo[DOF], Fo[DOF];
     ElemT<double, double> e;
     elem_rows<C, V>(e, c, po, G);
     fluxes_fluid<C, V>(e, fd, G.g, Fo, 5, 5 + C);
@@ -406,6 +409,14 @@ GRIM_D double face_lane(const DevCfg& c, int x, const GT& G, const double* ps, c
     fluxes_fluid<C, V>(e, 0, G.g, Uo, 5, 5 + C);
     fluxes_B(e, 0, G.g, Uo + NF);
     char_speeds<C, V>(e, G, DIR, c, mno, mxo);
+    Fo0 = Fo[0];
+    Uo0 = Uo[0];
+#pragma unroll
+    for (int r = 1; r < DOF; r++)
+      if (fb[r] != 0.) {
+        sFo += fb[r] * Fo[r];
+        sUo += fb[r] * Uo[r];
+      }
   }
   D q[DOF];
 #pragma unroll
@@ -427,30 +438,36 @@ GRIM_D double face_lane(const DevCfg& c, int x, const GT& G, const double* ps, c
   fluxes_B(e, fd, G.g, Fs + NF);
   const bool hll = c.riemann == GRIM_HLL;
   const D cm = dmax2(cmax, -cmin);
-  double fb[DOF];
-#pragma unroll
-  for (int r = 0; r < DOF; r++) fb[r] = fbIn[r];
+  double fb0 = fb[0];
   if constexpr (!GT::flat && DIR == 0) {
     // the torus flux filter on the density flux of the inner / outer X1
     // faces: min(F, 0) / max(F, 0), so its derivative is 1 or 0
     if (c.problem == GRIM_PROBLEM_TORUS && (x == c.g1 || x == c.N1 + c.g1)) {
-      const double FL = LEFT ? Fs[0].v : Fo[0], FR = LEFT ? Fo[0] : Fs[0].v;
-      const double dU = LEFT ? Uo[0] - Us[0].v : Us[0].v - Uo[0];
+      const double FL = LEFT ? Fs[0].v : Fo0, FR = LEFT ? Fo0 : Fs[0].v;
+      const double dU = LEFT ? Uo0 - Us[0].v : Us[0].v - Uo0;
       const double F0 = hll ? (cmax.v * FL - cmin.v * FR + cmin.v * cmax.v * dU) / (cmax.v - cmin.v)
                             : 0.5 * (FL + FR - cm.v * dU);
-      if ((x == c.g1 && F0 > 0.) || (x == c.N1 + c.g1 && F0 < 0.)) fb[0] = 0.;
+      if ((x == c.g1 && F0 > 0.) || (x == c.N1 + c.g1 && F0 < 0.)) fb0 = 0.;
     }
   }
-  double sFo = 0., sFs = 0., dFs = 0., sdU = 0., dUs = 0.;
+  double sFs = 0., dFs = 0., sUs = 0., dUs = 0.;
 #pragma unroll
-  for (int r = 0; r < DOF; r++)
+  for (int r = 1; r < DOF; r++)
     if (fb[r] != 0.) {
-      sFo += fb[r] * Fo[r];
       sFs += fb[r] * Fs[r].v;
       dFs += fb[r] * Fs[r].d[0];
-      sdU += fb[r] * (Uo[r] - Us[r].v);
+      sUs += fb[r] * Us[r].v;
       dUs += fb[r] * Us[r].d[0];
     }
+  if (fb0 != 0.) {
+    sFo += fb0 * Fo0;
+    sUo += fb0 * Uo0;
+    sFs += fb0 * Fs[0].v;
+    dFs += fb0 * Fs[0].d[0];
+    sUs += fb0 * Us[0].v;
+    dUs += fb0 * Us[0].d[0];
+  }
+  const double sdU = sUo - sUs;
   if (!hll) {
     const double j = cm.v * dUs - cm.d[0] * sdU;
     return 0.5 * (LEFT ? dFs + j : dFs - j);
@@ -473,24 +490,27 @@ GRIM_D double face_lane(const DevCfg& c, int x, const GT& G, const double* ps, c
 // and gr = (dF/dpr)^T Fbar (pr: the left-face state of b), into gface
 // (rows 0..dof-1 gl, dof..2 dof-1 gr; zero on the faces the stencil does
 // not use).
-// A block takes 32 faces with one warp per variable: warp v reconstructs
-// variable v's two states into shared memory, then runs the tangent lane of
-// variable v on each side (one-lane tangents: the element, its fluxes and
+// A block takes 16 faces with half a warp per variable: it reconstructs
+// the variable's two states into shared memory, then runs the tangent lane of
+// the variable on each side (one-lane tangents: the element, its fluxes and
 // the speeds fit in registers; the other state is plain values).  Bound by
-// FP64 latency at the occupancy of its registers (206 in 2D ideal MHD, one
-// block per SM).  One thread per face with all dof lanes together kept its
-// tangents in local memory and took 357 us per launch at 192^2, three
-// quarters of a gradient; a gradient through 10 steps there went from 22.8
-// to 7.7 ms with this split and the row-parallel gathers below.
+// FP64 latency at the occupancy of its registers: 16 faces per block and three
+// blocks per SM (168 registers, 80 bytes of spills) against one block of 32
+// faces (206 registers, 64 us per launch at 192^2): a gradient through 10
+// steps there takes 6.6 instead of 7.5 ms; a fourth block spills more than it
+// hides (6.8).  One thread per face with all dof lanes together kept its
+// tangents in local memory and took 357 us per launch (22.8 ms per gradient,
+// three quarters of it in this kernel).
+constexpr int kFacesT = 16;  // faces per block
 template <int C, int V, bool FLAT, int DIR>
-__global__ void __launch_bounds__(32 * (8 + C + V)) k_faces_t(DevCfg c, const double* __restrict__ geoF,
+__global__ void __launch_bounds__(kFacesT * (8 + C + V), (C || V) ? 1 : 3) k_faces_t(DevCfg c, const double* __restrict__ geoF,
                                                                const double* __restrict__ P,
                                                                const double* __restrict__ Ft,
                                                                double* __restrict__ gface) {
   constexpr int DOF = 8 + C + V, dir = DIR;
-  __shared__ double sl[DOF][32], sr[DOF][32], sf[DOF][32];
-  const int t = threadIdx.x & 31, v = threadIdx.x >> 5;
-  const long long z = (long long)blockIdx.x * 32 + t;
+  __shared__ double sl[DOF][kFacesT], sr[DOF][kFacesT], sf[DOF][kFacesT];
+  const int t = threadIdx.x % kFacesT, v = threadIdx.x / kFacesT;
+  const long long z = (long long)blockIdx.x * kFacesT + t;
   const long long Z = c.Z, s = stride_of(c, dir);
   int i = 0, j = 0, k = 0, x = 0;
   bool in = false;
@@ -1194,7 +1214,7 @@ static void stencil_q(const DevCfg& c, const AdjointGeo& geo, const double* P, c
   k_ct_t_raw<<<nblk(c.Z, 256), 256, 0, s>>>(c, ebar, Ft);
   cudaMemsetAsync(q, 0, (size_t)c.dof * bZ, s);
   const bool flat = c.metric == GRIM_MINKOWSKI;
-  const unsigned nb = nblk(c.Z, 32);
+  const unsigned nb = nblk(c.Z, kFacesT);
   for (int d = 0; d < c.dim; d++) {
 #define GRIM_FACES_T(C, V)                                                                 \
   do {                                                                                     \
@@ -1204,7 +1224,7 @@ static void stencil_q(const DevCfg& c, const AdjointGeo& geo, const double* P, c
                        : (d == 0   ? &k_faces_t<C, V, false, 0>                            \
                           : d == 1 ? &k_faces_t<C, V, false, 1>                            \
                                    : &k_faces_t<C, V, false, 2>);                          \
-    kernel<<<nb, 32 * (8 + C + V), 0, s>>>(c, geo.geoF[d], P, Ft, gface);                  \
+    kernel<<<nb, kFacesT * (8 + C + V), 0, s>>>(c, geo.geoF[d], P, Ft, gface);                  \
   } while (0)
     if (c.conduction && c.viscosity) GRIM_FACES_T(1, 1);
     else if (c.conduction) GRIM_FACES_T(1, 0);
