@@ -528,14 +528,6 @@ static void enqueue_dt_speeds(grim_handle* h, const double* p, int mode) {
   g_launch_counter++;
 }
 
-// torus: setProblemSpecificBCs (inflow check + pole fix) after the
-// stage-start boundary fill (timestep.cpp:17-22, :186-191)
-static void enqueue_problem_bcs(grim_handle* h, double* p) {
-  if (h->cfg.problem != GRIM_PROBLEM_TORUS) return;
-  PROF(GRIM_PROF_BOUNDARY);
-  KNS_CALL(h, torus_bcs, h->dc, p, h->geo[GRIM_CENTER], h->stream);
-  g_launch_counter += 2;
-}
 // fullStepDiagnostics: NaN reset + floors on primOld (torus/problem.cpp:719-746)
 static void enqueue_full_diagnostics(grim_handle* h) {
   if (h->cfg.problem != GRIM_PROBLEM_TORUS) return;
@@ -546,12 +538,18 @@ static void enqueue_full_diagnostics(grim_handle* h) {
   g_launch_counter += 2;
 }
 
-// the stage-start boundary fill; with no outflow or mirror side (a periodic
+// the stage-start boundary fill, for the torus with setProblemSpecificBCs
+// (inflow check and pole fix, timestep.cpp:17-22, :186-191); with no outflow or mirror side (a periodic
 // side leaves its whole direction to grid::communicate) it would change
 // nothing and is not launched
-static void enqueue_ghost_fill(grim_handle* h, double* p) {
+static void enqueue_boundaries(grim_handle* h, double* p) {
   const DevCfg& c = h->dc;
   PROF(GRIM_PROF_BOUNDARY);
+  if (h->cfg.problem == GRIM_PROBLEM_TORUS) {
+    KNS_CALL(h, torus_bcs, c, p, h->geo[GRIM_CENTER], h->stream);
+    g_launch_counter += c.dim >= 2 ? 2 : 1;
+    return;
+  }
   bool fills = false;
   for (int d = 0; d < c.dim; d++) {
     const int lo = c.bc[2 * d], hi = c.bc[2 * d + 1];
@@ -577,8 +575,7 @@ static void enqueue_pre_half(grim_handle* h, bool timed) {
     g_launch_counter++;
   }
   // ---- half stage
-  enqueue_ghost_fill(h, h->primOld);
-  enqueue_problem_bcs(h, h->primOld);
+  enqueue_boundaries(h, h->primOld);
   if (!h->cfg.elemOldFromFullStep) enqueue_dt_speeds(h, h->primOld, 0);
   if (timed) cudaEventRecord(h->ev[1], s);
 }
@@ -594,8 +591,7 @@ static void enqueue_mid_finish(grim_handle* h) {
 }
 // the full stage's boundaries on primHalfStep
 static void enqueue_mid_fill(grim_handle* h) {
-  enqueue_ghost_fill(h, h->primHalf);
-  enqueue_problem_bcs(h, h->primHalf);
+  enqueue_boundaries(h, h->primHalf);
 }
 static void enqueue_mid(grim_handle* h) {
   enqueue_mid_finish(h);
@@ -1451,8 +1447,7 @@ int grim_stage_setup(grim_handle* h, int stage) {
   CK(cudaSetDevice(h->device));
   const DevCfg& c = h->dc;
   double* ps = (stage == GRIM_HALF_STEP) ? h->primOld : h->primHalf;
-  KNS_CALL(h, ghost_fill, c, ps, c.dof, h->stream);
-  enqueue_problem_bcs(h, ps);
+  enqueue_boundaries(h, ps);
   enqueue_stencil(h, stage);
   h->lastStage = stage;
   h->stageReady = true;

@@ -211,18 +211,10 @@ static __global__ void k_nan_flag(DevCfg c, const double* __restrict__ p, unsign
   if (threadIdx.x == 0 && bad) atomicAdd(flag, (unsigned long long)bad);
 }
 
-// inflowCheck (problem.cpp:941-1044) on the X1 ghost zones
+// inflowCheck (problem.cpp:941-1044) on one X1 ghost zone
 template <int COND, int VISC>
-__global__ void k_torus_inflow(DevCfg c, TorusCfg t, double* __restrict__ p, const double* __restrict__ geoC) {
-  // one thread per (ghost i, j, k); 2*ng columns of X1 ghosts
-  long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long cols = (long long)2 * c.ng * c.N2T * c.N3T;
-  if (n >= cols) return;
-  const int gi = (int)(n % (2 * c.ng));
-  const long long r = n / (2 * c.ng);
-  const int j = (int)(r % c.N2T), k = (int)(r / c.N2T);
-  const bool right = gi >= c.ng;
-  const int i = right ? (c.N1 + c.ng + (gi - c.ng)) : gi;
+GRIM_D void inflow_zone(const DevCfg& c, const TorusCfg& t, double* p, const double* geoC, int i, int j, int k) {
+  const bool right = i >= c.ng;
   const long long Z = c.Z;
   const long long z = zidx(c, i, j, k);
   ZoneGeo<double> G;
