@@ -141,7 +141,7 @@ GRIM_D bool same_sign(S a, S b) { return (a < S(0.)) == (b < S(0.)); }
 template <class S>
 GRIM_D S ppm_half_slope(S a, S b) {
   const S m = fmin(S(0.25) * fabs(a + b), fmin(fabs(a), fabs(b)));
-  return same_sign(a, b) ? (a < S(0.) ? -m : m) : S(0.);
+  return same_sign(a, b) ? copysign(m, a) : S(0.);  // the sign by a bit operation, not a compare
 }
 template <class S>
 GRIM_D void ppm_offsets(S y0, S y1, S y2, S y3, S y4, S& al, S& ar) {
@@ -191,7 +191,7 @@ GRIM_D void weno5_faces_fast(S y0, S y1, S y2, S y3, S y4, S& lo, S& ro) {
 template <class S>
 GRIM_D S slope_mm_fast(S bwd, S fwd, double theta) {
   const S m = fmin(S(0.5) * fabs(bwd + fwd), theta * fmin(fabs(bwd), fabs(fwd)));
-  return same_sign(bwd, fwd) ? (bwd < S(0.) ? -m : m) : S(0.);
+  return same_sign(bwd, fwd) ? copysign(m, bwd) : S(0.);
 }
 
 // face values of zone i
