@@ -793,6 +793,13 @@ static __global__ void k_emf(DevCfg c, const double* __restrict__ F1, const doub
 // stream that wants warps in flight more than registers (measured on the
 // 3D torus: 64 registers with a few spills beat 85 and 98 without)
 constexpr int kEpiMinBlocks[3] = {4, 5, 8};
+// extended MHD: the Kerr-Schild centre half needs 168 registers (96 spilled
+// 272 bytes), the flux half 80 (64 spilled 256); epilogue of the EMHD torus
+// 96x64x32, us per step: 177 -> 157
+constexpr int epi_min_blocks(int part, bool emhd, bool flat) {
+  if (!emhd) return kEpiMinBlocks[part];
+  return part == 1 ? (flat ? 5 : 3) : 6;
+}
 template <int COND, int VISC, bool FLAT, int PART>
 GRIM_D void epilogue_zone(const DevCfg& c, int stage, const StageBufs& b, long long n) {
   constexpr int NF = 5 + COND + VISC;
@@ -1085,7 +1092,7 @@ GRIM_D void epilogue_zone(const DevCfg& c, int stage, const StageBufs& b, long l
 }
 
 template <int COND, int VISC, bool FLAT, int PART>
-__global__ void __launch_bounds__(128, kEpiMinBlocks[PART]) k_stage_epilogue(DevCfg c, int stage, StageBufs b) {
+__global__ void __launch_bounds__(128, epi_min_blocks(PART, COND || VISC, FLAT)) k_stage_epilogue(DevCfg c, int stage, StageBufs b) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n < c.Zint) epilogue_zone<COND, VISC, FLAT, PART>(c, stage, b, n);
 }
