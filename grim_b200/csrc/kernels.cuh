@@ -1806,8 +1806,15 @@ GRIM_D bool fast_newton_final(const DevCfg& c, const StageConst<5 + COND + VISC>
 // of spills in Kerr-Schild, none in Minkowski) takes 495 us per torus step, 3
 // (168, none) 525.
 constexpr int kNewtonMinBlocks = 4;
+// dst non-null (ideal MHD in Minkowski, every active direction periodic): the
+// stage's finish too.  The zone's result goes to dst, and to the ghost zones
+// that grid::communicate copies it into (the zone shifted by the grid's size
+// along each direction); after the full stage also its term of the next
+// computeDt, the non-finite count and the time advance, as k_stage_finish.
 template <int COND, int VISC, bool FLAT, class T>
-GRIM_D void newton_block(const DevCfg& c, int stage, const StageBufs& b) {
+GRIM_D void newton_block(const DevCfg& c, int stage, const StageBufs& b, double* dst = nullptr, int dtOn = 0) {
+  [[maybe_unused]] double best = 0.;
+  [[maybe_unused]] int bad = 0;
   constexpr int NF = 5 + COND + VISC;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   int unconv = 0, itsMax = 0;
@@ -1833,6 +1840,32 @@ GRIM_D void newton_block(const DevCfg& c, int stage, const StageBufs& b) {
     itsMax = it;
 #pragma unroll
     for (int v = 0; v < NF; v++) b.prim[(long long)v * Z + z] = P[v];
+    if constexpr (FLAT && !COND && !VISC)
+      if (dst) {
+        double q[8];
+#pragma unroll
+        for (int v = 0; v < 5; v++) q[v] = P[v];
+#pragma unroll
+        for (int v = 0; v < 3; v++) q[5 + v] = K.B[v];
+        for (int kk = k - (c.dim > 2 ? c.N3 : 0); kk < c.N3T; kk += c.N3) {
+          if (kk < 0) continue;
+          for (int jj = j - (c.dim > 1 ? c.N2 : 0); jj < c.N2T; jj += c.N2) {
+            if (jj < 0) continue;
+            for (int ii = i - c.N1; ii < c.N1T; ii += c.N1) {
+              if (ii < 0) continue;
+              const long long zz = zidx(c, ii, jj, kk);
+#pragma unroll
+              for (int v = 0; v < 8; v++) dst[(long long)v * Z + zz] = q[v];
+            }
+          }
+        }
+        if (stage == GRIM_FULL_STEP) {
+          if (dtOn) best = zone_inv_dt<0, 0>(c, q, G);
+#pragma unroll
+          for (int v = 0; v < 8; v++)
+            if (!isfinite(q[v])) bad = 1;
+        }
+      }
     if (b.nanCount) {
 #pragma unroll
       for (int v = 0; v < NF; v++) nanZone |= isnan(P[v]);
@@ -1851,6 +1884,13 @@ GRIM_D void newton_block(const DevCfg& c, int stage, const StageBufs& b) {
     if (nUnconv) atomicAdd(&b.st->finalUnconv[stage], (unsigned long long)nUnconv);
     if (nNan) atomicAdd(b.nanCount, (unsigned long long)nNan);
   }
+  if constexpr (FLAT && !COND && !VISC)
+    if (dst && stage == GRIM_FULL_STEP) {
+      if (blockIdx.x == 0 && threadIdx.x == 0) b.st->time += b.st->dt;  // nothing in this kernel reads it
+      block_max_to(best, &b.st->maxInvDt);
+      bad = __syncthreads_count(bad);
+      if (threadIdx.x == 0 && bad) atomicAdd(&b.st->nonFinite, (unsigned long long)bad);
+    }
 }
 
 template <int COND, int VISC, bool FLAT, class T>
@@ -1861,10 +1901,10 @@ __global__ void __launch_bounds__(128, (COND || VISC || sizeof(T) == 8) ? 1 : kN
 // launch: nothing of a zone's solve depends on another zone's epilogue, and a
 // thread reads back only what it wrote itself.
 template <bool FLAT, class T>
-__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 1 : kNewtonMinBlocks) k_stage_solve(DevCfg c, int stage, StageBufs b) {
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 1 : kNewtonMinBlocks) k_stage_solve(DevCfg c, int stage, StageBufs b, double* dst, int dtOn) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (n < c.Zint) epilogue_zone<0, 0, FLAT, FLAT ? 0 : 2>(c, stage, b, n);
-  newton_block<0, 0, FLAT, T>(c, stage, b);
+  newton_block<0, 0, FLAT, T>(c, stage, b, dst, dtOn);
 }
 
 #ifdef GRIM_FAST_MATH
@@ -2546,11 +2586,11 @@ void newton_fast(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaS
   GRIM_GEO_DISPATCH(c, newton_fast_t, c, stage, b, mode, s);
 }
 #ifdef GRIM_FAST_MATH
-void stage_solve(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s) {
+void stage_solve(const DevCfg& c, int stage, const StageBufs& b, int mode, double* dst, int dtOn, cudaStream_t s) {
   auto kernel = mode == GRIM_NEWTON_MIXED32
                     ? (c.metric == GRIM_MINKOWSKI ? &k_stage_solve<true, float> : &k_stage_solve<false, float>)
                     : (c.metric == GRIM_MINKOWSKI ? &k_stage_solve<true, double> : &k_stage_solve<false, double>);
-  kernel<<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b);
+  kernel<<<nblk(c.Zint, 128), 128, 0, s>>>(c, stage, b, dst, dtOn);
 }
 #endif
 

@@ -100,8 +100,9 @@ void adjoint_stencil_t(const DevCfg& c, const AdjointGeo& geo, const double* P, 
 namespace grim {
 namespace fast {
 // the flux half of the epilogue and the per-zone Newton in one launch (ideal
-// MHD)
-void stage_solve(const DevCfg& c, int stage, const StageBufs& b, int mode, cudaStream_t s);
+// MHD); with dst (Minkowski, every active direction periodic) also the
+// stage's finish into dst
+void stage_solve(const DevCfg& c, int stage, const StageBufs& b, int mode, double* dst, int dtOn, cudaStream_t s);
 // the deferred-tail Newton (ideal MHD, mixed form, maxIter >= 2): one
 // persistent launch per stage; false when the configuration is not one it
 // runs (the caller then runs newton_fast)
