@@ -1607,12 +1607,18 @@ __global__ void __launch_bounds__(128) k_newton_fd_init(DevCfg c, int stage, Sta
   if (threadIdx.x == 0 && unconv) atomicAdd(&b.st->count[stage][0], (unsigned long long)unconv);
 }
 
+// Blocks per SM of the FD iteration: ideal MHD in Kerr-Schild takes 204
+// registers unbounded, two blocks; three (168, 216 bytes of spills) take the
+// ragged torus 99x71x33 from 2241 to 2022 us per two steps.  In Minkowski (150
+// registers, three blocks) a fourth costs more in spills than it hides (128^2
+// wave 149 -> 154), and extended MHD needs the 255.
+constexpr int fd_min_blocks(bool emhd, bool flat) { return !emhd && !flat ? 3 : 1; }
 // Parity Newton, iteration `it` (solve.cpp:80-199): FD Jacobian, pivoted
 // solve, quadratic backtracking, update; then the floor + residual + count
 // of iteration it+1.  Returns at once when iteration `it` found every zone
 // converged (the reference's global break).
 template <int COND, int VISC, bool FLAT>
-__global__ void __launch_bounds__(128) k_newton_fd_iter(DevCfg c, int stage, int it, StageBufs b) {
+__global__ void __launch_bounds__(128, fd_min_blocks(COND || VISC, FLAT)) k_newton_fd_iter(DevCfg c, int stage, int it, StageBufs b) {
   constexpr int NF = 5 + COND + VISC;
   if (b.st->count[stage][it] == 0ULL) return;
   long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
