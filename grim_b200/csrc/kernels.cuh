@@ -17,6 +17,7 @@
 //   k_newton_*         per-zone Newton (solve.cpp / residual.cpp)
 #pragma once
 #include <algorithm>
+#include <type_traits>
 
 #include "physics.cuh"
 #include "recon.cuh"
@@ -1445,6 +1446,17 @@ GRIM_D void load_stage_const(StageConst<5 + COND + VISC>& K, const DevCfg& c, in
 #pragma unroll
       for (int m = 0; m < 4; m++) g0[m] = G.gcon[0][m];
     }
+    if constexpr (!GT::flat) {  // the FP32 Jacobian's constants (emhd_tangents)
+      K.refRho = er.rho; K.refNu = VISC ? er.nu : 0.; K.refChi = COND ? er.chi : 0.;
+      K.refTau = er.tau; K.refT = er.temperature;
+#pragma unroll
+      for (int m = 0; m < 4; m++) K.refBCon[m] = er.bCon[m];
+      K.refBSqr = er.bSqr; K.refBNorm = er.bNorm; K.refUCon0 = er.uCon[0];
+      K.refQTilde = COND ? er.qTilde : 0.;
+      K.refDPTilde = VISC ? er.deltaPTilde : 0.;
+      if (COND) K.normQ = (c.hoCond) ? er.temperature * sqrt(er.rho * er.chi * er.tau) : er.tau;
+      if (VISC) K.normDP = (c.hoVisc) ? sqrt(er.rho * er.nu * er.temperature * er.tau) : er.tau;
+    }
     K.rowT = 0.;
     if (COND) {
       const double norm = (c.hoCond) ? er.temperature * sqrt(er.rho * er.chi * er.tau) : er.tau;
@@ -1720,7 +1732,12 @@ GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>&
   D Pd[NF], Rd[NF];
 #pragma unroll
   for (int v = 0; v < NF; v++) Pd[v] = D::var((T)P[v], v);
-  zone_residual<COND, VISC, D, T>(Pd, K, Gt, c, Rd);
+#ifdef GRIM_FAST_MATH
+  if constexpr ((COND || VISC) && !GT::flat && std::is_same<T, float>::value)
+    emhd_tangents<COND, VISC, D, T>(Pd, K, Gt, c, Rd);
+  else
+#endif
+    zone_residual<COND, VISC, D, T>(Pd, K, Gt, c, Rd);
 #pragma unroll
   for (int r = 0; r < NF; r++)
 #pragma unroll

@@ -714,8 +714,8 @@ struct StageConst {
   // is fixed for the stage, so it is folded into these once per zone:
   //   R_q  = rowU U_q / sqrt(-g) + rowP q~  + rowK + sum_mu rowA_mu (u_mu - uOld_mu) + rowT (T - TOld)
   // (row 0: q, row 1: deltaP, whose rowT is zero).  A residual then has no
-  // division or square root of these rows, and the FP32 tangent pass
-  // neither.  With the speeds' and the sources' divisions hoisted the same
+  // division or square root of these rows, and in Minkowski the FP32 tangent
+  // pass neither (in Kerr-Schild it has expressions of its own, emhd_tangents).  With the speeds' and the sources' divisions hoisted the same
   // way (us per step, one B200): EMHD torus 96x64x32 1735 -> 915, 256^2
   // stratified 299 -> 224.
   double rowU[2], rowP[2], rowK[2], rowA[2][4], rowT;
@@ -822,5 +822,97 @@ GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, cons
   }
 #endif
 }
+
+#ifdef GRIM_FAST_MATH
+// The extended-MHD residual's tangents for the FP32 Jacobian in Kerr-Schild,
+// in the plain expressions (lowered u^mu, quotients where they stand, the q
+// and deltaP rows term by term).  A few torus zones take all their updates
+// without converging, and there an update's last FP32 bits decide what the
+// capped Newton returns (to 0.2 of a velocity in a zone of 2e5), while the
+// converged solutions agree to 1e-9: the Jacobian's roundings are kept, the
+// FP64 residual has the folded form (folded Jacobian and residual took the
+// 96x64x32 torus 690 us per step, this 774, both unfolded 1737).  P holds the unknowns' tangents; only
+// the tangents of Rout are used.
+template <int COND, int VISC, class S, class T>
+GRIM_D void emhd_tangents(const S* P, const StageConst<5 + COND + VISC>& K, const ZoneGeo<T>& G, const DevCfg& c,
+                          S* Rout) {
+  constexpr int NF = 5 + COND + VISC, Q = 5, DP = 5 + COND;
+  const T Gam = (T)c.Gam;
+  const T B1 = (T)K.B[0], B2 = (T)K.B[1], B3 = (T)K.B[2];
+  const S v1 = P[2], v2 = P[3], v3 = P[4];
+  const S rho = dmaxc(P[0], (T)c.rhoFloor), u = dmaxc(P[1], (T)c.uFloor);
+  const S pressure = (Gam - T(1.)) * u;
+  const S temperature = dmaxc(pressure / rho, (T)c.TFloor);
+  const S cs = dsqrt(Gam * pressure / (rho + Gam * u));
+  const S gsq = T(1) + G.gcov[1][1] * v1 * v1 + G.gcov[2][2] * v2 * v2 + G.gcov[3][3] * v3 * v3 +
+                T(2) * (G.gcov[1][2] * v1 * v2 + G.gcov[1][3] * v1 * v3 + G.gcov[2][3] * v2 * v3);
+  const S rgam = drsqrt(gsq);
+  const S gam = gsq * rgam;
+  S uCon[4], uCov[4], bCon[4], bCov[4];
+  uCon[0] = gam * G.ialpha;
+  uCon[1] = v1 - gam * G.gcon[0][1] * G.alpha;
+  uCon[2] = v2 - gam * G.gcon[0][2] * G.alpha;
+  uCon[3] = v3 - gam * G.gcon[0][3] * G.alpha;
+#pragma unroll
+  for (int m = 0; m < 4; m++) uCov[m] = lower(G, m, uCon);
+  bCon[0] = B1 * uCov[1] + B2 * uCov[2] + B3 * uCov[3];
+  const S iu0 = G.alpha * rgam;
+  bCon[1] = (B1 + bCon[0] * uCon[1]) * iu0;
+  bCon[2] = (B2 + bCon[0] * uCon[2]) * iu0;
+  bCon[3] = (B3 + bCon[0] * uCon[3]) * iu0;
+#pragma unroll
+  for (int m = 0; m < 4; m++) bCov[m] = lower(G, m, bCon);
+  const S bSqr = bCon[0] * bCov[0] + bCon[1] * bCov[1] + bCon[2] * bCov[2] + bCon[3] * bCov[3] + (T)c.bSqrFloor;
+  const S bNorm = dsqrt(bSqr);
+  S q = COND ? P[Q] : S(T(0)), dP = VISC ? P[DP] : S(T(0));
+  if (COND && c.hoCond == 1) q = P[Q] * temperature * dsqrt(rho * (T)c.CondAlpha * cs * cs);
+  if (VISC && c.hoVisc == 1) dP = P[DP] * dsqrt(temperature * rho * (T)c.ViscAlpha * cs * cs);
+  const S w = rho + u + pressure + bSqr, pt = pressure + T(0.5) * bSqr;
+  const S fr = G.g * (rho * uCon[0]);
+  S U[NF];
+  U[0] = fr;
+#pragma unroll
+  for (int nu = 0; nu < 4; nu++) {
+    const T d = (nu == 0) ? T(1.) : T(0.);
+    S r = w * uCon[0] * uCov[nu] + pt * d - bCon[0] * bCov[nu];
+    if (COND) r += q / bNorm * (uCon[0] * bCov[nu] + bCon[0] * uCov[nu]);
+    if (VISC) r += (-dP) * (bCon[0] * bCov[nu] / bSqr - T(1. / 3.) * (d + uCon[0] * uCov[nu]));
+    U[1 + nu] = nu == 0 ? G.g * r + fr : G.g * r;
+  }
+  if (COND) U[Q] = G.g * (uCon[0] * P[Q]);
+  if (VISC) U[DP] = G.g * (uCon[0] * P[DP]);
+  const T dtp = (T)K.dtp;
+#pragma unroll
+  for (int v = 0; v < NF; v++) Rout[v] = U[v] / dtp;
+  S dtu[4];
+#pragma unroll
+  for (int m = 0; m < 4; m++) dtu[m] = uCov[m] / dtp;
+  S div = S(T(0.));
+#pragma unroll
+  for (int m = 0; m < 4; m++) div = div + G.gcon[0][m] * dtu[m];
+  const T rr = (T)K.refRho, rnu = (T)K.refNu, rchi = (T)K.refChi, rtau = (T)K.refTau, rT = (T)K.refT;
+  const T rbn = (T)K.refBNorm, rbs = (T)K.refBSqr;
+  if (VISC) {
+    S d0 = -div * rr * rnu;
+#pragma unroll
+    for (int m = 0; m < 4; m++) d0 += T(3.) * rr * rnu * (T)K.refBCon[0] * (T)K.refBCon[m] / rbs * dtu[m];
+    if (c.hoVisc == 1) d0 = d0 * (T)sqrt((double)(rtau / rr / rnu / rT));
+    S sdt = -G.g * (d0) / rtau;
+    if (c.hoVisc == 1) sdt = sdt - T(0.5) * G.g * div * (T)K.refDPTilde;
+    const S simp = G.g * (P[DP]) / rtau;
+    Rout[DP] = (Rout[DP] + T(0.5) * simp + sdt) * (T)K.normDP;
+  }
+  if (COND) {
+    S qq = -rr * rchi * (T)K.refBCon[0] / rbn * temperature / dtp;
+#pragma unroll
+    for (int m = 0; m < 4; m++) qq -= rr * rchi * rT * (T)K.refBCon[m] / rbn * (T)K.refUCon0 * dtu[m];
+    if (c.hoCond == 1) qq = qq * ((T)sqrt((double)(rtau / rr / rchi)) / rT);
+    S sdt = -G.g * (qq) / rtau;
+    if (c.hoCond == 1) sdt = sdt - T(0.5) * G.g * div * (T)K.refQTilde;
+    const S simp = G.g * (P[Q]) / rtau;
+    Rout[Q] = (Rout[Q] + T(0.5) * simp + sdt) * (T)K.normQ;
+  }
+}
+#endif
 
 }  // namespace grim
