@@ -104,18 +104,25 @@ static __global__ void k_ghost_fill(DevCfg c, double* __restrict__ prim, int nv)
   ghost_ijk(c, n, i, j, k);
   fill_zone(c, prim, nv, i, j, k);
 }
-// The same with the torus's inflow check of the X1 ghost zones, which reads
-// and writes the zone it checks only: one dependent launch fewer at the start
-// of each stage (boundary launches 59 -> 45 us per step on the torus
-// 256x128x64, event overhead included; the 64x48x24 step 116 -> 109 us).
-template <int COND, int VISC>
+// The torus's X1 ghost zones: FILL, the fill of every ghost zone and the
+// inflow check of those along X1 in one launch; not FILL, the inflow check
+// alone, after k_ghost_fill.  The check rewrites its own zone, so one launch
+// may do both only where no ghost zone's fill reads an X1 ghost zone, which is
+// when the fill maps every X1 index to the interior: both X1 sides outflow or
+// mirror (torus_fill_checks).  A periodic or exchanged X1 side keeps its
+// columns, and a ghost plane of X2 or X3 then copies from zones the check
+// rewrites.  One dependent launch fewer at the start of each stage: boundary
+// launches 59 -> 45 us per step on the torus 256x128x64, event overhead
+// included; the 64x48x24 step 116 -> 109 us.
+template <int COND, int VISC, bool FILL>
 __global__ void __launch_bounds__(128) k_torus_ghosts(DevCfg c, TorusCfg t, double* prim, const double* __restrict__ geoC) {
   const long long n = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= c.Z - c.Zint) return;
+  // the X1 ghost columns come first in ghost_ijk's order
+  if (n >= (FILL ? c.Z - c.Zint : 2LL * c.g1 * c.N2T * c.N3T)) return;
   int i, j, k;
   ghost_ijk(c, n, i, j, k);
-  fill_zone(c, prim, 8 + COND + VISC, i, j, k);
-  if (i < c.g1 || i >= c.N1 + c.g1) inflow_zone<COND, VISC>(c, t, prim, geoC, i, j, k);
+  if constexpr (FILL) fill_zone(c, prim, 8 + COND + VISC, i, j, k);
+  if (!FILL || i < c.g1 || i >= c.N1 + c.g1) inflow_zone<COND, VISC>(c, t, prim, geoC, i, j, k);
 }
 
 // grid::communicate (grid.cpp:306-360) with PETSc DMDA semantics: periodic
@@ -2730,7 +2737,12 @@ void torus_nan_flag(const DevCfg& c, const double* p, unsigned long long* flag, 
 }
 template <int C, int V>
 static void torus_bcs_t(const DevCfg& c, double* p, const double* geoC, cudaStream_t s) {
-  k_torus_ghosts<C, V><<<nblk(c.Z - c.Zint, 128), 128, 0, s>>>(c, torus_cfg(c), p, geoC);
+  if (torus_fill_checks(c)) {
+    k_torus_ghosts<C, V, true><<<nblk(c.Z - c.Zint, 128), 128, 0, s>>>(c, torus_cfg(c), p, geoC);
+  } else {
+    ghost_fill(c, p, c.dof, s);
+    k_torus_ghosts<C, V, false><<<nblk(2LL * c.g1 * c.N2T * c.N3T, 128), 128, 0, s>>>(c, torus_cfg(c), p, geoC);
+  }
   if (c.dim >= 2) k_torus_poles<<<nblk(2LL * c.N1T * c.N3T, 128), 128, 0, s>>>(c, p, geoC);
 }
 void torus_bcs(const DevCfg& c, double* p, const double* geoC, cudaStream_t s) {

@@ -561,7 +561,7 @@ static void enqueue_boundaries(grim_handle* h, double* p) {
   PROF(GRIM_PROF_BOUNDARY);
   if (h->cfg.problem == GRIM_PROBLEM_TORUS) {
     KNS_CALL(h, torus_bcs, c, p, h->geo[GRIM_CENTER], h->stream);
-    g_launch_counter += c.dim >= 2 ? 2 : 1;
+    g_launch_counter += (torus_fill_checks(c) ? 1 : 2) + (c.dim >= 2 ? 1 : 0);
     return;
   }
   bool fills = false;

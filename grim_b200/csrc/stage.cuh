@@ -52,4 +52,10 @@ struct StageBufs {
                                  // rows) holds a NaN (fullStepDiagnostics' count of the full stage)
 };
 
+// whether the torus's boundary fill and its inflow check are one launch (see
+// k_torus_ghosts); otherwise torus_bcs launches the one before the other
+inline bool torus_fill_checks(const DevCfg& c) {
+  return (c.bc[0] == GRIM_OUTFLOW || c.bc[0] == GRIM_MIRROR) && (c.bc[1] == GRIM_OUTFLOW || c.bc[1] == GRIM_MIRROR);
+}
+
 }  // namespace grim
