@@ -24,6 +24,7 @@
 #include <string>
 #include <vector>
 
+#include "chains.h"
 #include "launch.h"
 
 namespace grim {
@@ -2054,11 +2055,8 @@ struct grim_batch {
   // the chains of a step: one per problem in a captured step; launched
   // eagerly, streams made at the first such step, the problems dealt to them
   // largest first so that each carries about the same number of zones
-  std::vector<cudaStream_t> chain;
-  std::vector<int> chainOf;  // per problem
-  std::vector<int> order;    // problems, largest first
-  cudaEvent_t fork = nullptr;
-  std::vector<cudaEvent_t> join;
+  Chains chains;
+  std::vector<int> order;  // problems, largest first
   bool graphOn = false;
   cudaGraphExec_t graph = nullptr;
 };
@@ -2074,33 +2072,9 @@ static void batch_free(grim_batch* B) {
     h->stream = nullptr;  // the batch's stream, destroyed below
     grim_destroy(h);
   }
-  for (cudaStream_t s : B->chain) cudaStreamDestroy(s);
-  for (cudaEvent_t e : B->join) cudaEventDestroy(e);
-  if (B->fork) cudaEventDestroy(B->fork);
+  B->chains.release();
   if (B->stream) cudaStreamDestroy(B->stream);
   delete B;
-}
-
-// streams and events of the chains, and which problem runs on which
-static int batch_chains(grim_batch* B) {
-  const int n = (int)B->h.size(), m = std::min(n, kBatchStreams);
-  for (int k = 0; k < m; k++) {
-    cudaStream_t s = nullptr;
-    CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    B->chain.push_back(s);
-    cudaEvent_t e = nullptr;
-    CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    B->join.push_back(e);
-  }
-  CK(cudaEventCreateWithFlags(&B->fork, cudaEventDisableTiming));
-  std::vector<long long> load(m, 0);
-  B->chainOf.resize(n);
-  for (int p : B->order) {
-    const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-    B->chainOf[p] = k;
-    load[k] += B->h[p]->dc.Zint;
-  }
-  return GRIM_OK;
 }
 
 int grim_batch_create(const grim_config* cfgs, int n, int device, grim_batch** out) {
@@ -2188,21 +2162,23 @@ static int enqueue_batch_step(grim_batch* B, bool capturing) {
     fork.join();
     return GRIM_OK;
   }
-  if (B->chain.empty()) {
-    const int rc = batch_chains(B);
-    if (rc) return rc;
+  Chains& ch = B->chains;
+  if (!ch.made()) {
+    std::vector<long long> zones;
+    for (grim_handle* h : B->h) zones.push_back(h->dc.Zint);
+    CK(ch.make(zones, B->order, kBatchStreams));
   }
-  CK(cudaEventRecord(B->fork, B->stream));
-  for (cudaStream_t s : B->chain) CK(cudaStreamWaitEvent(s, B->fork, 0));
+  CK(cudaEventRecord(ch.fork, B->stream));
+  for (cudaStream_t s : ch.stream) CK(cudaStreamWaitEvent(s, ch.fork, 0));
   for (int p : B->order) {
     grim_handle* h = B->h[p];
-    h->stream = B->chain[B->chainOf[p]];
+    h->stream = ch.stream[ch.of[p]];
     enqueue_step(h, false);
     h->stream = B->stream;
   }
-  for (size_t k = 0; k < B->chain.size(); k++) {
-    CK(cudaEventRecord(B->join[k], B->chain[k]));
-    CK(cudaStreamWaitEvent(B->stream, B->join[k], 0));
+  for (size_t k = 0; k < ch.stream.size(); k++) {
+    CK(cudaEventRecord(ch.join[k], ch.stream[k]));
+    CK(cudaStreamWaitEvent(B->stream, ch.join[k], 0));
   }
   return GRIM_OK;
 }
