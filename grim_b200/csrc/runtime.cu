@@ -82,6 +82,7 @@ struct grim_handle {
   bool graphOn = false;
   cudaGraphExec_t graph = nullptr;
   bool capturing = false;  // the step being enqueued is captured: it may branch (GraphFork)
+  cudaError_t captureError = cudaSuccess;  // the first of that capture's branching calls that failed
   grim_stats stats;
   long long launchesPerStep = 0;
   size_t bytesZ = 0;
@@ -354,47 +355,9 @@ static long long g_launch_counter = 0;
 // grim_newton_solve) keep it in prim
 static bool step_guess_old(const grim_handle* h) { return !is_fd(h); }
 
-// Parallel branches of a graph being captured on one stream: each branch's
-// first launch depends on what the fork's did, and what follows join()
-// depends on every branch's last launches.  Works on the capture's
-// dependency set directly, so a first step needs no side streams or events
-// (making three streams and four events took 0.35 ms of a new handle's first
-// pass).  Inactive (one stream, in order) when the stream is not capturing.
-class GraphFork {
- public:
-  GraphFork(cudaStream_t s, bool on) : s_(s), on_(on) {
-    if (on_) on_ = deps(root_);
-    open_ = false;
-  }
-  void branch() {
-    if (!on_) return;
-    if (open_) collect();
-    cudaStreamUpdateCaptureDependencies(s_, root_.data(), root_.size(), cudaStreamSetCaptureDependencies);
-    open_ = true;
-  }
-  void join() {
-    if (!on_ || !open_) return;
-    collect();
-    cudaStreamUpdateCaptureDependencies(s_, tails_.data(), tails_.size(), cudaStreamSetCaptureDependencies);
-    on_ = false;
-  }
-
- private:
-  bool deps(std::vector<cudaGraphNode_t>& out) const {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    const cudaGraphNode_t* d = nullptr;
-    size_t n = 0;
-    if (cudaStreamGetCaptureInfo_v2(s_, &st, nullptr, nullptr, &d, &n) != cudaSuccess ||
-        st != cudaStreamCaptureStatusActive)
-      return false;
-    out.insert(out.end(), d, d + n);
-    return true;
-  }
-  void collect() { deps(tails_); }
-  cudaStream_t s_;
-  bool on_, open_;
-  std::vector<cudaGraphNode_t> root_, tails_;
-};
+static void note_capture(grim_handle* h, cudaError_t e) {
+  if (h->captureError == cudaSuccess) h->captureError = e;
+}
 
 // whether direction d's face kernel is one of the TMA-staged variants, whose
 // persistent grid divides the faces over the whole GPU's resident blocks
@@ -445,6 +408,7 @@ static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false, bo
     g_launch_counter++;
   }
   fork.join();
+  note_capture(h, fork.error());
   if (!fluxHalf) return;
   KNS_CALL(h, stage_epilogue, c, stage, b, false, s);
   g_launch_counter++;
@@ -966,6 +930,19 @@ static int take_async_error(grim_handle* h) {
   return GRIM_ETIMEOUT;
 }
 
+// Ends a capture.  With an error of one of its branching calls the graph may
+// lack a dependency: it is dropped and the error returned.
+static cudaError_t end_capture(cudaStream_t s, cudaError_t branching, cudaGraph_t* g) {
+  cudaError_t e = cudaStreamEndCapture(s, g);
+  if (branching != cudaSuccess) e = branching;
+  if (e != cudaSuccess) {
+    if (*g) cudaGraphDestroy(*g);
+    *g = nullptr;
+    (void)cudaGetLastError();  // the error is reported through the return value
+  }
+  return e;
+}
+
 static int run_steps(grim_handle* h, int nsteps) {
   {
     const int rc = take_async_error(h);
@@ -977,14 +954,15 @@ static int run_steps(grim_handle* h, int nsteps) {
     const bool last = (n == nsteps - 1);
     if (h->graphOn) {
       if (!h->graph) {
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
         long long before = g_launch_counter;
         h->capturing = true;
+        h->captureError = cudaSuccess;
         enqueue_step(h, false);
         h->capturing = false;
         h->launchesPerStep = g_launch_counter - before;
-        CK(cudaStreamEndCapture(h->stream, &g));
+        CK(end_capture(h->stream, h->captureError, &g));
         cudaError_t e = cudaGraphInstantiate(&h->graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) { set_err("graph instantiate: %s", cudaGetErrorString(e)); return GRIM_ECUDA; }
@@ -2150,18 +2128,22 @@ int grim_batch_set_newton_mode(grim_batch* B, int mode, double rtol) {
 // one; side by side they fill it.  Measured on the 16-problem family (2.04 M
 // zones, one B200), us per step: problem after problem with one worklist
 // Newton per stage over all of them 1951, chains with the per-zone Newton 1192.
-static int enqueue_batch_step(grim_batch* B, bool capturing) {
-  if (capturing) {
-    GraphFork fork(B->stream, true);
-    for (int p : B->order) {
-      fork.branch();
-      B->h[p]->capturing = true;
-      enqueue_step(B->h[p], false);
-      B->h[p]->capturing = false;
-    }
-    fork.join();
-    return GRIM_OK;
+static cudaError_t capture_batch_step(grim_batch* B) {
+  GraphFork fork(B->stream, true);
+  cudaError_t e = cudaSuccess;
+  for (int p : B->order) {
+    grim_handle* h = B->h[p];
+    fork.branch();
+    h->capturing = true;
+    h->captureError = cudaSuccess;
+    enqueue_step(h, false);
+    h->capturing = false;
+    if (e == cudaSuccess) e = h->captureError;
   }
+  fork.join();
+  return e == cudaSuccess ? fork.error() : e;
+}
+static int enqueue_batch_step(grim_batch* B) {
   Chains& ch = B->chains;
   if (!ch.made()) {
     std::vector<long long> zones;
@@ -2198,18 +2180,17 @@ int grim_batch_time_steps(grim_batch* B, int nsteps) {
   for (int n = 0; n < nsteps; n++) {
     if (B->graphOn) {
       if (!B->graph) {
-        cudaGraph_t g;
+        cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = enqueue_batch_step(B, true);
-        CK(cudaStreamEndCapture(B->stream, &g));
-        if (rc) { cudaGraphDestroy(g); return rc; }
+        const cudaError_t branching = capture_batch_step(B);
+        CK(end_capture(B->stream, branching, &g));
         cudaError_t e = cudaGraphInstantiate(&B->graph, g, 0);
         cudaGraphDestroy(g);
         if (e != cudaSuccess) { set_err("batch graph instantiate: %s", cudaGetErrorString(e)); return GRIM_ECUDA; }
       }
       CK(cudaGraphLaunch(B->graph, B->stream));
     } else {
-      const int rc = enqueue_batch_step(B, false);
+      const int rc = enqueue_batch_step(B);
       if (rc) return rc;
     }
   }

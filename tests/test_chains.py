@@ -14,6 +14,8 @@ FAKES = r"""
 #include "chains.h"
 static int calls, failAt, live;  // the call to fail (-1: none), objects alive
 static cudaError_t next() { return calls++ == failAt ? cudaErrorMemoryAllocation : cudaSuccess; }
+static cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+static std::vector<cudaGraphNode_t> now;
 extern "C" {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
   const cudaError_t e = next();
@@ -23,6 +25,21 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* s, unsigned) {
   const cudaError_t e = next();
   if (!e) *s = (cudaEvent_t)(long)++live;
+  return e;
+}
+// a capture: its dependency set is what the next launch depends on
+cudaError_t cudaStreamGetCaptureInfo_v2(cudaStream_t, cudaStreamCaptureStatus* st, unsigned long long*, cudaGraph_t*,
+                                        const cudaGraphNode_t** d, size_t* n) {
+  const cudaError_t e = next();
+  if (e) return e;
+  *st = status;
+  if (d) *d = now.data();
+  if (n) *n = now.size();
+  return e;
+}
+cudaError_t cudaStreamUpdateCaptureDependencies(cudaStream_t, cudaGraphNode_t* d, size_t n, unsigned) {
+  const cudaError_t e = next();
+  if (!e) now.assign(d, d + n);
   return e;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { live--; return cudaSuccess; }
@@ -72,5 +89,66 @@ int main() {
     }
     for (int p = n; p < 40; p++) work.push_back(1000 + 37 * p);
   }
+}
+""")
+
+
+def test_a_fork_orders_its_branches_or_reports_the_failure(tmp_path):
+    _run(tmp_path, r"""
+static long node;
+static std::vector<cudaGraphNode_t> launch() {  // a launch: its dependencies, and it is the next one's
+  std::vector<cudaGraphNode_t> on = now;
+  now.assign(1, (cudaGraphNode_t)(++node));
+  return on;
+}
+int main() {
+  for (int branches = 1; branches <= 4; branches++) {
+    int total = 0;
+    for (int f = -1; f < total || f < 0; f++) {
+      node = 0;
+      now.assign(1, (cudaGraphNode_t)(++node));
+      const std::vector<cudaGraphNode_t> root = now;
+      calls = 0; failAt = f;
+      GraphFork fork(nullptr, true);
+      std::vector<cudaGraphNode_t> tails;
+      bool apart = true;
+      for (int k = 0; k < branches; k++) {
+        fork.branch();
+        apart = apart && launch() == root;
+        launch();
+        tails.push_back(now[0]);
+      }
+      fork.join();
+      if (f < 0) {
+        assert(fork.error() == cudaSuccess && apart && now == tails);
+        total = calls;
+        assert(total > 2 * branches);
+      } else {
+        assert(fork.error() == cudaErrorMemoryAllocation);
+      }
+    }
+  }
+  failAt = -1;
+  // not capturing: in order, no error
+  status = cudaStreamCaptureStatusNone;
+  GraphFork none(nullptr, true);
+  none.branch(); none.branch(); none.join();
+  assert(none.error() == cudaSuccess);
+  // invalidated before or between the branches: reported
+  status = cudaStreamCaptureStatusInvalidated;
+  GraphFork bad(nullptr, true);
+  bad.branch(); bad.join();
+  assert(bad.error() != cudaSuccess);
+  status = cudaStreamCaptureStatusActive;
+  GraphFork late(nullptr, true);
+  late.branch();
+  status = cudaStreamCaptureStatusInvalidated;
+  late.branch(); late.join();
+  assert(late.error() != cudaSuccess);
+  // off: not one call
+  calls = 0;
+  GraphFork off(nullptr, false);
+  off.branch(); off.join();
+  assert(calls == 0 && off.error() == cudaSuccess);
 }
 """)
