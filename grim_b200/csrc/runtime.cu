@@ -53,6 +53,12 @@ static void set_err(const char* fmt, ...) {
     }                                                                               \
   } while (0)
 
+// which Newton a step runs
+struct NewtonForm {
+  int mode, perZone;
+  double rtol;
+};
+
 struct grim_handle {
   grim_config cfg;
   DevCfg dc;
@@ -81,6 +87,8 @@ struct grim_handle {
   cudaEvent_t ev[8];
   bool graphOn = false;
   cudaGraphExec_t graph = nullptr;
+  long long settings = 0;  // changes of what a step launches: graphs captured before one are out of date
+  const NewtonForm* form = nullptr;  // the batch's Newton, while its step is enqueued
   bool capturing = false;  // the step being enqueued is captured: it may branch (GraphFork)
   cudaError_t captureError = cudaSuccess;  // the first of that capture's branching calls that failed
   grim_stats stats;
@@ -267,9 +275,21 @@ static int make_devcfg(const grim_config& c, DevCfg& d) {
 }
 
 static bool use_exact(const grim_handle* h) { return h->cfg.newtonMode == GRIM_NEWTON_PARITY_FD64; }
+// the Newton of the step being enqueued: the handle's own, or in a batch step
+// the batch's.  The stencil is the handle's in either.
+static NewtonForm newton_form(const grim_handle* h) {
+  if (h->form) return *h->form;
+  return {h->cfg.newtonMode, h->cfg.perZoneConvergence, h->cfg.nonlinearsolve_rtol};
+}
 // the reference's FD-Jacobian Newton with global break, in either unit
-static bool is_fd(const grim_handle* h) {
-  return h->cfg.newtonMode == GRIM_NEWTON_PARITY_FD64 || h->cfg.newtonMode == GRIM_NEWTON_FD64_FAST;
+static bool is_fd(const NewtonForm& f) {
+  return f.mode == GRIM_NEWTON_PARITY_FD64 || f.mode == GRIM_NEWTON_FD64_FAST;
+}
+static bool is_fd(const grim_handle* h) { return is_fd(newton_form(h)); }
+// a graph captured before is out of date
+static void settings_changed(grim_handle* h) {
+  h->settings++;
+  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
 }
 
 // the three tensor maps (X1, X2, X3 box shapes) of a prim array of this
@@ -425,30 +445,32 @@ static bool newton_counts_nan(const grim_handle* h) {
 // returns whether the launch counts the NaN zones (countNan asked for it
 // and the Newton form does it)
 static bool enqueue_newton(grim_handle* h, int stage, bool guessOld = false, bool countNan = false) {
-  const DevCfg& c = h->dc;
+  const NewtonForm f = newton_form(h);
+  DevCfg c = h->dc;
+  c.rtol = f.rtol;
   cudaStream_t s = h->stream;
   StageBufs b = stage_bufs(h, stage, guessOld);
   PROF(GRIM_PROF_NEWTON);
   countNan = countNan && newton_counts_nan(h);
   if (countNan) b.nanCount = &h->st->nanFlag;  // zero since the step began
-  if (h->cfg.newtonMode == GRIM_NEWTON_PARITY_FD64) {
+  if (f.mode == GRIM_NEWTON_PARITY_FD64) {
     grim::exact::newton_fd_init(c, stage, b, s);
     g_launch_counter++;
     for (int it = 0; it < c.maxIter; it++) {
       grim::exact::newton_fd_iter(c, stage, it, b, s);
       g_launch_counter++;
     }
-  } else if (h->cfg.newtonMode == GRIM_NEWTON_FD64_FAST) {
+  } else if (f.mode == GRIM_NEWTON_FD64_FAST) {
     grim::fast::newton_fd_init(c, stage, b, s);
     g_launch_counter++;
     for (int it = 0; it < c.maxIter; it++) {
       grim::fast::newton_fd_iter(c, stage, it, b, s);
       g_launch_counter++;
     }
-  } else if (h->cfg.perZoneConvergence == 3 && grim::fast::newton_defer(c, stage, b, h->cfg.newtonMode, s)) {
+  } else if (f.perZone == 3 && grim::fast::newton_defer(c, stage, b, f.mode, s)) {
     g_launch_counter++;
   } else {
-    grim::fast::newton_fast(c, stage, b, h->cfg.newtonMode, s);
+    grim::fast::newton_fast(c, stage, b, f.mode, s);
     g_launch_counter++;
   }
   return countNan;
@@ -464,7 +486,7 @@ static bool enqueue_newton(grim_handle* h, int stage, bool guessOld = false, boo
 constexpr long long kFuseMax = 1LL << 17;
 static bool stage_fused(const grim_handle* h) {
   const DevCfg& c = h->dc;
-  return !is_fd(h) && h->cfg.perZoneConvergence != 3 && !h->profOn && !c.conduction && !c.viscosity &&
+  return !use_exact(h) && !is_fd(h) && newton_form(h).perZone != 3 && !h->profOn && !c.conduction && !c.viscosity &&
          c.Zint <= kFuseMax;
 }
 // whether that launch finishes the stage as well: periodic Minkowski grids,
@@ -493,7 +515,10 @@ static bool enqueue_stage(grim_handle* h, int stage, bool guessOld, bool countNa
   countNan = countNan && newton_counts_nan(h);
   if (countNan) b.nanCount = &h->st->nanFlag;
   double* dst = !stage_finishes(h) ? nullptr : (stage == GRIM_HALF_STEP ? h->primHalf : h->primOld);
-  grim::fast::stage_solve(h->dc, stage, b, h->cfg.newtonMode, dst, h->cfg.elemOldFromFullStep ? 1 : 0, h->stream);
+  const NewtonForm f = newton_form(h);
+  DevCfg c = h->dc;
+  c.rtol = f.rtol;
+  grim::fast::stage_solve(c, stage, b, f.mode, dst, h->cfg.elemOldFromFullStep ? 1 : 0, h->stream);
   g_launch_counter++;
   return countNan;
 }
@@ -1662,7 +1687,7 @@ int grim_set_newton_mode(grim_handle* h, int mode, int perZone, double rtol) {
   h->cfg.perZoneConvergence = perZone;
   h->cfg.nonlinearsolve_rtol = rtol;
   h->dc.rtol = rtol;
-  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+  settings_changed(h);
   return GRIM_OK;
 }
 
@@ -1781,7 +1806,7 @@ int grim_autotune(grim_handle* h, int* variants, double* msBest) {
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+  settings_changed(h);
   CK(cudaGetLastError());
   return GRIM_OK;
 }
@@ -1795,14 +1820,14 @@ int grim_set_face_variant(grim_handle* h, int dir, int variant) {
     return GRIM_EINVAL;
   }
   h->faceVariant[use_exact(h) ? 0 : 1][dir] = variant;
-  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+  settings_changed(h);
   return GRIM_OK;
 }
 
 int grim_set_dt_mode(grim_handle* h, int fixed) {
   if (!h) return GRIM_EINVAL;
   h->fixedDt = fixed != 0;
-  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+  settings_changed(h);
   return GRIM_OK;
 }
 
@@ -2035,6 +2060,10 @@ struct grim_batch {
   // largest first so that each carries about the same number of zones
   Chains chains;
   std::vector<int> order;  // problems, largest first
+  // the Newton of a batch step, per problem: a mode that a problem's handle
+  // is given is for steps of its own
+  std::vector<NewtonForm> form;
+  std::vector<long long> settings;  // the problems' when the graph was captured
   bool graphOn = false;
   cudaGraphExec_t graph = nullptr;
 };
@@ -2078,7 +2107,8 @@ int grim_batch_create(const grim_config* cfgs, int n, int device, grim_batch** o
     cudaStreamDestroy(h->stream);
     h->stream = B->stream;
     h->cfg.newtonMode = GRIM_NEWTON_MIXED32;
-    h->cfg.perZoneConvergence = 2;
+    h->cfg.perZoneConvergence = 1;
+    B->form.push_back(newton_form(h));
     B->h.push_back(h);
   }
   long long total = 0;
@@ -2113,9 +2143,10 @@ int grim_batch_set_newton_mode(grim_batch* B, int mode, double rtol) {
     set_err("grim_batch_set_newton_mode: the batch runs the tangent or mixed Newton");
     return GRIM_EINVAL;
   }
-  for (grim_handle* h : B->h) {
-    int rc = grim_set_newton_mode(h, mode, 2, rtol);
+  for (size_t p = 0; p < B->h.size(); p++) {
+    int rc = grim_set_newton_mode(B->h[p], mode, 1, rtol);
     if (rc) return rc;
+    B->form[p] = newton_form(B->h[p]);
   }
   batch_drop_graph(B);
   return GRIM_OK;
@@ -2136,7 +2167,9 @@ static cudaError_t capture_batch_step(grim_batch* B) {
     fork.branch();
     h->capturing = true;
     h->captureError = cudaSuccess;
+    h->form = &B->form[p];
     enqueue_step(h, false);
+    h->form = nullptr;
     h->capturing = false;
     if (e == cudaSuccess) e = h->captureError;
   }
@@ -2155,7 +2188,9 @@ static int enqueue_batch_step(grim_batch* B) {
   for (int p : B->order) {
     grim_handle* h = B->h[p];
     h->stream = ch.stream[ch.of[p]];
+    h->form = &B->form[p];
     enqueue_step(h, false);
+    h->form = nullptr;
     h->stream = B->stream;
   }
   for (size_t k = 0; k < ch.stream.size(); k++) {
@@ -2177,6 +2212,10 @@ int grim_batch_time_steps(grim_batch* B, int nsteps) {
   CK(cudaSetDevice(B->device));
   for (grim_handle* h : B->h)
     if (h->fixedDt != B->h[0]->fixedDt) { set_err("grim_batch_time_steps: mixed dt modes"); return GRIM_EINVAL; }
+  std::vector<long long> settings;
+  for (grim_handle* h : B->h) settings.push_back(h->settings);
+  if (settings != B->settings) batch_drop_graph(B);
+  B->settings = settings;
   for (int n = 0; n < nsteps; n++) {
     if (B->graphOn) {
       if (!B->graph) {
@@ -2239,7 +2278,7 @@ int grim_set_debug(grim_handle* h, int setting, int value) {
   if (!h) return GRIM_EINVAL;
   if (setting != GRIM_DEBUG_SKIP_BULK_COPIES) { set_err("grim_set_debug: unknown setting %d", setting); return GRIM_EINVAL; }
   h->dc.dbgSkipCopies = value != 0;
-  if (h->graph) { cudaGraphExecDestroy(h->graph); h->graph = nullptr; }
+  settings_changed(h);
   return GRIM_OK;
 }
 

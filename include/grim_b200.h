@@ -489,7 +489,10 @@ int grim_set_dt_mode(grim_handle* h, int fixed);
  *      boundaries, metric and reconstruction.  grim_batch_problem returns
  *      problem p's handle for set/get of its state and its statistics;
  *      that handle is owned by the batch (do not destroy it) and runs on
- *      the batch's stream. */
+ *      the batch's stream.  A batch step runs the batch's Newton (mixed, or
+ *      what grim_batch_set_newton_mode set) on every problem; a Newton mode
+ *      set on a problem's handle chooses that handle's stencil arithmetic and
+ *      the Newton of steps of its own. */
 typedef struct grim_batch grim_batch;
 int grim_batch_create(const grim_config* cfgs, int n, int device, grim_batch** out);
 int grim_batch_destroy(grim_batch* b);
