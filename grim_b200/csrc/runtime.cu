@@ -92,7 +92,8 @@ struct grim_handle {
   bool capturing = false;  // the step being enqueued is captured: it may branch (GraphFork)
   cudaError_t captureError = cudaSuccess;  // the first of that capture's branching calls that failed
   grim_stats stats;
-  long long launchesPerStep = 0;
+  long long launchesPerStep = 0;  // of the last step
+  long long graphLaunches = 0;    // of a step of the captured graph
   size_t bytesZ = 0;
   int lastStage = GRIM_HALF_STEP;
   // the stage constants (consOld, divF, Sexp, the field guess) are those
@@ -986,7 +987,7 @@ static int run_steps(grim_handle* h, int nsteps) {
         h->captureError = cudaSuccess;
         enqueue_step(h, false);
         h->capturing = false;
-        h->launchesPerStep = g_launch_counter - before;
+        h->graphLaunches = g_launch_counter - before;
         CK(end_capture(h->stream, h->captureError, &g));
         cudaError_t e = cudaGraphInstantiate(&h->graph, g, 0);
         cudaGraphDestroy(g);
@@ -994,6 +995,7 @@ static int run_steps(grim_handle* h, int nsteps) {
       }
       if (last) cudaEventRecord(h->ev[0], h->stream);
       CK(cudaGraphLaunch(h->graph, h->stream));
+      h->launchesPerStep = h->graphLaunches;
       if (last) cudaEventRecord(h->ev[7], h->stream);
     } else {
       long long before = g_launch_counter;

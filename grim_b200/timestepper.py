@@ -206,7 +206,9 @@ class timeStepper:
 
     def profileSteps(self, nsteps=1):
         """Advance nsteps without the graph, timing every kernel group with
-        CUDA events on the stepper's stream: {group: (ms, launch runs)}."""
+        CUDA events on the stepper's stream: {group: (ms, launch runs)}.  The
+        groups are launched apart and in order, also where a step fuses them
+        or runs them side by side."""
         n = len(self.PROF_GROUPS)
         ms = (ctypes.c_double * n)()
         cnt = (ctypes.c_longlong * n)()

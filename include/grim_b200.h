@@ -126,9 +126,11 @@ typedef struct grim_stats {
   long long nonFinite;         /* NaN/Inf primitives after the last step */
   double msStep;               /* whole grim_time_step */
   double msStencil;            /* stencil kernels, both stages */
-  double msNewton;             /* Newton kernels, both stages */
+  double msNewton;             /* Newton kernels, both stages; on grids of up to 131072 zones (ideal
+                                  MHD, tangent / mixed modes) with the flux half of the stencil and,
+                                  periodic Minkowski, the stage finish, which are one launch with them */
   double msOther;              /* ghost fill, dt, copies */
-  long long kernelLaunches;    /* launches of this library's kernels in the step */
+  long long kernelLaunches;    /* launches of this library's kernels in the last step */
   long long waitTimeouts;      /* bounded waits on asynchronous copies that gave up, since creation */
   long long drainTimeouts;     /* of those, give-ups whose copies in flight did not land either */
   double reserved[6];
@@ -411,7 +413,11 @@ int grim_measure_peaks(int device, double* fp64_tflops, double* fp32_tflops, dou
  * grim_profile_steps runs nsteps steps without the graph and returns the
  * device time of each kernel group, measured with CUDA events recorded
  * around its launches on the handle's stream, summed over the steps, and
- * the number of bracketed launch runs per group. */
+ * the number of bracketed launch runs per group.  Every group is launched
+ * apart and in order: what a step fuses (up to 131072 zones: the flux half of
+ * the epilogue, the Newton, the stage finish) or runs side by side as a graph
+ * gives the same bits here, but the sum of the groups is then more than the
+ * time of a step. */
 enum {
   GRIM_PROF_BOUNDARY = 0,    /* ghost fill, communicate, inflow / pole hooks */
   GRIM_PROF_FACES_X1 = 1,    /* reconstruction + Riemann fluxes at X1 faces */

@@ -417,6 +417,23 @@ def test_profile_steps_and_flop_counts():
     assert f["solve32"] == f["solve64"] and 60 <= f["solve64"] <= 200, f
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_stats_count_the_last_steps_launches(graph):
+    """kernelLaunches is of the last step, also when a step replays a graph
+    captured before a profiled one, whose pieces are launched apart."""
+    cfg = PR.fast_mode_config(N=32, newtonMode=C.NEWTON_MIXED32, perZoneConvergence=1)
+    from grim_b200.timestepper import timeStepper
+    ts = timeStepper(cfg)
+    ts.primOld.setVars(PR.fast_mode_prims(cfg))
+    ts.enableGraph(graph)
+    ts.timeSteps(1)
+    n = ts.stats()["kernelLaunches"]
+    prof = ts.profileSteps(1)
+    assert ts.stats()["kernelLaunches"] > n  # the profiled step's own
+    ts.timeSteps(1)
+    assert ts.stats()["kernelLaunches"] == n and prof["newton"][1] == 2
+
+
 @pytest.mark.parametrize("mode", [C.NEWTON_PARITY_FD64, C.NEWTON_MIXED32])
 def test_autotuned_face_kernels_give_identical_results(mode):
     """The autotuner only changes launch shapes.  In the FP64 parity unit
