@@ -2447,67 +2447,41 @@ static void face_strip_tma_launch(const DevCfg& c, int dir, const CUtensorMap* t
 template <int C, int V, bool F>
 static void face_flux_t(const DevCfg& c, int dir, const double* ps, const double* geoF, const double* geoC,
                         double* flux, int variant, const CUtensorMap* tmap, DevState* st, cudaStream_t s) {
+  variant = face_kernel(kFastMath, C || V, dir, variant, tmap && st);
   if constexpr (kFastMath && C == 0 && V == 0) {
-    const bool tma = tmap && st;
     if (dir == 0) {
-      if ((variant == 2 || variant == 5) && tma) face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s);
-      else if (variant == 3 && tma) face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s);
-      else if (variant == 1 || variant == 3) face_x1_launch<C, V, F, 5>(c, ps, geoF, flux, s);
-      else face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s);
-      return;
-    }
-    if (variant >= 8 && tma) {
-      if (variant & 1) face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s);
+      switch (variant) {
+        case 1: face_x1_launch<C, V, F, 5>(c, ps, geoF, flux, s); break;
+        case 2: face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s); break;
+        case 3: face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s); break;
+        default: face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s); break;
+      }
       return;
     }
     switch (variant) {
       case 1: face_strip_launch<C, V, F, 4, 5>(c, dir, ps, geoF, geoC, flux, s); break;
       case 2: face_strip_launch<C, V, F, 2, 4>(c, dir, ps, geoF, geoC, flux, s); break;
       case 3: face_strip_launch<C, V, F, 2, 5>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 4: case 6: face_strip_launch<C, V, F, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 4: face_strip_launch<C, V, F, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
       case 5: face_strip_launch<C, V, F, 8, 5>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 8: face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+      case 9: face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s); break;
       default: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
     }
-  } else if constexpr (kFastMath) {
-    constexpr int MB = F ? 4 : 3;  // resident blocks: 110 registers in Minkowski, 158 in Kerr-Schild
-    const bool tma = variant == 1 && tmap && st;
+  } else if constexpr (!kFastMath && C == 0 && V == 0) {
     if (dir == 0) {
-      if (tma) face_x1_tma_launch<C, V, F, MB>(c, &tmap[0], geoF, flux, st, s);
-      else face_x1_launch<C, V, F, MB>(c, ps, geoF, flux, s);
-    } else {
-      if (tma) face_strip_tma_launch<C, V, F, MB>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_launch<C, V, F, 4, MB>(c, dir, ps, geoF, geoC, flux, s);
-    }
-  } else if constexpr (C == 0 && V == 0) {
-    if (dir == 0) {
-      if ((variant == 2 || variant == 3 || variant == 5) && tmap && st) {
-        if (variant == 5) face_x1_tma_launch<C, V, F, 3, true>(c, &tmap[0], geoF, flux, st, s);
-        else if (variant == 3) face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s);
-        else face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s);
-      } else if (variant == 6) {
-        face_x1_launch<C, V, F, 4, true>(c, ps, geoF, flux, s);
-      } else if (variant == 4 || variant == 5) {
-        face_x1_launch<C, V, F, 3, true>(c, ps, geoF, flux, s);
-      } else if (variant == 1 || variant == 3) {
-        face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s);
-      } else {
-        face_x1_launch<C, V, F, 3>(c, ps, geoF, flux, s);
+      switch (variant) {
+        case 1: face_x1_launch<C, V, F, 4>(c, ps, geoF, flux, s); break;
+        case 2: face_x1_tma_launch<C, V, F, 3>(c, &tmap[0], geoF, flux, st, s); break;
+        case 3: face_x1_tma_launch<C, V, F, 4>(c, &tmap[0], geoF, flux, st, s); break;
+        case 4: face_x1_launch<C, V, F, 3, true>(c, ps, geoF, flux, s); break;
+        case 5: face_x1_tma_launch<C, V, F, 3, true>(c, &tmap[0], geoF, flux, st, s); break;
+        case 6: face_x1_launch<C, V, F, 4, true>(c, ps, geoF, flux, s); break;
+        default: face_x1_launch<C, V, F, 3>(c, ps, geoF, flux, s); break;
       }
       return;
     }
-    if (variant >= 8 && tmap && st) {
-      if (variant == 11) face_strip_tma_launch<C, V, F, 4, true>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else if (variant == 10) face_strip_tma_launch<C, V, F, 3, true>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else if (variant == 9) face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s);
-      return;
-    }
     switch (variant) {
-      case 8: face_strip_launch<C, V, F, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 10: face_strip_launch<C, V, F, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 11: face_strip_launch<C, V, F, 4, 4, true>(c, dir, ps, geoF, geoC, flux, s); break;
-      case 9: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
       case 1: face_strip_launch<C, V, F, 4, 4>(c, dir, ps, geoF, geoC, flux, s); break;
       case 2: face_strip_launch<C, V, F, 2, 3>(c, dir, ps, geoF, geoC, flux, s); break;
       case 3: face_strip_launch<C, V, F, 2, 4>(c, dir, ps, geoF, geoC, flux, s); break;
@@ -2515,17 +2489,25 @@ static void face_flux_t(const DevCfg& c, int dir, const double* ps, const double
       case 5: face_strip_launch<C, V, F, 8, 4>(c, dir, ps, geoF, geoC, flux, s); break;
       case 6: face_strip_launch<C, V, F, 8, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
       case 7: face_strip_launch<C, V, F, 4, 3, true>(c, dir, ps, geoF, geoC, flux, s); break;
+      case 8: face_strip_tma_launch<C, V, F, 3>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+      case 9: face_strip_tma_launch<C, V, F, 4>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+      case 10: face_strip_tma_launch<C, V, F, 3, true>(c, dir, tmap, geoF, geoC, flux, st, s); break;
+      case 11:
+        if (tmap && st) face_strip_tma_launch<C, V, F, 4, true>(c, dir, tmap, geoF, geoC, flux, st, s);
+        else face_strip_launch<C, V, F, 4, 4, true>(c, dir, ps, geoF, geoC, flux, s);
+        break;
       default: face_strip_launch<C, V, F, 4, 3>(c, dir, ps, geoF, geoC, flux, s); break;
     }
   } else {
-    // EMHD elements need more registers: two resident blocks; variant 1
-    // stages the stencils with TMA
+    // EMHD elements need more registers (fast path: 110 in Minkowski, 158 in
+    // Kerr-Schild); variant 1 stages the stencils with TMA
+    constexpr int MB = !kFastMath ? 2 : F ? 4 : 3;
     if (dir == 0) {
-      if (variant == 1 && tmap && st) face_x1_tma_launch<C, V, F, 2>(c, &tmap[0], geoF, flux, st, s);
-      else face_x1_launch<C, V, F, 2>(c, ps, geoF, flux, s);
+      if (variant == 1) face_x1_tma_launch<C, V, F, MB>(c, &tmap[0], geoF, flux, st, s);
+      else face_x1_launch<C, V, F, MB>(c, ps, geoF, flux, s);
     } else {
-      if (variant == 1 && tmap && st) face_strip_tma_launch<C, V, F, 2>(c, dir, tmap, geoF, geoC, flux, st, s);
-      else face_strip_launch<C, V, F, 4, 2>(c, dir, ps, geoF, geoC, flux, s);
+      if (variant == 1) face_strip_tma_launch<C, V, F, MB>(c, dir, tmap, geoF, geoC, flux, st, s);
+      else face_strip_launch<C, V, F, 4, MB>(c, dir, ps, geoF, geoC, flux, s);
     }
   }
 }
@@ -2545,7 +2527,7 @@ void face_flux(const DevCfg& c, int dir, const double* ps, const double* geoF, c
 // in Minkowski), X1: 0 = 4 blocks, 1 = 5 (a few spills in Kerr-Schild), 2 / 3
 // = TMA-staged, 3 / 4 blocks; 4, 6 run 0 and 5 runs 2.  X2 / X3: 0-5 = 4, 2, 8
 // i per warp x 4 / 5 blocks; 8, 9 = TMA-staged, 3 / 4 blocks; 7 runs 0, 6
-// runs 4, 10 and 11 run 8 and 9.
+// runs 4, 10 and 11 run 8 and 9 (face_kernel).
 // EMHD (9 or 10 dof), every direction: 0 = plain, 1 = TMA-staged.
 // tmap points at the caller's three tensor maps (X1, X2, X3 box shapes) of
 // the prim array, or is null (the TMA variants then run their plain

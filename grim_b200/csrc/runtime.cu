@@ -384,9 +384,10 @@ static void note_capture(grim_handle* h, cudaError_t e) {
 // persistent grid divides the faces over the whole GPU's resident blocks
 static bool persistent_faces(const grim_handle* h, const double* ps, int d) {
   const DevCfg& c = h->dc;
-  const int v = h->faceVariant[use_exact(h) ? 0 : 1][d];
-  if (!tmap_for(h, ps, d)) return false;
-  if (c.conduction || c.viscosity) return v == 1;
+  const bool emhd = c.conduction || c.viscosity, tma = tmap_for(h, ps, d) != nullptr;
+  const int v = face_kernel(!use_exact(h), emhd, d, h->faceVariant[use_exact(h) ? 0 : 1][d], tma);
+  if (!tma) return false;
+  if (emhd) return v == 1;
   return d == 0 ? (v == 2 || v == 3 || v == 5) : v >= 8;
 }
 
@@ -1790,6 +1791,7 @@ int grim_autotune(grim_handle* h, int* variants, double* msBest) {
     double best = 1e30;
     int bestV = 0;
     for (int v = 0; v < nv; v++) {
+      if (face_kernel(unit == 1, c.conduction || c.viscosity, d, v, tmap_for(h, b.ps, d) != nullptr) != v) continue;
       KNS_CALL(h, face_flux, c, d, b.ps, b.geoF[d], b.geoC, h->flux[d], v, tmap_for(h, b.ps, d), h->st,
                h->stream);  // warm-up
       CK(cudaEventRecord(e0, h->stream));

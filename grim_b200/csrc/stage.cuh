@@ -58,4 +58,19 @@ inline bool torus_fill_checks(const DevCfg& c) {
   return (c.bc[0] == GRIM_OUTFLOW || c.bc[0] == GRIM_MIRROR) && (c.bc[1] == GRIM_OUTFLOW || c.bc[1] == GRIM_MIRROR);
 }
 
+// The lowest face-flux variant that launches the same kernel as this one:
+// unit (fast or parity), extended MHD, direction, and whether the caller has a
+// tensor map (without one the staged variants run plain ones).  The launcher
+// picks its kernel by this number and the autotuner times each kernel once.
+inline int face_kernel(bool fast, bool emhd, int dir, int variant, bool tma) {
+  static const int kFastX1[2][7] = {{0, 1, 0, 1, 0, 0, 0}, {0, 1, 2, 3, 0, 2, 0}};
+  static const int kFastStrip[2][12] = {{0, 1, 2, 3, 4, 5, 4, 0, 0, 0, 0, 0}, {0, 1, 2, 3, 4, 5, 4, 0, 8, 9, 8, 9}};
+  static const int kPlainX1[7] = {0, 1, 0, 1, 4, 4, 6};
+  static const int kPlainStrip[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 7, 11};
+  if (emhd) return tma ? variant : 0;
+  if (fast) return dir == 0 ? kFastX1[tma][variant] : kFastStrip[tma][variant];
+  if (tma) return variant;
+  return dir == 0 ? kPlainX1[variant] : kPlainStrip[variant];
+}
+
 }  // namespace grim
