@@ -333,7 +333,7 @@ def rooflines(cfg, prof, prof_fd, device):
 # the sources that define the step's kernels: a DRAM capture describes the
 # kernels these files built
 KERNEL_SOURCES = ("kernels.cuh", "physics.cuh", "recon.cuh", "stage.cuh", "common.cuh", "torus.cuh",
-                  "launch.h", "kernels_fast.cu", "faces_fast.cu")
+                  "launch.h", "kernels_fast.cu", "faces_fast.cu", "faces_fast_flat.cu")
 
 
 def kernel_sources_sha16():

@@ -1,8 +1,8 @@
 """Builds libgrim_b200.so in place (nvcc, sm_100a).
 
-kernels_exact.cu, faces_exact.cu and geometry.cu are compiled with
+kernels_exact.cu, faces_exact*.cu and geometry.cu are compiled with
 --fmad=false so the FP64 parity path keeps the reference's operation order
-without FMA contraction; kernels_fast.cu and faces_fast.cu (tangent /
+without FMA contraction; kernels_fast.cu and faces_fast*.cu (tangent /
 mixed-precision Newton) keep contraction on.
 Objects are rebuilt only when a source or header is newer.
 """
@@ -24,7 +24,9 @@ UNITS = {
     "kernels_exact.cu": EXACT,
     "kernels_fast.cu": [],
     "faces_exact.cu": EXACT,
+    "faces_exact_flat.cu": EXACT,
     "faces_fast.cu": [],
+    "faces_fast_flat.cu": [],
     "geometry.cu": EXACT,
     "runtime.cu": [],
     "peaks.cu": [],
