@@ -393,24 +393,38 @@ static bool persistent_faces(const grim_handle* h, const double* ps, int d) {
 
 // The face kernels of the directions and the epilogue's centre half read
 // the same primitives and write arrays of their own: in a captured step
-// they are parallel branches of the graph, joined before the flux half (each
-// fills the GPU for one to a few waves only, one after another, on all but
-// the largest grids).  Measured on one B200, us per step in order / side by
-// side: 64^2 wave 16.1 / 14.0, Orszag-Tang 512^2 236 / 219, extended MHD
-// 256^2 228 / 209, torus 64x48x24 144 / 137, EMHD torus 96x64x32 907 / 862;
-// torus 256x128x64, whose kernels each run many waves, 2465 / 2467.  Past a
-// million zones there is nothing left to gain, and a persistent grid that has
-// to share the GPU finishes late (its blocks' shares are fixed): 2390 / 2500
-// on that torus with two such kernels, so those stay in order.
-constexpr long long kForkPersistentMax = 1LL << 20;
+// they may be parallel branches of the graph, joined before the flux half,
+// which helps while each fills the GPU for one to a few waves only.  Measured
+// on one B200, us per step in order / side by side:
+//   fast path: wave 64^2 36 / 30; torus 48x32x24 101 / 92, 64x48x24 142 / 130,
+//     128x64x64 630 / 635; Orszag-Tang 128^2 53 / 41, 512^2 206 / 199; extended
+//     MHD 256^2 179 / 162, 1024^2 2165 / 2140; EMHD torus 96x64x32, two steps
+//     alone 1599 / 1620, queued behind others 1589 / 1556;
+//   parity path, two or three resident blocks per SM: Orszag-Tang 128^2 173 / 139;
+//     torus 48x32x24 236 / 227, 64x48x24 380 / 385, 64x48x40 550 / 577, 96x64x32
+//     775 / 800, 99x71x33 901 / 924.
+// In the parity path's Kerr-Schild kernels the branches' blocks take the few
+// slots of one another's, so past kForkParityMax zones, about two waves of them,
+// they stay in order (a graph of branches also takes 0.3 ms more to
+// instantiate).  A persistent grid that has to share the GPU finishes late
+// (its blocks' shares are fixed): Orszag-Tang 1024^2 787 / 834, torus
+// 256x128x64 2390 / 2500, torus 128x64x64 622 / 623, so those stay in order past
+// kForkPersistentMax.
+constexpr long long kForkParityMax = 1LL << 16;
+constexpr long long kForkPersistentMax = 1LL << 19;
+static bool stencil_forks(const grim_handle* h, const double* ps) {
+  const DevCfg& c = h->dc;
+  if (use_exact(h) && c.metric != GRIM_MINKOWSKI && c.Zint > kForkParityMax) return false;
+  bool persistent = false;
+  for (int d = 0; d < c.dim; d++) persistent = persistent || persistent_faces(h, ps, d);
+  return !(persistent && c.Zint > kForkPersistentMax);
+}
 static void enqueue_stencil(grim_handle* h, int stage, bool guessOld = false, bool fluxHalf = true) {
   const DevCfg& c = h->dc;
   cudaStream_t s = h->stream;
   StageBufs b = stage_bufs(h, stage, guessOld);
   const bool emhd = c.conduction || c.viscosity, split = emhd || c.metric != GRIM_MINKOWSKI;
-  bool persistent = false;
-  for (int d = 0; d < c.dim; d++) persistent = persistent || persistent_faces(h, b.ps, d);
-  GraphFork fork(s, h->capturing && !(persistent && c.Zint > kForkPersistentMax));
+  GraphFork fork(s, h->capturing && stencil_forks(h, b.ps));
   for (int d = 0; d < c.dim; d++) {
     fork.branch();
     PROF(GRIM_PROF_FACES_X1 + d);
