@@ -248,27 +248,31 @@ GRIM_D void recon_zone(const DevCfg& c, const double* __restrict__ ps, long long
 #ifdef GRIM_FAST_MATH
 // the weights a and signal speeds s of flux = aL (F_L - sL U_L) + aR (F_R -
 // sR U_R), sqrt(-g) included: HLL, or LLF as HLL with the speeds -c, c
+template <class S>
 struct FaceWeights {
-  double aL, sL, aR, sR;
+  S aL, sL, aR, sR;
 };
-GRIM_D FaceWeights face_weights(const DevCfg& c, double g, double cmin, double cmax) {
-  FaceWeights f;
+// (templated on the scalar for the operation counts; double in the kernels)
+template <class S, class RG>
+GRIM_D FaceWeights<S> face_weights(const DevCfg& c, RG g, S cmin, S cmax) {
+  FaceWeights<S> f;
   if (c.riemann == GRIM_HLL) {
-    const double id = g / (cmax - cmin);
+    const S id = g / (cmax - cmin);
     f.aL = cmax * id;
     f.sL = cmin;
     f.aR = -cmin * id;
     f.sR = cmax;
   } else {
-    const double cm = fmax(cmax, -cmin);
-    f.aL = f.aR = 0.5 * g;
+    const S cm = fmax(cmax, -cmin);
+    f.aL = f.aR = S(0.5) * g;
     f.sL = -cm;
     f.sR = cm;
   }
   return f;
 }
+// the parity path's form: named by the branch that PAIR discards here
 template <int COND, int VISC, class GT>
-GRIM_D void riemann_face(const DevCfg&, int, const double*, const GT&, double*, long long, double*);  // parity path only
+GRIM_D void riemann_face(const DevCfg&, int, const double*, const GT&, double*, long long, double*);
 #else
 // Shared memory holds what waits: the right face state (slot 2, put there
 // by the caller) while the left element is evaluated, then the left
@@ -358,7 +362,7 @@ GRIM_D void riemann_face_pair(const DevCfg& c, int dir, const double* pl, const 
   double mn[2], mx[2], L[DOF], R[DOF];
 #pragma unroll
   for (int sd = 0; sd < 2; sd++) char_speeds<COND, VISC>(e[sd], G, dir, c, mn[sd], mx[sd]);
-  const FaceWeights fw = face_weights(c, G.g, fmin(mn[0], mn[1]), fmax(mx[0], mx[1]));
+  const FaceWeights<double> fw = face_weights(c, G.g, fmin(mn[0], mn[1]), fmax(mx[0], mx[1]));
   side_flux<COND, VISC>(e[0], dir, fw.sL, L);
   side_flux<COND, VISC>(e[1], dir, fw.sR, R);
 #pragma unroll
@@ -1726,6 +1730,8 @@ __global__ void __launch_bounds__(128, fd_min_blocks(COND || VISC, FLAT)) k_newt
 // and solve in FP32, residual in FP64, i.e. FP32 inexact Newton refined by
 // the FP64 residual).
 // ---------------------------------------------------------------------------
+// whether a scalar is 32-bit (the counting scalar of one too)
+template <class T> struct IsFp32 : std::is_same<T, float> {};
 template <int COND, int VISC, class T, bool GENERIC = false, class GT>
 GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>& K, const GT& Gt,
                              const DevCfg& c, T J[5 + COND + VISC][5 + COND + VISC]) {
@@ -1740,7 +1746,7 @@ GRIM_D void tangent_jacobian(const double* P, const StageConst<5 + COND + VISC>&
 #pragma unroll
   for (int v = 0; v < NF; v++) Pd[v] = D::var((T)P[v], v);
 #ifdef GRIM_FAST_MATH
-  if constexpr ((COND || VISC) && !GT::flat && std::is_same<T, float>::value)
+  if constexpr ((COND || VISC) && !GT::flat && IsFp32<T>::value)
     emhd_tangents<COND, VISC, D, T>(Pd, K, Gt, c, Rd);
   else
 #endif

@@ -69,26 +69,45 @@ struct Lift<Cnt<B>> {
   GRIM_HD static Cnt<B> of(double x) { return Cnt<B>(x); }
 };
 
+// Minkowski: the products with one that the compiler drops are not counted
+template <class B>
+struct FlatGeo<Cnt<B>> {
+  static constexpr bool flat = true;
+  One g, alpha, ialpha;
+  Cnt<B> x1, x2, dyn;
+};
+template <class B>
+GRIM_D void convert_geo(FlatGeo<Cnt<B>>& Gt, const FlatGeo<double>& G) {
+  Gt.x1 = Cnt<B>(G.x1);
+  Gt.x2 = Cnt<B>(G.x2);
+  Gt.dyn = Cnt<B>(0);
+}
+
 namespace GRIM_KNS {
 
+template <>
+struct IsFp32<Cnt<float>> : std::true_type {};
+
 // One thread, one zone z of the stage buffers b (filled by a stage set-up):
-// out = {residual fp64, Jacobian(fp32) fp32, Jacobian(fp64) fp64,
+// out = {residual evaluation fp64 (as the line search does it: the trial
+//        state, its residual and the norm), Jacobian(fp32) fp32, Jacobian(fp64) fp64,
 //        solve fp32, solve fp64, residual divides, residual sqrt+exp,
 //        generic forward-tangent pass fp32, reconstruction of one zone
 //        along one direction (all dof), Riemann solve of one face,
 //        epilogue centre work of one zone (element, conserved vector,
 //        geometric source contraction; CT and divergence not counted)};
 // the Jacobian is the closed form for ideal MHD and the forward tangent
-// otherwise; the counts are the general metric's arithmetic also where the
-// step runs the Minkowski kernels
-template <int COND, int VISC>
+// otherwise (extended MHD in Kerr-Schild: the FP32 one is emhd_tangents).
+// Every part runs the functions the step's kernels run, on the metric's own
+// form of the geometry.
+template <int COND, int VISC, bool FLAT>
 __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, double* out) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   constexpr int NF = 5 + COND + VISC;
   const long long Z = c.Z;
   int i, j, k;
   zijk(c, z, i, j, k);
-  ZoneGeo<double> G;
+  Geo<FLAT, double> G;
   load_geo(G, c, b.geoC, z, i, j, 0.5, 0.5);
   StageConst<NF> K;
   load_stage_const<COND, VISC>(K, c, stage, b, z, G);
@@ -105,14 +124,15 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
   // residual, FP64
   {
     typedef Cnt<double> C8;
-    ZoneGeo<C8> Gc;
-    for (int m = 0; m < 4; m++)
-      for (int q = 0; q < 4; q++) { Gc.gcov[m][q] = C8(G.gcov[m][q]); Gc.gcon[m][q] = C8(G.gcon[m][q]); }
-    Gc.g = C8(G.g); Gc.alpha = C8(G.alpha); Gc.ialpha = C8(G.ialpha); Gc.x1 = C8(G.x1); Gc.x2 = C8(G.x2); Gc.dyn = C8(G.dyn);
+    Geo<FLAT, C8> Gc;
+    convert_geo(Gc, G);
     C8 P[NF], R[NF];
-    for (int v = 0; v < NF; v++) P[v] = C8(Pd[v]);
+    const C8 lam(0.);
     clear();
+    for (int v = 0; v < NF; v++) P[v] = C8(Pd[v]) + lam * C8(1.);
     zone_residual<COND, VISC, C8, C8>(P, K, Gc, c, R);
+    C8 l2(0.);
+    for (int v = 0; v < NF; v++) l2 = v ? l2 + R[v] * R[v] : R[v] * R[v];
     out[0] = flops(0);
     out[5] = (double)g_op_tally[0][2];
     out[6] = (double)(g_op_tally[0][3] + g_op_tally[0][4]);
@@ -120,10 +140,8 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
   // tangent pass in FP32 and in FP64
   {
     typedef Cnt<float> C4;
-    ZoneGeo<C4> Gt;
-    for (int m = 0; m < 4; m++)
-      for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = C4(G.gcov[m][q]); Gt.gcon[m][q] = C4(G.gcon[m][q]); }
-    Gt.g = C4(G.g); Gt.alpha = C4(G.alpha); Gt.ialpha = C4(G.ialpha); Gt.x1 = C4(G.x1); Gt.x2 = C4(G.x2); Gt.dyn = C4(G.dyn);
+    Geo<FLAT, C4> Gt;
+    convert_geo(Gt, G);
     C4 J[NF][NF];
     clear();
     tangent_jacobian<COND, VISC, C4, true>(Pd, K, Gt, c, J);
@@ -139,10 +157,8 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
   }
   {
     typedef Cnt<double> C8;
-    ZoneGeo<C8> Gt;
-    for (int m = 0; m < 4; m++)
-      for (int q = 0; q < 4; q++) { Gt.gcov[m][q] = C8(G.gcov[m][q]); Gt.gcon[m][q] = C8(G.gcon[m][q]); }
-    Gt.g = C8(G.g); Gt.alpha = C8(G.alpha); Gt.ialpha = C8(G.ialpha); Gt.x1 = C8(G.x1); Gt.x2 = C8(G.x2); Gt.dyn = C8(G.dyn);
+    Geo<FLAT, C8> Gt;
+    convert_geo(Gt, G);
     C8 J[NF][NF];
     clear();
     tangent_jacobian<COND, VISC, C8>(Pd, K, Gt, c, J);
@@ -157,10 +173,8 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
   {
     typedef Cnt<double> C8;
     constexpr int DOF = NF + 3;
-    ZoneGeo<C8> Gc;
-    for (int m = 0; m < 4; m++)
-      for (int q = 0; q < 4; q++) { Gc.gcov[m][q] = C8(G.gcov[m][q]); Gc.gcon[m][q] = C8(G.gcon[m][q]); }
-    Gc.g = C8(G.g); Gc.alpha = C8(G.alpha); Gc.ialpha = C8(G.ialpha); Gc.x1 = C8(G.x1); Gc.x2 = C8(G.x2); Gc.dyn = C8(G.dyn);
+    Geo<FLAT, C8> Gc;
+    convert_geo(Gc, G);
     const double* ps = b.ps;
     // reconstruction of every dof of the zone along X1
     clear();
@@ -171,31 +185,22 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
                            ro[v]);
     }
     out[8] = flops(0);
-    // one face: both states through the element, fluxes along X1 and X0,
-    // characteristic speeds, then the HLL / LLF combination
+    // one face: both states through the element and the characteristic
+    // speeds, then one flux vector per side and their sum (riemann_face_pair)
     clear();
-    C8 F[2][DOF], U[2][DOF], mn[2], mx[2];
+    C8 mn[2], mx[2], L[DOF], R[DOF], fl[DOF];
+    ElemT<C8, C8> e[2];
     for (int side = 0; side < 2; side++) {
       const C8* q = side ? lo : ro;
-      ElemT<C8, C8> e;
-      elem_set<COND, VISC>(e, q[0], q[1], q[2], q[3], q[4], q[NF], q[NF + 1], q[NF + 2], COND ? q[5] : C8(0.),
+      elem_set<COND, VISC>(e[side], q[0], q[1], q[2], q[3], q[4], q[NF], q[NF + 1], q[NF + 2], COND ? q[5] : C8(0.),
                            VISC ? q[5 + COND] : C8(0.), Gc, c);
-      fluxes_fluid<COND, VISC>(e, 1, Gc.g, F[side], 5, 5 + COND);
-      fluxes_B(e, 1, Gc.g, F[side] + NF);
-      fluxes_fluid<COND, VISC>(e, 0, Gc.g, U[side], 5, 5 + COND);
-      fluxes_B(e, 0, Gc.g, U[side] + NF);
-      char_speeds<COND, VISC>(e, Gc, 0, c, mn[side], mx[side]);
+      char_speeds<COND, VISC>(e[side], Gc, 0, c, mn[side], mx[side]);
     }
-    const C8 cmin = mn[0] <= mn[1] ? mn[0] : mn[1], cmax = mx[0] >= mx[1] ? mx[0] : mx[1];
-    C8 fl[DOF];
-    if (c.riemann == GRIM_HLL) {
-      const C8 id = C8(1.) / (cmax - cmin);
-      for (int v = 0; v < DOF; v++)
-        fl[v] = (cmax * F[0][v] - cmin * F[1][v] + cmin * cmax * (U[1][v] - U[0][v])) * id;
-    } else {
-      const C8 cm = cmax >= -cmin ? cmax : -cmin;
-      for (int v = 0; v < DOF; v++) fl[v] = C8(0.5) * (F[0][v] + F[1][v] - cm * (U[1][v] - U[0][v]));
-    }
+    const FaceWeights<C8> fw = face_weights(c, Gc.g, dmin2(mn[0], mn[1]), dmax2(mx[0], mx[1]));
+    side_flux<COND, VISC>(e[0], 0, fw.sL, L);
+    side_flux<COND, VISC>(e[1], 0, fw.sR, R);
+    for (int v = 0; v < DOF; v++) fl[v] = fw.aL * L[v] + fw.aR * R[v];
+    (void)fl;
     out[9] = flops(0);
     // epilogue centre: element, conserved vector, -g T^k_l Gamma^l_kn
     clear();
@@ -207,30 +212,31 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
       C8 Uc[NF], UB[3];
       fluxes_fluid<COND, VISC>(e, 0, Gc.g, Uc, 5, 5 + COND);
       fluxes_B(e, 0, Gc.g, UB);
-      if (c.metric != GRIM_MINKOWSKI) {
-        C8 T[4][4];
+      if constexpr (!FLAT) {
+        C8 T[4][4], acc[4];
         for (int ka = 0; ka < 4; ka++)
           for (int la = 0; la < 4; la++) T[ka][la] = tmunu<COND, VISC>(e, ka, la);
-        C8 S[4];
-        for (int nu = 0; nu < 4; nu++) {
-          S[nu] = C8(0.);
+        for (int la = 0; la < 4; la++)
           for (int ka = 0; ka < 4; ka++)
-            for (int la = 0; la < 4; la++) S[nu] = S[nu] - Gc.g * T[ka][la] * C8(1.);
-        }
-        (void)S;
+            for (int nu = ka; nu < 4; nu++) {
+              const C8 gv = Gc.g * C8(1.);
+              acc[nu] -= T[ka][la] * gv;
+              if (nu != ka) acc[ka] -= T[nu][la] * gv;
+            }
+        (void)acc;
       }
     }
     out[10] = flops(0);
   }
 }
 
-template <int C, int V>
+template <int C, int V, bool F>
 static void count_ops_t(const DevCfg& c, int stage, const StageBufs& b, long long z, double* out,
                         cudaStream_t s) {
-  k_count_ops<C, V><<<1, 32, 0, s>>>(c, stage, b, z, out);
+  k_count_ops<C, V, F><<<1, 32, 0, s>>>(c, stage, b, z, out);
 }
 void count_ops(const DevCfg& c, int stage, const StageBufs& b, long long z, double* out, cudaStream_t s) {
-  GRIM_EMHD_DISPATCH(c, count_ops_t, c, stage, b, z, out, s);
+  GRIM_GEO_DISPATCH(c, count_ops_t, c, stage, b, z, out, s);
 }
 
 }  // namespace GRIM_KNS

@@ -40,6 +40,11 @@ struct FlatGeo {
   R x1, x2;
   R dyn;
 };
+// a factor of one in an expression shared with cases that have another
+struct One {};
+template <class X> GRIM_HD X operator*(One, const X& x) { return x; }
+template <class X> GRIM_HD X operator*(const X& x, One) { return x; }
+template <class X> GRIM_HD X operator/(One, const X& x) { return X(1) / x; }
 template <bool FLAT, class R> struct GeoSel { typedef ZoneGeo<R> type; };
 template <class R> struct GeoSel<true, R> { typedef FlatGeo<R> type; };
 template <bool FLAT, class R> using Geo = typename GeoSel<FLAT, R>::type;
@@ -751,7 +756,7 @@ GRIM_D void zone_residual(const S* P, const StageConst<5 + COND + VISC>& K, cons
 #ifdef GRIM_FAST_MATH
   // U without its sqrt(-g), which goes with 1 / dt'; the unknown-independent
   // terms folded into one constant per row
-  fluxes_fluid<COND, VISC>(e, 0, T(1), U, Q, DP);
+  fluxes_fluid<COND, VISC>(e, 0, One(), U, Q, DP);
   const R gi = G.g * (R)K.idtp;
 #pragma unroll
   for (int v = 0; v < 5; v++) Rout[v] = U[v] * gi + (T)K.Kc[v];

@@ -254,8 +254,9 @@ class timeStepper:
         return out
 
     def countFlops(self):
-        """Algorithmic flops of one zone: residual (FP64), tangent pass
-        (FP32 and FP64), pivoted solve (FP32 and FP64)."""
+        """Algorithmic flops of one zone: a residual evaluation of the line
+        search (FP64: trial state, residual, norm), tangent pass (FP32 and
+        FP64), pivoted solve (FP32 and FP64)."""
         out = (ctypes.c_double * 11)()
         _lib.check(_lib.lib().grim_count_flops(self._h, out), "count_flops")
         keys = ("residual64", "tangent32", "tangent64", "solve32", "solve64", "residual_div", "residual_sqrt_exp",

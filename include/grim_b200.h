@@ -437,8 +437,9 @@ int grim_profile_steps(grim_handle* h, int nsteps, double* msPerGroup, long long
                        int ngroups);
 /* Algorithmic flop counts of one zone (the middle interior zone of the
  * last set-up stage), counted by running the kernels' templated physics on
- * a counting scalar: out[0] residual (FP64), out[1] Jacobian in FP32 (the
- * closed form for ideal MHD, the forward tangent otherwise), out[2] the
+ * a counting scalar, in the metric's own form: out[0] one residual evaluation
+ * of the line search (trial state, residual, norm; FP64), out[1] Jacobian in
+ * FP32 (the closed form for ideal MHD, the forward tangent otherwise), out[2] the
  * same in FP64, out[3] pivoted solve FP32, out[4] the same in FP64, out[5]
  * divisions and out[6] sqrt+exp of the residual, out[7] the generic
  * forward-tangent pass in FP32; stencil work in FP64: out[8] the
@@ -449,7 +450,7 @@ int grim_profile_steps(grim_handle* h, int nsteps, double* msPerGroup, long long
 int grim_count_flops(grim_handle* h, double* out);
 /* Autotuner of the face-flux kernels' launch shapes (register budget per
  * thread, lane split between i and the face direction): times every
- * variant of each direction on the state in primOld for the handle's
+ * kernel of each direction on the state in primOld for the handle's
  * current Newton mode (its compilation unit) and keeps the fastest.
  * variants[d] and msBest[d] (may be null) receive the choice and its time
  * per launch.  In the FP64 parity path (no FMA contraction) every variant

@@ -649,3 +649,38 @@ def test_flux_ct_divergence_is_the_field_update(dim):
         ref = divF[b1 + b][s3, s2, s1]
         scale = max(np.max(np.abs(ref)), 1e-30)
         assert np.max(np.abs(got - ref)) <= 1e-12 * scale, (b, np.max(np.abs(got - ref)) / scale)
+
+
+@pytest.mark.parametrize("emhd", [0, 1])
+def test_flop_counts_are_the_metrics_own(emhd):
+    """The counts run the functions the step's kernels run: in Minkowski
+    without the products with the metric's zeros and ones, so fewer of each
+    part than in Kerr-Schild on the same numbers; a face with one flux vector
+    per side, so the two sides' combination is 3 operations per row and not the
+    8 of fluxes and conserved variables formed apart."""
+    from grim_b200.timestepper import timeStepper
+    counts = []
+    for metric in (C.MINKOWSKI, C.MODIFIED_KERR_SCHILD):
+        cfg = PR.fast_mode_config(N=16, metric=metric, conduction=emhd, viscosity=emhd, riemannSolver=C.HLL,
+                                  newtonMode=C.NEWTON_MIXED32, perZoneConvergence=1)
+        ts = timeStepper(cfg)
+        if metric == C.MODIFIED_KERR_SCHILD:
+            eta = np.zeros((4, 4) + ts.zshape)
+            for m in range(4):
+                eta[m, m] = -1. if m == 0 else 1.
+            one = np.ones(ts.zshape)
+            for loc in (C.CENTER, C.LEFT, C.RIGHT, C.TOP, C.BOTTOM):
+                ts.setGeometry(loc, eta, eta, one, one, gamma=np.zeros((64,) + ts.zshape))
+        ts.primOld.setVars(PR.fast_mode_prims(cfg))
+        ts.stageSetup(C.HALF_STEP)
+        counts.append(ts.countFlops())
+    flat, curved = counts
+    for part in ("residual64", "tangent32", "tangent64", "riemann_face", "epilogue_zone"):
+        assert 0 < flat[part] < curved[part], part
+    for part in ("solve32", "solve64", "recon_zone_dir"):
+        assert flat[part] == curved[part], part
+    # ideal MHD in Minkowski, HLL, by hand: two elements (38 operations each),
+    # two pairs of speeds (30), two sides (36), the weights (4) and 8 x 3; F and
+    # U of both sides apart, combined row by row, take 100 more
+    if not emhd:
+        assert 220 <= flat["riemann_face"] <= 250, flat
