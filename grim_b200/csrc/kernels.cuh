@@ -225,12 +225,9 @@ __global__ void k_emhd_prepass(DevCfg c, const double* __restrict__ ps, const do
 template <int DOF, int RS>
 GRIM_D void recon_zone_rs(const DevCfg& c, const double* __restrict__ ps, long long z, long long s, double* lo,
                           double* ro) {
-#pragma unroll
-  for (int v = 0; v < DOF; v++) {
-    const double* a = ps + (long long)v * c.Z + z;
-    const double y0 = __ldg(a - 2 * s), y1 = __ldg(a - s), y2 = __ldg(a), y3 = __ldg(a + s), y4 = __ldg(a + 2 * s);
-    recon_faces_rs<RS, kFastMath>(c.reconstruction, c.theta, y0, y1, y2, y3, y4, lo[v], ro[v]);
-  }
+  recon_vars<DOF, RS, kFastMath>(
+      c.reconstruction, c.theta,
+      [&](int v, int m) { return __ldg(ps + (long long)v * c.Z + z + (m - 2) * s); }, lo, ro);
 }
 // the scheme is chosen once, outside the loop over the variables, so the
 // path a warp executes is one scheme's contiguous code
@@ -563,11 +560,8 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_x1_tma(const __grid_con
     const int iu = reconOK ? iz : i0 - 1;  // a zone inside the buffer
     const double* rb = rows + buf * ROW;
     double lo[DOF], ro[DOF];
-#pragma unroll
-    for (int v = 0; v < DOF; v++) {
-      const double* a = rb + v * kX1Box + (iu - x0);
-      recon_faces_rs<RS, kFastMath>(c.reconstruction, c.theta, a[-2], a[-1], a[0], a[1], a[2], lo[v], ro[v]);
-    }
+    recon_vars<DOF, RS, kFastMath>(
+        c.reconstruction, c.theta, [&](int v, int m) { return rb[v * kX1Box + (iu - x0) + m - 2]; }, lo, ro);
     __syncwarp();  // the buffer is read; it may be refilled two items on
     double pl[DOF];
 #pragma unroll
@@ -663,12 +657,9 @@ __global__ void __launch_bounds__(128, MINB) k_face_flux_strip_tma(const __grid_
     const bool reconOK = i < c.N1T && x <= NT - 3;
     const double* rb = bufs + buf * BOX;
     double lo[DOF], ro[DOF];
-#pragma unroll
-    for (int v = 0; v < DOF; v++) {
-      const double* a = rb + (v * kStripRows + jj) * QI + ii;  // rows jj .. jj+4 hold x-2 .. x+2
-      recon_faces_rs<RS, kFastMath>(c.reconstruction, c.theta, a[0], a[QI], a[2 * QI], a[3 * QI], a[4 * QI], lo[v],
-                                    ro[v]);
-    }
+    // rows jj .. jj+4 hold x-2 .. x+2
+    recon_vars<DOF, RS, kFastMath>(
+        c.reconstruction, c.theta, [&](int v, int m) { return rb[(v * kStripRows + jj + m) * QI + ii]; }, lo, ro);
     __syncwarp();  // the buffer is read; it may be refilled two items on
     double pl[DOF];
 #pragma unroll
@@ -982,36 +973,56 @@ GRIM_D void epilogue_zone(const DevCfg& c, int stage, const StageBufs& b, long l
     // computeEMHDGradients (physics.cpp:502-586) from the pre-pass u_mu, T
     double gu[4][4], gT[4];
     const double* uT = b.uT;
-    auto st = [&](int m, int dir, double dx) -> double {
+    [[maybe_unused]] int top = 0;
+    // the slope of row m along dir; plain: the parity path's form
+    auto st = [&](int m, int dir, auto plain) -> double {
       const long long sd = stride_of(c, dir);
       const double* a = uT + (long long)m * Z + z;
-      if constexpr (kFastMath)
-        return recon_slope_fast(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.invdX[dir]);
+      if constexpr (!kFastMath || decltype(plain)::value)
+        return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.dX[dir]);
       else
-        return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], dx);
+        return recon_slope_fast(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.invdX[dir], top);
     };
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) {
       gu[0][mu] = 0.;
-      gu[1][mu] = st(mu, 0, c.dX[0]);
-      gu[2][mu] = (c.dim > 1) ? st(mu, 1, c.dX[1]) : 0.;
-      gu[3][mu] = (c.dim > 2) ? st(mu, 2, c.dX[2]) : 0.;
-      if constexpr (!FLAT && kFastMath) {
 #pragma unroll
-        for (int nu = 0; nu < 4; nu++) gu[nu][mu] -= nu <= mu ? gu0[nu][mu] : gu0[mu][nu];
-      } else if constexpr (!FLAT) {
+      for (int d = 0; d < 3; d++) gu[d + 1][mu] = (d < c.dim) ? st(mu, d, std::false_type()) : 0.;
+    }
+    gT[0] = 0.;
+    if (COND) {
 #pragma unroll
-        for (int nu = 0; nu < 4; nu++)
+      for (int d = 0; d < 3; d++) gT[d + 1] = (d < c.dim) ? st(4, d, std::false_type()) : 0.;
+    }
+    // as the faces' second pass (recon_vars)
+    if constexpr (kFastMath) {
+      if (__builtin_expect(top >= kNonFinite, 0)) {
+#pragma unroll 1
+        for (int m = 0; m < (COND ? 5 : 4); m++)
 #pragma unroll
-          for (int la = 0; la < 4; la++)
-            gu[nu][mu] -= __ldg(b.gamma + (long long)(la * 16 + nu * 4 + mu) * c.GZ + gidx(c, i, j)) * e.uCov[la];
+          for (int d = 0; d < 3; d++) {
+            if (d >= c.dim) continue;
+            const double sl = st(m, d, std::true_type());
+#pragma unroll
+            for (int mu = 0; mu < 4; mu++)
+              if (mu == m) gu[d + 1][mu] = sl;
+            if (m == 4) gT[d + 1] = sl;
+          }
       }
     }
-    if (COND) {
-      gT[0] = 0.;
-      gT[1] = st(4, 0, c.dX[0]);
-      gT[2] = (c.dim > 1) ? st(4, 1, c.dX[1]) : 0.;
-      gT[3] = (c.dim > 2) ? st(4, 2, c.dX[2]) : 0.;
+    if constexpr (!FLAT) {
+#pragma unroll
+      for (int mu = 0; mu < 4; mu++)
+#pragma unroll
+        for (int nu = 0; nu < 4; nu++) {
+          if constexpr (kFastMath) {
+            gu[nu][mu] -= nu <= mu ? gu0[nu][mu] : gu0[mu][nu];
+          } else {
+#pragma unroll
+            for (int la = 0; la < 4; la++)
+              gu[nu][mu] -= __ldg(b.gamma + gidx(c, i, j) + (long long)(la * 16 + nu * 4 + mu) * c.GZ) * e.uCov[la];
+          }
+        }
     }
     double dv = 0.;
     // in Minkowski only the diagonal enters, and nothing along X^0 (gu[0]

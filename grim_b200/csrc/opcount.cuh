@@ -179,10 +179,11 @@ __global__ void k_count_ops(DevCfg c, int stage, StageBufs b, long long z, doubl
     // reconstruction of every dof of the zone along X1
     clear();
     C8 lo[DOF], ro[DOF];
+    int top = 0;
     for (int v = 0; v < DOF; v++) {
       const double* a = ps + (long long)v * Z + z;
       recon_faces_fast<C8>(c.reconstruction, c.theta, C8(a[-2]), C8(a[-1]), C8(a[0]), C8(a[1]), C8(a[2]), lo[v],
-                           ro[v]);
+                           ro[v], top);
     }
     out[8] = flops(0);
     // one face: both states through the element and the characteristic

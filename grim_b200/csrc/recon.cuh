@@ -127,38 +127,54 @@ GRIM_D S mp5(S vm2, S vm1, S v0, S vp1, S vp2) {
 // operations per variable (adds, products, compares): PPM 58 -> 30, WENO5
 // about 130 -> 85, minmod 20 -> 9; the reconstruction was over half of a
 // face kernel's work.
-// whether two numbers' signs agree (a zero counts as either; the callers'
-// result is zero then)
-GRIM_D bool same_sign(double a, double b) { return (__double2hiint(a) ^ __double2hiint(b)) >= 0; }
+// The limiters below keep a NaN of their differences, where the plain forms
+// drop it from a minimum and take it for positive, and so do with an infinity
+// what the plain forms do or make it a NaN.  A zone where one shows is done again
+// in the plain form: `top` keeps the largest exponent word among the variables'
+// last products, kNonFinite and above says so.
+constexpr int kNonFinite = 0x7ff00000;
+GRIM_D void note_exponent(int& top, double x) { top = max(top, __double2hiint(x) & 0x7fffffff); }
 template <class S>
-GRIM_D bool same_sign(S a, S b) { return (a < S(0.)) == (b < S(0.)); }
+GRIM_D void note_exponent(int&, S) {}
+// the smaller of the two, x if x is a NaN (a compare and a select: fewer
+// instructions than fmin, which drops it)
+template <class S>
+GRIM_D S min_keep(S x, S y) { return x >= y ? y : x; }
+// +-1, a's sign, where the two finite numbers' signs agree, else 0 (a zero
+// counts as either; the callers' result is zero then)
+GRIM_D double common_sign(double a, double b) {
+  const int ha = __double2hiint(a);
+  return __hiloint2double((ha ^ __double2hiint(b)) >= 0 ? (ha & 0x80000000) | 0x3ff00000 : 0, 0);
+}
+template <class S>
+GRIM_D S common_sign(S a, S b) { return (a < S(0.)) == (b < S(0.)) ? copysign(S(1.), a) : S(0.); }
 
 // PPM: with the differences e = y[k+1] - y[k], a limited slope is twice
 // h = sgn min(|e0 + e1| / 4, |e0|, |e1|) (zero at an extremum) and the zone's
 // offsets to its faces are al = y2 - l, ar = r - y2.  The three corrections
 // become: offsets of opposite sign vanish, neither exceeds twice the other.
-// The comparisons leave a NaN offset in place.
 template <class S>
 GRIM_D S ppm_half_slope(S a, S b) {
-  const S m = fmin(S(0.25) * fabs(a + b), fmin(fabs(a), fabs(b)));
-  return same_sign(a, b) ? copysign(m, a) : S(0.);  // the sign by a bit operation, not a compare
+  return common_sign(a, b) * min_keep(S(0.25) * fabs(a + b), min_keep(fabs(a), fabs(b)));
 }
 template <class S>
-GRIM_D void ppm_offsets(S y0, S y1, S y2, S y3, S y4, S& al, S& ar) {
+GRIM_D void ppm_offsets(S y0, S y1, S y2, S y3, S y4, S& al, S& ar, int& top) {
   const S e0 = y1 - y0, e1 = y2 - y1, e2 = y3 - y2, e3 = y4 - y3;
   const S h1 = ppm_half_slope(e0, e1), h2 = ppm_half_slope(e1, e2), h3 = ppm_half_slope(e2, e3);
   const S l = S(0.5) * e1 + S(1. / 3.) * (h2 - h1);
   const S r = S(0.5) * e2 - S(1. / 3.) * (h3 - h2);
   const S l2 = l + l, r2 = r + r;
-  const bool flat = l * r <= S(0.);
+  const S lr = l * r;
+  note_exponent(top, lr);
+  const bool flat = lr <= S(0.);
   al = (fabs(l) > fabs(r2)) ? r2 : l;
   ar = (fabs(r) > fabs(l2)) ? l2 : r;
   if (flat) al = ar = S(0.);
 }
 template <class S>
-GRIM_D void ppm_faces_fast(S y0, S y1, S y2, S y3, S y4, S& leftV, S& rightV) {
+GRIM_D void ppm_faces_fast(S y0, S y1, S y2, S y3, S y4, S& leftV, S& rightV, int& top) {
   S al, ar;
-  ppm_offsets(y0, y1, y2, y3, y4, al, ar);
+  ppm_offsets(y0, y1, y2, y3, y4, al, ar, top);
   leftV = y2 - al;
   rightV = y2 + ar;
 }
@@ -189,9 +205,11 @@ GRIM_D void weno5_faces_fast(S y0, S y1, S y2, S y3, S y4, S& lo, S& ro) {
 
 // minmod: the limited slope is the smallest of the three where all signs agree
 template <class S>
-GRIM_D S slope_mm_fast(S bwd, S fwd, double theta) {
-  const S m = fmin(S(0.5) * fabs(bwd + fwd), theta * fmin(fabs(bwd), fabs(fwd)));
-  return same_sign(bwd, fwd) ? copysign(m, bwd) : S(0.);
+GRIM_D S slope_mm_fast(S bwd, S fwd, double theta, int& top) {
+  const S slope = common_sign(bwd, fwd) *
+                  min_keep(S(0.5) * fabs(bwd + fwd), S(theta) * min_keep(fabs(bwd), fabs(fwd)));
+  note_exponent(top, slope);
+  return slope;
 }
 
 // face values of zone i
@@ -216,13 +234,13 @@ GRIM_D void recon_faces(int scheme, double theta, S y0, S y1, S y2, S y3, S y4,
 }
 template <class S>
 GRIM_D void recon_faces_fast(int scheme, double theta, S y0, S y1, S y2, S y3, S y4,
-                             S& lo, S& ro) {
+                             S& lo, S& ro, int& top) {
   if (scheme == GRIM_WENO5) {
     weno5_faces_fast(y0, y1, y2, y3, y4, lo, ro);
   } else if (scheme == GRIM_PPM) {
-    ppm_faces_fast(y0, y1, y2, y3, y4, lo, ro);
+    ppm_faces_fast(y0, y1, y2, y3, y4, lo, ro, top);
   } else if (scheme == GRIM_MINMOD) {
-    const S s = slope_mm_fast(y2 - y1, y3 - y2, theta);
+    const S s = slope_mm_fast(y2 - y1, y3 - y2, theta, top);
     lo = y2 - S(0.5) * s;
     ro = y2 + S(0.5) * s;
   } else {
@@ -230,16 +248,36 @@ GRIM_D void recon_faces_fast(int scheme, double theta, S y0, S y1, S y2, S y3, S
   }
 }
 
-// face values with the scheme fixed at compile time (RS >= 0: one scheme's
-// code in the kernel) or read at run time (RS < 0); FAST selects the
-// reassociated WENO5 weights
-template <int RS, bool FAST, class S>
-GRIM_D void recon_faces_rs(int scheme, double theta, S y0, S y1, S y2, S y3, S y4, S& lo, S& ro) {
+// face values of DOF variables, get(v, m) their stencils' points, with the
+// scheme fixed at compile time (RS >= 0: one scheme's code in the kernel) or
+// read at run time (RS < 0); FAST selects the fast path's forms.  The second
+// pass, hardly ever taken, is a loop of one variable's code with loads of its
+// own: unrolled, or on the values of the first pass, its code and registers
+// slowed every face (PPM vortex 301x187 127 -> 148 us).
+template <int DOF, int RS, bool FAST, class Get>
+GRIM_D void recon_vars(int scheme, double theta, const Get& get, double* lo, double* ro) {
   const int rs = RS < 0 ? scheme : RS;  // a constant scheme folds the choice
-  if constexpr (FAST)
-    recon_faces_fast(rs, theta, y0, y1, y2, y3, y4, lo, ro);
-  else
-    recon_faces(rs, theta, y0, y1, y2, y3, y4, lo, ro);
+  [[maybe_unused]] int top = 0;
+#pragma unroll
+  for (int v = 0; v < DOF; v++) {
+    const double y0 = get(v, 0), y1 = get(v, 1), y2 = get(v, 2), y3 = get(v, 3), y4 = get(v, 4);
+    if constexpr (FAST)
+      recon_faces_fast(rs, theta, y0, y1, y2, y3, y4, lo[v], ro[v], top);
+    else
+      recon_faces(rs, theta, y0, y1, y2, y3, y4, lo[v], ro[v]);
+  }
+  if constexpr (FAST) {
+    if (__builtin_expect((rs == GRIM_PPM || rs == GRIM_MINMOD) && top >= kNonFinite, 0)) {
+#pragma unroll 1
+      for (int v = 0; v < DOF; v++) {
+        double l, r;
+        recon_faces(rs, theta, get(v, 0), get(v, 1), get(v, 2), get(v, 3), get(v, 4), l, r);
+#pragma unroll
+        for (int u = 0; u < DOF; u++)
+          if (u == v) { lo[u] = l; ro[u] = r; }
+      }
+    }
+  }
 }
 
 // the slope() used by the EMHD gradients (reconstruction.cpp:39-64); MP5
@@ -254,15 +292,15 @@ GRIM_D S recon_slope(int scheme, double theta, S y0, S y1, S y2, S y3,
     default: return slope_mm(y1, y2, y3, dX, theta);
   }
 }
-// the same in the fast path's forms, idX = 1 / dX
+// the same in the fast path's forms, idX = 1 / dX; top as for the faces
 template <class S>
-GRIM_D S recon_slope_fast(int scheme, double theta, S y0, S y1, S y2, S y3, S y4, double idX) {
+GRIM_D S recon_slope_fast(int scheme, double theta, S y0, S y1, S y2, S y3, S y4, double idX, int& top) {
   if (scheme == GRIM_PPM) {
     S al, ar;
-    ppm_offsets(y0, y1, y2, y3, y4, al, ar);
+    ppm_offsets(y0, y1, y2, y3, y4, al, ar, top);
     return (al + ar) * idX;
   }
-  if (scheme == GRIM_MINMOD) return slope_mm_fast((y2 - y1) * idX, (y3 - y2) * idX, theta);
+  if (scheme == GRIM_MINMOD) return slope_mm_fast((y2 - y1) * idX, (y3 - y2) * idX, theta, top);
   return (S(8.) * (y3 - y1) - (y4 - y0)) * (S(1. / 12.) * idX);
 }
 
