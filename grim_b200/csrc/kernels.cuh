@@ -974,40 +974,45 @@ GRIM_D void epilogue_zone(const DevCfg& c, int stage, const StageBufs& b, long l
     double gu[4][4], gT[4];
     const double* uT = b.uT;
     [[maybe_unused]] int top = 0;
-    // the slope of row m along dir; plain: the parity path's form
-    auto st = [&](int m, int dir, auto plain) -> double {
+    auto st = [&](int m, int dir) -> double {
       const long long sd = stride_of(c, dir);
       const double* a = uT + (long long)m * Z + z;
-      if constexpr (!kFastMath || decltype(plain)::value)
-        return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.dX[dir]);
-      else
+      if constexpr (kFastMath)
         return recon_slope_fast(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.invdX[dir], top);
+      else
+        return recon_slope(c.reconstruction, c.theta, a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.dX[dir]);
     };
 #pragma unroll
     for (int mu = 0; mu < 4; mu++) {
       gu[0][mu] = 0.;
 #pragma unroll
-      for (int d = 0; d < 3; d++) gu[d + 1][mu] = (d < c.dim) ? st(mu, d, std::false_type()) : 0.;
+      for (int d = 0; d < 3; d++) gu[d + 1][mu] = (d < c.dim) ? st(mu, d) : 0.;
     }
     gT[0] = 0.;
     if (COND) {
 #pragma unroll
-      for (int d = 0; d < 3; d++) gT[d + 1] = (d < c.dim) ? st(4, d, std::false_type()) : 0.;
+      for (int d = 0; d < 3; d++) gT[d + 1] = (d < c.dim) ? st(4, d) : 0.;
     }
-    // as the faces' second pass (recon_vars)
+    // in the plain form, as the faces' second pass (recon_vars)
     if constexpr (kFastMath) {
       if (__builtin_expect(top >= kNonFinite, 0)) {
 #pragma unroll 1
-        for (int m = 0; m < (COND ? 5 : 4); m++)
+        for (int q = 0; q < (COND ? 15 : 12); q++) {
+          const int m = q / 3, d = q - 3 * m;
+          if (d >= c.dim) continue;
+          const long long sd = stride_of(c, d);
+          const double* a = uT + (long long)m * Z + z;
+          const double sl = c.reconstruction == GRIM_PPM
+                                ? slope_ppm(a[-2 * sd], a[-sd], a[0], a[sd], a[2 * sd], c.dX[d])
+                                : slope_mm(a[-sd], a[0], a[sd], c.dX[d], c.theta);
 #pragma unroll
-          for (int d = 0; d < 3; d++) {
-            if (d >= c.dim) continue;
-            const double sl = st(m, d, std::true_type());
+          for (int e1 = 0; e1 < 3; e1++) {
 #pragma unroll
             for (int mu = 0; mu < 4; mu++)
-              if (mu == m) gu[d + 1][mu] = sl;
-            if (m == 4) gT[d + 1] = sl;
+              if (mu == m && e1 == d) gu[e1 + 1][mu] = sl;
+            if (m == 4 && e1 == d) gT[e1 + 1] = sl;
           }
+        }
       }
     }
     if constexpr (!FLAT) {
