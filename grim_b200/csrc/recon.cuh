@@ -124,8 +124,8 @@ GRIM_D S mp5(S vm2, S vm1, S v0, S vp1, S vp2) {
 // to the forms above to a few ulp of the stencil's largest value (WENO5: to
 // what the weights' rounding allows; the differences form its smoothness
 // measures without the cancellation of the expanded squares).  FP64-pipe
-// operations per variable (adds, products, compares): PPM 58 -> 30, WENO5
-// about 130 -> 85, minmod 20 -> 9; the reconstruction was over half of a
+// operations per variable (adds, products, compares): PPM 58 -> 33, WENO5
+// about 130 -> 85, minmod 20 -> 10; the reconstruction was over half of a
 // face kernel's work.
 // The limiters below keep a NaN of their differences, where the plain forms
 // drop it from a minimum and take it for positive, and so do with an infinity

@@ -581,10 +581,9 @@ static void enqueue_boundaries(grim_handle* h, double* p) {
   g_launch_counter++;
 }
 
-// The step in segments around the two stencil + Newton pairs, so that a
-// batch of problems can interleave its problems around one shared Newton
-// launch: pre_half -> stencil(half) -> Newton(half) -> mid -> stencil(full)
-// -> Newton(full) -> post.
+// The step in segments around the two stencil + Newton pairs, as a slab-
+// decomposed run exchanges its halos between them: pre_half -> stencil(half)
+// -> Newton(half) -> mid -> stencil(full) -> Newton(full) -> post.
 static void enqueue_pre_half(grim_handle* h, bool timed) {
   cudaStream_t s = h->stream;
   if (timed) cudaEventRecord(h->ev[0], s);

@@ -6,7 +6,7 @@ In the FP64 parity form the two give the same bits (adding a zero and
 multiplying by one are exact; with conduction or viscosity too); in the mixed
 form the compiler contracts the two differently, so they agree to rounding:
 1e-12 of each variable's scale, some 1e3 operations at 1e-16 on these
-well-conditioned states.  A non-finite value, which a zero term spreads
+well-conditioned states (largest seen: 3.4e-14, with extended MHD 3.2e-14).  A non-finite value, which a zero term spreads
 (0 x Inf is NaN), is lost in the same zones.
 """
 import numpy as np
@@ -68,7 +68,7 @@ def test_minkowski_kernels_match_the_general_ones(dim, emhd, solver, scheme):
     assert np.all(np.isfinite(b)) and np.array_equal(a, b)
     tol = dict(nonlinearsolve_rtol=1e-12, nonlinearsolve_atol=1e-28, nonlinearsolve_ulps=8., maxNonLinearIter=6)
     a, b = _pair(_config(dim, emhd, scheme, solver, **tol), C.NEWTON_MIXED32, P)
-    assert scaled_err(a, b) <= (1e-9 if emhd else 1e-12)
+    assert scaled_err(a, b) <= 1e-12
 
 
 @pytest.mark.parametrize("mode", [C.NEWTON_PARITY_FD64, C.NEWTON_MIXED32])

@@ -299,6 +299,32 @@ def test_closed_form_jacobian_on_kerr_schild():
     assert _column_err(J64, Jfd, keep) <= 1e-6
 
 
+@pytest.mark.parametrize("steps", [0, 3])
+def test_emhd_fp32_tangents_on_kerr_schild(steps):
+    """The FP32 Jacobian of the mixed Newton with conduction and viscosity in
+    Kerr-Schild, whose tangents are written out apart from the folded residual
+    (emhd_tangents), against the FP64 forward tangents of that residual on the
+    torus, at the first half stage and three steps on: 7e-5 of each zone's column
+    scale, a thousand FP32 roundings (largest seen 1.7e-5); a term left out
+    or a wrong sign is of order one."""
+    from grim_b200.timestepper import timeStepper as TS
+    cfg = T.torus_config(N1=64, N2=32, N3=8, emhd=True)
+    ts = TS(cfg)
+    P, _ = T.torus_prims(cfg, ts.getGeometry(C.CENTER))
+    ts.primOld.setVars(P)
+    ts.problemInit()
+    if steps:
+        ts.timeSteps(steps)
+    ts.stageSetup(C.HALF_STEP)
+    guess = ts.prim.getVars()
+    J64, J32 = ts.jacobianForm(guess, TS.JAC_FAST64), ts.jacobianForm(guess, TS.JAC_FAST32)
+    keep = np.zeros(ts.zshape + (1, 1), bool)
+    keep[C.interior_slices(cfg)] = True
+    keep = np.broadcast_to(keep, J64.shape)
+    assert np.all(np.isfinite(J64[keep]))
+    assert _column_err(J32, J64, keep) <= 7e-5
+
+
 def test_torus_fast_steps_match_parity_path():
     """The fast form of the torus step (FP32 closed-form Jacobian, FP64
     residual, per-zone convergence, FMA arithmetic, its fused floors / dt /
